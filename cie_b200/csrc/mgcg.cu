@@ -37,6 +37,7 @@ struct MgScalars {
     int done, error, errorKind, flexible;
     long long errorIter, chunkIter, chunkLimit, cycles;
     double cgamma, calpha, cbeta;  // coarse solve
+    double cgammaPrev, calphaPrev;  // of the step before
     int cfrozen;
 };
 
@@ -316,7 +317,6 @@ __global__ void __launch_bounds__(kT) coarse_start_kernel(long m, const double* 
         v.r[i] = bi;
         v.u[i] = dinv[i] * bi;
         v.z[i] = 0.0;
-        v.q[i] = 0.0;
         v.s[i] = 0.0;
         v.p[i] = 0.0;
     }
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(csr_threads<K>())
 
 struct CoarsePipeOp {
     struct Pre {
-        double z, q, s, p, x, r, u, w, m, d;
+        double z, s, p, x, r, w, d;
     };
     const double* __restrict__ dinv;
     CoarseVectors v;
@@ -366,19 +366,17 @@ struct CoarsePipeOp {
     double alpha, beta;
     double gamma, delta;
     __device__ __forceinline__ Pre pre(int i) const {
-        return Pre{v.z[i], v.q[i], v.s[i], v.p[i], v.x[i], v.r[i], v.u[i], v.w[i], mcur[i], dinv[i]};
+        return Pre{v.z[i], v.s[i], v.p[i], v.x[i], v.r[i], v.w[i], dinv[i]};
     }
     __device__ __forceinline__ void post(int i, const Pre& a, double n) {
-        const double z = fma(beta, a.z, n), q = fma(beta, a.q, a.m), s = fma(beta, a.s, a.w),
-                     p = fma(beta, a.p, a.u);
-        const double r = fma(-alpha, s, a.r), u = fma(-alpha, q, a.u), w = fma(-alpha, z, a.w);
+        const double z = fma(beta, a.z, n), s = fma(beta, a.s, a.w), p = fma(beta, a.p, a.d * a.r);
+        const double r = fma(-alpha, s, a.r), w = fma(-alpha, z, a.w);
+        const double u = a.d * r;
         v.z[i] = z;
-        v.q[i] = q;
         v.s[i] = s;
         v.p[i] = p;
         v.x[i] = fma(alpha, p, a.x);
         v.r[i] = r;
-        v.u[i] = u;
         v.w[i] = w;
         mnext[i] = a.d * w;
         gamma = fma(r, u, gamma);
@@ -401,6 +399,62 @@ __global__ void __launch_bounds__(csr_threads<K>())
         const double beta = tot[0] / s->cgamma;
         const double denom = tot[1] - beta * tot[0] / s->calpha;
         if (!(0.0 < tot[0]) || !(0.0 < denom)) {  // converged to rounding or broken down: no further steps
+            s->calpha = 0.0;
+            s->cbeta = 0.0;
+            s->cfrozen = 1;
+            return;
+        }
+        s->cgammaPrev = s->cgamma;
+        s->calphaPrev = s->calpha;
+        s->cbeta = beta;
+        s->calpha = tot[0] / denom;
+        s->cgamma = tot[0];
+    }
+}
+
+// The recurrences for w = A u and z = A q (q = D^-1 s) lose what a product would
+// keep: after 80 iterations on a finite-cell matrix (alpha = 1e-6, 41^2 rows) the
+// iterate was up to 5e-6 from the Jacobi-PCG's.  Every kCoarseReplace iterations
+// both are recomputed as products (an elementwise kernel and two row passes)
+// together with the next alpha and beta.
+constexpr int kCoarseReplace = 16;
+
+__global__ void __launch_bounds__(kT) coarse_precondition_kernel(long m, const double* __restrict__ dinv,
+                                                                 CoarseVectors v) {
+    for (long i = blockIdx.x * static_cast<long>(kT) + threadIdx.x; i < m; i += static_cast<long>(gridDim.x) * kT) {
+        const double d = dinv[i];
+        v.u[i] = d * v.r[i];
+        v.q[i] = d * v.s[i];
+    }
+}
+
+struct CoarseProductOp {
+    struct Pre {};
+    double* __restrict__ out;
+    __device__ __forceinline__ Pre pre(int) const { return Pre{}; }
+    __device__ __forceinline__ void post(int i, const Pre&, double sum) const { out[i] = sum; }
+};
+
+template <int K>
+__global__ void __launch_bounds__(csr_threads<K>()) coarse_product_kernel(CsrArgs<double> A, CoarseVectors v) {
+    CoarseProductOp op{v.z};
+    csr_rows<K, double, double, false>(A, v.q, op);
+}
+
+template <int K>
+__global__ void __launch_bounds__(csr_threads<K>())
+    coarse_replace_kernel(CsrArgs<double> A, const double* __restrict__ dinv, CoarseVectors v, int cur, MgScalars* s,
+                          double* partials, unsigned* counter) {
+    double* const m = cur ? v.m[1] : v.m[0];
+    v.m[0] = m;
+    CoarseFirstOp op{dinv, v, 0.0, 0.0};  // w, m, gamma, delta from u
+    csr_rows<K, double, double, false>(A, v.u, op);
+    double mine[2] = {op.gamma, op.delta}, tot[2];
+    if (grid_reduce_last<2, csr_threads<K>()>(mine, partials, counter, tot) && threadIdx.x == 0) {
+        if (s->cfrozen) return;
+        const double beta = tot[0] / s->cgammaPrev;
+        const double denom = tot[1] - beta * tot[0] / s->calphaPrev;
+        if (!(0.0 < tot[0]) || !(0.0 < denom)) {
             s->calpha = 0.0;
             s->cbeta = 0.0;
             s->cfrozen = 1;
@@ -887,10 +941,22 @@ int coarse_solve(ciecu_mgcg_s* M, cudaStream_t st) {
         coarse_first_kernel<K><<<fit_grid(coarse_first_kernel<K>, csr_threads<K>(), grid), csr_threads<K>(), 0,
                                  st>>>(Ac->args<double>(), M->dinvc, v, M->d_s, M->partials, M->counter);
         const int g = fit_grid(coarse_pipe_kernel<K>, csr_threads<K>(), grid);
-        for (int it = 0; it < M->options.coarseIterations; ++it)
+        const int gr = fit_grid(coarse_replace_kernel<K>, csr_threads<K>(), grid);
+        const int gp = fit_grid(coarse_product_kernel<K>, csr_threads<K>(), grid);
+        const int its = M->options.coarseIterations;
+        for (int it = 0; it < its; ++it) {
             coarse_pipe_kernel<K><<<g, csr_threads<K>(), 0, st>>>(Ac->args<double>(), M->dinvc, v, it & 1, M->d_s,
                                                                  M->partials, M->counter);
-        count_launch(1 + M->options.coarseIterations);
+            if ((it + 1) % kCoarseReplace == 0 && it + 1 < its) {
+                coarse_precondition_kernel<<<grid_of(m), kT, 0, st>>>(m, M->dinvc, v);
+                coarse_product_kernel<K><<<gp, csr_threads<K>(), 0, st>>>(Ac->args<double>(), v);
+                coarse_replace_kernel<K><<<gr, csr_threads<K>(), 0, st>>>(Ac->args<double>(), M->dinvc, v,
+                                                                         (it + 1) & 1, M->d_s, M->partials,
+                                                                         M->counter);
+                count_launch(3);
+            }
+        }
+        count_launch(1 + its);
         return CIECU_OK;
     });
 }

@@ -6,16 +6,19 @@
 //   (numeric/src/GaussLegendreQuadrature.cpp:82-175), then
 //   Assembler::addContribution (graph/impl/Assembler_impl.hpp:156-194).
 //
-// B200 design: the element -> CSR slot map (the reference's per-entry lower_bound)
-// is computed once per pattern on the device; cells are sorted by colour so that
-// one launch per colour scatters without atomics; the parametric gradient table
-// G[q][d][a] is shared by every cell and sits in shared memory.
+// B200 design: the element -> CSR map (the reference's per-entry lower_bound) is
+// computed once per pattern on the device, as the list of every matrix row's
+// incident cells in colour order and the positions of their columns in the row.
+// Each row is then summed and written by one group of lanes (row_gather_kernel):
+// no atomics, no launch per colour, and the order of every sum is the colours'.
+// The reference element's integral is shared by every cell and computed once.
 //
 //   K_e[a][b] = scale_e * sum_q w_q sum_d f_d G[q][d][a] G[q][d][b]
 //   reference convention (0): scale_e = kappa_e prod_d 2/h_d, f_d = 1
 //   physical convention  (1): scale_e = kappa_e prod_d h_d/2, f_d = (2/h_d)^2
 #include "assembly.cuh"
 #include "space.cuh"
+#include "sortscan.cuh"
 
 #include <cmath>
 #include <string>
@@ -72,71 +75,74 @@ namespace {
 
 constexpr int kT = 256;
 
-// slot[e][a][b] = index of column dof[b] in row dof[a]; -1 if absent.
-__global__ void slot_kernel(long ncells, int nb, const int* __restrict__ dofmap, int nrows,
-                            const int* __restrict__ rowptr, const int* __restrict__ col, int* __restrict__ slots,
-                            int* missing) {
-    const long total = ncells * nb * nb;
+// ---- incidence lists of the row gather (assembly.cuh) --------------------------
+
+// Incidences per row; a row number outside the matrix sets *missing.
+__global__ void incidence_count_kernel(long total, const int* __restrict__ dofmap, int nrows, int* __restrict__ count,
+                                       int* missing) {
     const long stride = static_cast<long>(gridDim.x) * blockDim.x;
     for (long t = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
-        const long e = t / (nb * nb);
-        const int ab = static_cast<int>(t - e * nb * nb);
-        const int row = dofmap[e * nb + ab / nb];
-        const int target = dofmap[e * nb + ab % nb];
-        if (row < 0 || row >= nrows) {
-            slots[t] = -1;
+        const int row = dofmap[t];
+        if (row < 0 || row >= nrows)
             atomicExch(missing, 1);
-            continue;
-        }
-        int lo = rowptr[row], hi = rowptr[row + 1];
-        const int end = hi;
+        else
+            atomicAdd(count + row, 1);
+    }
+}
+
+// Appends the incidences of one colour's cells to their rows: cells of a colour
+// share no row, so each row takes at most one per launch and a row's list is in
+// colour order whatever the schedule.
+__global__ void incidence_fill_kernel(long cells, int nb, const int* __restrict__ cellOrder,
+                                      const int* __restrict__ dofmap, int nrows, int* __restrict__ cursor,
+                                      int* __restrict__ inc) {
+    const long total = cells * nb;
+    const long stride = static_cast<long>(gridDim.x) * blockDim.x;
+    for (long t = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
+        const long le = t / nb;
+        const int ea = cellOrder[le] * nb + static_cast<int>(t - le * nb);
+        const int row = dofmap[ea];
+        if (row >= 0 && row < nrows) inc[atomicAdd(cursor + row, 1)] = ea;
+    }
+}
+
+// pos[i][b] = position of column dof[b] within the row of incidence i; an absent
+// column sets *missing.
+template <typename POS>
+__global__ void incidence_position_kernel(const int* __restrict__ d_total, int nb, const int* __restrict__ dofmap,
+                                          const int* __restrict__ inc, const int* __restrict__ rowptr,
+                                          const int* __restrict__ col, POS* __restrict__ pos, int* missing) {
+    const long total = static_cast<long>(*d_total) * nb;  // incidences of valid rows only
+    const long stride = static_cast<long>(gridDim.x) * blockDim.x;
+    for (long t = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
+        const long i = t / nb;
+        const int b = static_cast<int>(t - i * nb);
+        const int ea = inc[i];
+        const int row = dofmap[ea], target = dofmap[ea - ea % nb + b];
+        const int begin = rowptr[row], end = rowptr[row + 1];
+        int lo = begin, hi = end;
         while (lo < hi) {
             const int mid = lo + ((hi - lo) >> 1);
             if (col[mid] < target) lo = mid + 1;
             else hi = mid;
         }
         if (lo == end || col[lo] != target) {
-            slots[t] = -1;
+            pos[t] = 0;
             atomicExch(missing, 1);
         } else {
-            slots[t] = lo;
+            pos[t] = static_cast<POS>(lo - begin);
         }
     }
 }
 
-// One thread per (cell, a, b) of one colour: integrate and add into the CSR entry.
-__global__ void stiffness_scatter_kernel(long count, int nb, int dim, int nq, const int* __restrict__ cellOrder,
-                                         const double* __restrict__ gtab, const double* __restrict__ wq,
-                                         const double* __restrict__ kappa, double scale, double f0, double f1,
-                                         double f2, const int* __restrict__ slots, double* __restrict__ val) {
-    extern __shared__ double s_tab[];
-    const int tabSize = nq * dim * nb;
-    for (int k = threadIdx.x; k < tabSize; k += blockDim.x) s_tab[k] = gtab[k];
-    double* s_w = s_tab + tabSize;
-    for (int k = threadIdx.x; k < nq; k += blockDim.x) s_w[k] = wq[k];
-    __syncthreads();
-    const int nb2 = nb * nb;
-    const long total = count * nb2;
-    const double f[3] = {f0, f1, f2};
-    const long stride = static_cast<long>(gridDim.x) * blockDim.x;
-    for (long t = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
-        const long le = t / nb2;
-        const int ab = static_cast<int>(t - le * nb2);
-        const int a = ab / nb, b = ab - (ab / nb) * nb;
-        const int e = cellOrder[le];
-        double s = 0.0;
-        for (int q = 0; q < nq; ++q) {
-            const double* g = s_tab + q * dim * nb;
-            double gg = 0.0;
-            for (int d = 0; d < dim; ++d) gg = fma(f[d] * g[d * nb + a], g[d * nb + b], gg);
-            s = fma(s_w[q], gg, s);
-        }
-        const int slot = slots[static_cast<long>(e) * nb2 + ab];
-        // one rounding per contribution, written out so that the host restatement
-        // of this summation order reproduces the matrix bit for bit
-        val[slot] = fma(kappa[e] * scale, s, val[slot]);
-    }
-}
+// kappa_e scale times one shared element matrix.
+struct UniformSource {
+    const double* __restrict__ kappa;
+    double scale;
+    __device__ __forceinline__ bool adds(int) const { return true; }
+    __device__ __forceinline__ double coef(int e) const { return kappa[e] * scale; }
+    __device__ __forceinline__ const double* matrix(int, const double* K) const { return K; }
+};
 
 // Reference element matrix (kappa = 1) K1[a][b], computed once per call.
 __global__ void unit_element_kernel(int nb, int dim, int nq, const double* __restrict__ gtab,
@@ -146,10 +152,13 @@ __global__ void unit_element_kernel(int nb, int dim, int nq, const double* __res
     for (int ab = blockIdx.x * blockDim.x + threadIdx.x; ab < nb * nb; ab += gridDim.x * blockDim.x) {
         const int a = ab / nb, b = ab % nb;
         double s = 0.0;
-        for (int q = 0; q < nq; ++q) {
+#pragma unroll 8
+        for (int q = 0; q < nq; ++q) {  // the points' loads and products run ahead of the ordered sum
             const double* g = gtab + q * dim * nb;
             double gg = 0.0;
-            for (int d = 0; d < dim; ++d) gg = fma(f[d] * g[d * nb + a], g[d * nb + b], gg);
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (d < dim) gg = fma(f[d] * g[d * nb + a], g[d * nb + b], gg);
             s = fma(wq[q], gg, s);
         }
         K1[ab] = scale * s;
@@ -180,17 +189,55 @@ __global__ void element_gradient_kernel(long ncells, int nb, const int* __restri
     }
 }
 
+// Symmetric elimination in two sweeps that may run in any order: the entries of
+// boundary columns, found by reading the columns flat (a boundary entry (i, j) is
+// the diagonal one when it lies in row j), and the rows of boundary DoFs.
+// Bound by reading the columns once: 3D Q1 128^3, 228 MB; a thread per row that
+// reads its extents, its columns and their flags one after another took 109 us,
+// this kernel 91 us.
 template <typename V>
-__global__ void dirichlet_kernel(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
-                                 V* __restrict__ val, const uint8_t* __restrict__ bnd, double* __restrict__ rhs) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const bool bi = bnd[i] != 0;
-        for (int k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-            const int j = col[k];
-            if (bi || bnd[j]) val[k] = (i == j) ? V(1) : V(0);
-        }
-        if (rhs && bi) rhs[i] = 0.0;
+__global__ void __launch_bounds__(kT) dirichlet_kernel(int n, long nnz, long head, const int* __restrict__ rowptr,
+                                                       const int* __restrict__ col, V* __restrict__ val,
+                                                       const uint8_t* __restrict__ bnd, double* __restrict__ rhs) {
+    const long threads = static_cast<long>(gridDim.x) * kT;
+    const long t = static_cast<long>(blockIdx.x) * kT + threadIdx.x;
+    auto column = [&](long k, int j) {
+        if (bnd[j]) val[k] = (rowptr[j] <= k && k < rowptr[j + 1]) ? V(1) : V(0);
+    };
+    // `head` entries up to the first 16-byte boundary of col, then 16 bytes a load
+    const long groups = (nnz - head) >> 2;
+    const int4* __restrict__ col4 = reinterpret_cast<const int4*>(col + head);
+#pragma unroll 4
+    for (long g = t; g < groups; g += threads) {
+        const int4 j = __ldcs(col4 + g);
+        const long k = head + 4 * g;
+        column(k, j.x);
+        column(k + 1, j.y);
+        column(k + 2, j.z);
+        column(k + 3, j.w);
     }
+    if (t < head) column(t, col[t]);
+    const long tail = head + 4 * groups;
+    if (tail + t < nnz) column(tail + t, col[tail + t]);
+    // boundary rows: eight lanes each
+    const int l = threadIdx.x & 7;
+    for (long i = t >> 3; i < n; i += threads >> 3) {
+        if (!bnd[i]) continue;
+        for (int k = rowptr[i] + l; k < rowptr[i + 1]; k += 8) val[k] = col[k] == i ? V(1) : V(0);
+        if (rhs && l == 0) rhs[i] = 0.0;
+    }
+}
+
+template <typename V>
+int launch_dirichlet(const ciecu_csr_s* csr, const uint8_t* d_isBoundary, V* d_entries, double* d_rhs) {
+    const long toAligned = (16 - static_cast<long>(reinterpret_cast<uintptr_t>(csr->col) % 16)) % 16 / 4;
+    const long head = std::min<long>(toAligned, csr->nnz);
+    const long work = std::max<long>(csr->nnz / 4, 8L * csr->rows);
+    dirichlet_kernel<V><<<grid_for(work, kT, 8), kT, 0, csr->space->stream>>>(
+        csr->rows, csr->nnz, head, csr->rowptr, csr->col, d_entries, d_isBoundary, d_rhs);
+    count_launch();
+    CIECU_CHECK_LAUNCH("dirichlet_kernel");
+    return CIECU_OK;
 }
 
 // out = v with the entries of eliminated (boundary) DoFs set to zero.
@@ -207,7 +254,8 @@ __global__ void interior_kernel(int n, const double* __restrict__ v, const uint8
 // the local indices of the face's basis functions (the others vanish there).
 __global__ void penalty_matrix_kernel(long faces, int nb, int nf, int nqf, const int* __restrict__ faceCells,
                                       const int* __restrict__ onFace, const double* __restrict__ table,
-                                      const double* __restrict__ wq, double scale, const int* __restrict__ slots,
+                                      const double* __restrict__ wq, double scale, const int* __restrict__ dofmap,
+                                      const int* __restrict__ rowptr, const int* __restrict__ col,
                                       double* __restrict__ val) {
     const long total = faces * nf * nf;
     for (long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; t < total;
@@ -218,8 +266,15 @@ __global__ void penalty_matrix_kernel(long faces, int nb, int nf, int nqf, const
         double s = 0.0;
         for (int q = 0; q < nqf; ++q) s = fma(wq[q] * table[q * nb + a], table[q * nb + b], s);
         const long e = faceCells[f];
-        const int slot = slots[e * nb * nb + a * nb + b];
-        val[slot] = fma(scale, s, val[slot]);
+        const int row = dofmap[e * nb + a], target = dofmap[e * nb + b];
+        int lo = rowptr[row], hi = rowptr[row + 1];  // the entry is there: the plan's set-up checked it
+        const int end = hi;
+        while (lo < hi) {
+            const int mid = lo + ((hi - lo) >> 1);
+            if (col[mid] < target) lo = mid + 1;
+            else hi = mid;
+        }
+        if (lo < end) val[lo] = fma(scale, s, val[lo]);
     }
 }
 
@@ -249,8 +304,8 @@ __global__ void penalty_rhs_kernel(long faces, int nb, int nf, int nqf, const in
 
 int unit_element(const ciecu_assembly_s* P, double scale, const double f[3], double* d_out, cudaStream_t st) {
     const int nb2 = P->nb * P->nb;
-    unit_element_kernel<<<(nb2 + kT - 1) / kT, kT, 0, st>>>(P->nb, P->dim, P->nq, P->d_gtab, P->d_wq, scale, f[0],
-                                                           f[1], f[2], d_out);
+    unit_element_kernel<<<(nb2 + 63) / 64, 64, 0, st>>>(P->nb, P->dim, P->nq, P->d_gtab, P->d_wq, scale, f[0], f[1],
+                                                        f[2], d_out);
     count_launch();
     CIECU_CHECK_LAUNCH("unit_element_kernel");
     return CIECU_OK;
@@ -313,48 +368,100 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
                 gtab[(static_cast<size_t>(q) * dim + dd) * nb + a] = g;
             }
     }
-    // Colour order (counting sort of cells by colour).
+    // Colour order (counting sort of cells by colour); without colours the caller
+    // promises that no two cells share a DoF.
     std::vector<int> order_(static_cast<size_t>(ncells));
+    std::vector<long> colorOffsets;
     {
         int colors = 0;
         for (long e = 0; e < ncells; ++e) colors = std::max(colors, h_color ? h_color[e] + 1 : 1);
         std::vector<long> count(static_cast<size_t>(colors) + 1, 0);
         for (long e = 0; e < ncells; ++e) ++count[(h_color ? h_color[e] : 0) + 1];
         for (int c = 0; c < colors; ++c) count[c + 1] += count[c];
-        P->colorOffsets = count;
+        colorOffsets = count;
         std::vector<long> fill(count.begin(), count.end() - 1);
         for (long e = 0; e < ncells; ++e) order_[fill[h_color ? h_color[e] : 0]++] = static_cast<int>(e);
-        if (!h_color) P->colorOffsets = {0, ncells};  // single colour: caller promises no sharing
+        if (!h_color) colorOffsets = {0, ncells};
     }
-    cudaError_t e = cudaSuccess;
-    const size_t slotCount = static_cast<size_t>(ncells) * nb * nb;
-    e = cudaMalloc(&P->d_cellOrder, sizeof(int) * std::max<size_t>(1, order_.size()));
-    if (e == cudaSuccess) e = cudaMalloc(&P->d_slots, sizeof(int) * std::max<size_t>(1, slotCount));
+    P->colors = static_cast<int>(colorOffsets.size()) - 1;
+    P->maxRow = csr->maxRow;
+    P->posBytes = P->maxRow <= 256 ? 1 : (P->maxRow <= 65536 ? 2 : 4);
+    const long incidences = ncells * nb;
+    const long rows = csr->rows;
+    if (incidences >= (1L << 31)) {
+        delete P;
+        return fail(CIECU_ERR_ARGUMENT, "assembly_create: more than 2^31 element rows");
+    }
+    // set-up scratch: cells by colour, counts per row (then the append cursors), scan work
+    const size_t scratchInts = static_cast<size_t>(ncells) + static_cast<size_t>(rows) + 1 +
+                               static_cast<size_t>(scan_work(std::max<long>(rows, 1)));
+    int* scratch = nullptr;
+    cudaError_t e = cudaMalloc(&P->d_incStart, sizeof(int) * (static_cast<size_t>(rows) + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&P->d_inc, sizeof(int) * std::max<size_t>(1, static_cast<size_t>(incidences)));
+    if (e == cudaSuccess)
+        e = cudaMalloc(&P->d_pos, std::max<size_t>(1, static_cast<size_t>(incidences) * nb * P->posBytes));
     if (e == cudaSuccess) e = cudaMalloc(&P->d_gtab, sizeof(double) * gtab.size());
     if (e == cudaSuccess) e = cudaMalloc(&P->d_wq, sizeof(double) * wq.size());
+    if (e == cudaSuccess) e = cudaMalloc(&P->d_unit, sizeof(double) * nb * nb);
+    if (e == cudaSuccess) e = pool_alloc(&scratch, sizeof(int) * scratchInts, st);
+    int* d_order = scratch;
+    int* d_count = scratch + ncells;
+    int* d_scan = d_count + rows + 1;
     if (e == cudaSuccess && ncells)
-        e = cudaMemcpyAsync(P->d_cellOrder, order_.data(), sizeof(int) * order_.size(), cudaMemcpyHostToDevice, st);
+        e = cudaMemcpyAsync(d_order, order_.data(), sizeof(int) * order_.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(P->d_gtab, gtab.data(), sizeof(double) * gtab.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(P->d_wq, wq.data(), sizeof(double) * wq.size(), cudaMemcpyHostToDevice, st);
     int* d_missing = reinterpret_cast<int*>(csr->space->d_result);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_missing, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_count, 0, sizeof(int) * (static_cast<size_t>(rows) + 1), st);
     if (e != cudaSuccess) {
+        pool_release({scratch});
         ciecu_assembly_destroy(P);
         return cuda_fail(e, "assembly_create");
     }
-    if (slotCount) {
-        slot_kernel<<<grid_for(static_cast<long>(slotCount), kT, 8), kT, 0, st>>>(ncells, nb, d_dofmap, csr->rows,
-                                                                                  csr->rowptr, csr->col, P->d_slots,
-                                                                                  d_missing);
+    int status = CIECU_OK;
+    if (incidences) {
+        incidence_count_kernel<<<grid_for(incidences, kT, 8), kT, 0, st>>>(incidences, d_dofmap, csr->rows, d_count,
+                                                                           d_missing);
         count_launch();
+        if (rows) {
+            status = exclusive_scan(d_count, P->d_incStart, rows, d_scan, st);
+            if (status == CIECU_OK) {
+                e = cudaMemcpyAsync(d_count, P->d_incStart, sizeof(int) * rows, cudaMemcpyDeviceToDevice, st);
+                for (size_t c = 0; c + 1 < colorOffsets.size(); ++c) {
+                    const long begin = colorOffsets[c], count = colorOffsets[c + 1] - begin;
+                    if (count == 0) continue;
+                    incidence_fill_kernel<<<grid_for(count * nb, kT, 8), kT, 0, st>>>(count, nb, d_order + begin,
+                                                                                      d_dofmap, csr->rows, d_count,
+                                                                                      P->d_inc);
+                    count_launch();
+                }
+                auto positions = [&](auto* pos) {
+                    incidence_position_kernel<<<grid_for(incidences * nb, kT, 8), kT, 0, st>>>(
+                        P->d_incStart + rows, nb, d_dofmap, P->d_inc, csr->rowptr, csr->col, pos, d_missing);
+                    count_launch();
+                };
+                if (P->posBytes == 1) positions(static_cast<uint8_t*>(P->d_pos));
+                else if (P->posBytes == 2) positions(static_cast<uint16_t*>(P->d_pos));
+                else positions(static_cast<int*>(P->d_pos));
+            }
+        }
+        if (e == cudaSuccess) e = cudaGetLastError();
+    } else {
+        e = cudaMemsetAsync(P->d_incStart, 0, sizeof(int) * (static_cast<size_t>(rows) + 1), st);
     }
     int missing = 0;
-    e = cudaMemcpyAsync(&missing, d_missing, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&missing, d_missing, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    pool_release({scratch});
+    if (status != CIECU_OK) {
+        ciecu_assembly_destroy(P);
+        return status;
+    }
     if (e != cudaSuccess) {
         ciecu_assembly_destroy(P);
-        return cuda_fail(e, "assembly_create: slot map");
+        return cuda_fail(e, "assembly_create: incidence lists");
     }
     if (missing) {
         ciecu_assembly_destroy(P);
@@ -367,8 +474,10 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
 int ciecu_assembly_destroy(ciecu_assembly P) {
     if (!P) return CIECU_OK;
     // No access to P->csr (it may already be gone); cudaFree synchronises the device.
-    cudaFree(P->d_cellOrder);
-    cudaFree(P->d_slots);
+    cudaFree(P->d_incStart);
+    cudaFree(P->d_inc);
+    cudaFree(P->d_pos);
+    cudaFree(P->d_unit);
     cudaFree(P->d_gtab);
     cudaFree(P->d_wq);
     delete P;
@@ -377,7 +486,7 @@ int ciecu_assembly_destroy(ciecu_assembly P) {
 
 int ciecu_assembly_color_count(ciecu_assembly P, int* h_count) {
     CIECU_REQUIRE(P && h_count, "assembly_color_count: null argument");
-    *h_count = static_cast<int>(P->colorOffsets.size()) - 1;
+    *h_count = P->colors;
     return CIECU_OK;
 }
 
@@ -386,29 +495,13 @@ int ciecu_assemble_stiffness(ciecu_assembly P, const double* d_kappa, const doub
     CIECU_REQUIRE(P && d_kappa && h_cellSize && d_entries, "assemble_stiffness: null argument");
     CIECU_REQUIRE(convention == 0 || convention == 1, "assemble_stiffness: convention must be 0 or 1");
     cudaStream_t st = P->csr->space->stream;
-    if (!accumulate) CIECU_CUDA(cudaMemsetAsync(d_entries, 0, sizeof(double) * P->csr->nnz, st));
     double scale, f[3];
     convention_factors(P->dim, h_cellSize, convention, scale, f);
-    const size_t smem = sizeof(double) * (static_cast<size_t>(P->nq) * P->dim * P->nb + P->nq);
-    if (smem > 48 * 1024) {
-        static bool attr = false;
-        if (!attr) {
-            CIECU_CUDA(cudaFuncSetAttribute(stiffness_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            200 * 1024));
-            attr = true;
-        }
-    }
-    const int nb2 = P->nb * P->nb;
-    for (size_t c = 0; c + 1 < P->colorOffsets.size(); ++c) {
-        const long begin = P->colorOffsets[c], count = P->colorOffsets[c + 1] - begin;
-        if (count == 0) continue;
-        stiffness_scatter_kernel<<<grid_for(count * nb2, kT, 8), kT, smem, st>>>(
-            count, P->nb, P->dim, P->nq, P->d_cellOrder + begin, P->d_gtab, P->d_wq, d_kappa, scale, f[0], f[1], f[2],
-            P->d_slots, d_entries);
-        count_launch();
-        CIECU_CHECK_LAUNCH("stiffness_scatter_kernel");
-    }
-    return CIECU_OK;
+    // the reference element's sums, once per call: each contribution to an entry is
+    // fma(kappa_e scale, S[a][b], entry), one rounding, so that the host restatement
+    // of this summation order reproduces the matrix bit for bit
+    CIECU_TRY(unit_element(P, 1.0, f, P->d_unit, st));
+    return launch_row_gather<double>(P, UniformSource{d_kappa, scale}, P->d_unit, accumulate ? 1 : 0, d_entries, st);
 }
 
 int ciecu_element_gradient(ciecu_assembly P, const double* h_cellSize, int convention, const double* d_lambda,
@@ -594,7 +687,8 @@ int ciecu_assemble_dirichlet_penalty(ciecu_assembly P, const int32_t* h_cells, c
             const long faces = static_cast<long>(l.size());
             if (faces == 0) continue;
             penalty_matrix_kernel<<<grid_for(faces * nf * nf, kT, 8), kT, 0, st>>>(
-                faces, nb, nf, nqf, faceCells, onFace, table, wq, scale, P->d_slots, d_entries);
+                faces, nb, nf, nqf, faceCells, onFace, table, wq, scale, P->d_dofmap, P->csr->rowptr, P->csr->col,
+                d_entries);
             count_launch();
             if (d_boundaryValues) {
                 penalty_rhs_kernel<<<grid_for(faces * nf, kT, 8), kT, 0, st>>>(
@@ -617,22 +711,14 @@ int ciecu_dirichlet_eliminate(ciecu_csr csr, const uint8_t* d_isBoundary, double
     CIECU_REQUIRE(csr && d_isBoundary && d_entries, "dirichlet_eliminate: null argument");
     CIECU_REQUIRE(csr->rows == csr->cols, "dirichlet_eliminate: square matrix expected");
     if (csr->rows == 0) return CIECU_OK;
-    dirichlet_kernel<double><<<grid_for(csr->rows, kT, 8), kT, 0, csr->space->stream>>>(
-        csr->rows, csr->rowptr, csr->col, d_entries, d_isBoundary, d_rhs);
-    count_launch();
-    CIECU_CHECK_LAUNCH("dirichlet_kernel");
-    return CIECU_OK;
+    return launch_dirichlet<double>(csr, d_isBoundary, d_entries, d_rhs);
 }
 
 int ciecu_dirichlet_eliminate_f32(ciecu_csr csr, const uint8_t* d_isBoundary, float* d_entries32) {
     CIECU_REQUIRE(csr && d_isBoundary && d_entries32, "dirichlet_eliminate_f32: null argument");
     CIECU_REQUIRE(csr->rows == csr->cols, "dirichlet_eliminate_f32: square matrix expected");
     if (csr->rows == 0) return CIECU_OK;
-    dirichlet_kernel<float><<<grid_for(csr->rows, kT, 8), kT, 0, csr->space->stream>>>(
-        csr->rows, csr->rowptr, csr->col, d_entries32, d_isBoundary, nullptr);
-    count_launch();
-    CIECU_CHECK_LAUNCH("dirichlet_kernel");
-    return CIECU_OK;
+    return launch_dirichlet<float>(csr, d_isBoundary, d_entries32, nullptr);
 }
 
 }  // extern "C"

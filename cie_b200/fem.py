@@ -142,9 +142,9 @@ class Assembler:
 
     def assemble_embedded_f32(self, entries32, center, radius, alpha, maxDepth, kappa=None, convention=0,
                               accumulate=False, origin=None):
-        """The finite-cell matrix in FP32 (values in the same pattern): the cut
-        cells' contractions on the tensor cores in split BF16 with FP32
-        accumulation (ciecu_assemble_embedded_f32).  Returns the number of cut cells."""
+        """The finite-cell matrix in FP32 (values in the same pattern): the FP64
+        element matrices rounded to FP32 and summed
+        (ciecu_assemble_embedded_f32).  Returns the number of cut cells."""
         m = self.mesh
         h = np.ascontiguousarray(m.h, dtype=np.float64)
         cells = np.ascontiguousarray(m.cells, dtype=np.int32)

@@ -21,7 +21,7 @@ typedef struct ciecu_assembly_s* ciecu_assembly;
  * points (the reference uses order + 1, definitions.hpp:36), device DoF map
  * (ncells x (order+1)^dim, local index first-1-D-index fastest), host colours
  * (cells of one colour must share no DoF; NULL = one colour).  Builds the
- * element -> CSR-entry map once and fails with CIECU_ERR_PATTERN if an element
+ * lists of every row's incident cells and of their entries' positions once and fails with CIECU_ERR_PATTERN if an element
  * entry is missing from the pattern (CIE_OUT_OF_RANGE_CHECK of
  * Assembler_impl.hpp:178-180). */
 int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder, int64_t ncells,
@@ -29,8 +29,8 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
 int ciecu_assembly_destroy(ciecu_assembly plan);
 int ciecu_assembly_color_count(ciecu_assembly plan, int* h_count);
 
-/* d_entries (+)= sum_e K_e scattered into the CSR values, one launch per colour,
- * no atomics.  K_e = kappa_e * |det J^-1| * sum_q w_q G_q^T G_q with parametric
+/* d_entries (+)= sum_e K_e, one group of lanes per CSR row, no atomics, every entry
+ * summed in colour order.  K_e = kappa_e * |det J^-1| * sum_q w_q G_q^T G_q with parametric
  * gradients (convention 0, the reference's TransformedIntegrand.hpp:73-83 with
  * the inverse Jacobian passed by integration.cpp:92-97) or the physical
  * kappa_e * det J * sum_q w_q (J^-T G_q)^T (J^-T G_q) (convention 1).
@@ -51,9 +51,9 @@ int ciecu_assemble_stiffness(ciecu_assembly plan, const double* d_kappa, const d
  * homogeneous and inside, at the maximum depth, or homogeneous at depth 0, and
  * refined while not homogeneous.  K_e in FP64, convention as
  * ciecu_assemble_stiffness; d_kappa may be NULL (kappa = 1).  The plan's basis has
- * at most 64 functions.  The cut cells' Gram contractions run on the tensor cores
- * in FP64 (eight CTAs per cut cell, one per depth-1 tree node); cells of one
- * colour are scattered together, so the result does not depend on the schedule.
+ * at most 64 functions.  The points of a cut cell enter through its Legendre
+ * moments (one CTA per cut cell, FP64), and every CSR entry sums its cells in
+ * colour order, so the result does not depend on the schedule.
  * d_work: nb*nb doubles (kept for the interface; the call allocates its own
  * work arrays).  h_cutCells (may be NULL): the number of cut cells.  The call
  * synchronises the stream. */
@@ -64,10 +64,7 @@ int ciecu_assemble_embedded(ciecu_assembly plan, const double* d_kappa, const do
 
 /* The same finite-cell matrix in single precision, for inner or preconditioner
  * operators: d_entries32 (FP32 values in the plan's CSR pattern) (+)= the element
- * matrices with the Gram contraction B^T W B on the tensor cores in BF16 with
- * FP32 accumulation, each operand split into a high and a low BF16 part and the
- * three significant products summed (about 16 significant bits per product); the
- * regular cells add the FP64 standard-rule matrix rounded to FP32. */
+ * matrices, computed in FP64 as above and rounded to FP32 before they are summed. */
 int ciecu_assemble_embedded_f32(ciecu_assembly plan, const double* d_kappa, const double* h_cellSize,
                                 const int32_t* h_cells, const double* h_origin, const double* h_center, double radius,
                                 double alpha, int maxDepth, int convention, int accumulate, float* d_entries32,

@@ -395,14 +395,15 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
     // set-up scratch: cells by colour, counts per row (then the append cursors), scan work
     const size_t scratchInts = static_cast<size_t>(ncells) + static_cast<size_t>(rows) + 1 +
                                static_cast<size_t>(scan_work(std::max<long>(rows, 1)));
+    // plan and scratch from the library's pool: a plan of a size created before maps no new memory
     int* scratch = nullptr;
-    cudaError_t e = cudaMalloc(&P->d_incStart, sizeof(int) * (static_cast<size_t>(rows) + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&P->d_inc, sizeof(int) * std::max<size_t>(1, static_cast<size_t>(incidences)));
+    cudaError_t e = pool_alloc(&P->d_incStart, sizeof(int) * (static_cast<size_t>(rows) + 1), st);
+    if (e == cudaSuccess) e = pool_alloc(&P->d_inc, sizeof(int) * std::max<size_t>(1, static_cast<size_t>(incidences)), st);
     if (e == cudaSuccess)
-        e = cudaMalloc(&P->d_pos, std::max<size_t>(1, static_cast<size_t>(incidences) * nb * P->posBytes));
-    if (e == cudaSuccess) e = cudaMalloc(&P->d_gtab, sizeof(double) * gtab.size());
-    if (e == cudaSuccess) e = cudaMalloc(&P->d_wq, sizeof(double) * wq.size());
-    if (e == cudaSuccess) e = cudaMalloc(&P->d_unit, sizeof(double) * nb * nb);
+        e = pool_alloc(&P->d_pos, std::max<size_t>(1, static_cast<size_t>(incidences) * nb * P->posBytes), st);
+    if (e == cudaSuccess) e = pool_alloc(&P->d_gtab, sizeof(double) * gtab.size(), st);
+    if (e == cudaSuccess) e = pool_alloc(&P->d_wq, sizeof(double) * wq.size(), st);
+    if (e == cudaSuccess) e = pool_alloc(&P->d_unit, sizeof(double) * nb * nb, st);
     if (e == cudaSuccess) e = pool_alloc(&scratch, sizeof(int) * scratchInts, st);
     int* d_order = scratch;
     int* d_count = scratch + ncells;
@@ -454,7 +455,7 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
     int missing = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&missing, d_missing, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    pool_release({scratch});
+    cudaFreeAsync(scratch, st);  // back to the pool; the stream is idle here
     if (status != CIECU_OK) {
         ciecu_assembly_destroy(P);
         return status;
@@ -473,13 +474,8 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
 
 int ciecu_assembly_destroy(ciecu_assembly P) {
     if (!P) return CIECU_OK;
-    // No access to P->csr (it may already be gone); cudaFree synchronises the device.
-    cudaFree(P->d_incStart);
-    cudaFree(P->d_inc);
-    cudaFree(P->d_pos);
-    cudaFree(P->d_unit);
-    cudaFree(P->d_gtab);
-    cudaFree(P->d_wq);
+    // No access to P->csr (it may already be gone); pool_release synchronises the device.
+    pool_release({P->d_incStart, P->d_inc, P->d_pos, P->d_gtab, P->d_wq, P->d_unit});
     delete P;
     return CIECU_OK;
 }

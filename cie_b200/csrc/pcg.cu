@@ -13,6 +13,7 @@
 // fixed number of iterations can be replayed until the host sees the flag.
 #include "graph.cuh"
 #include "dia.cuh"
+#include "dia_persistent.cuh"
 #include "pcg.cuh"
 
 #include <string>
@@ -558,6 +559,60 @@ __global__ void __launch_bounds__(kPT, 1) pcg_persistent_kernel(PersistentArgs P
     }
 }
 
+// The iteration's decisions in the single launch over a DIA copy
+// (dia_persistent.cuh): the last blocks' code of K1 and K2.
+struct PcgCtl {
+    using Scalars = PcgScalars;
+    static __device__ bool start(PcgScalars& s, DpCommand& c) {
+        c.go = c.step = 1;
+        c.beta = s.beta;
+        c.first = s.iter == 0;
+        c.parity = static_cast<int>(s.iter & 1);
+        return s.done == 0;
+    }
+    static __device__ void afterProduct(PcgScalars& s, DpCommand& c, double pq) {
+        s.pq = pq;
+        if (!(0.0 < pq)) {
+            s.done = 3;
+            s.error = CIECU_ERR_BREAKDOWN;
+            s.errorKind = 2;
+            s.errorIter = s.iter;
+            s.absres = sqrt(s.rr);
+            s.relres = s.absres / s.r0;
+            c.go = 0;
+        } else {
+            c.alpha = s.alpha = s.rz / pq;
+        }
+    }
+    static __device__ void afterUpdate(PcgScalars& s, DpCommand& c, double rr, double rz) {
+        s.rr = rr;
+        c.beta = s.beta = rz / s.rz;
+        s.rz = rz;
+        // The norms are wanted near the stopping threshold and at the end of a launch:
+        // a square root and a division that every block waits for otherwise.
+        const double target = fmax(s.absTol, s.relTol * s.r0);
+        if (!(rr > 1.01 * target * target) || s.iter + 1 >= s.maxIter || s.chunkIter + 1 >= s.chunkLimit) {
+            s.absres = sqrt(rr);
+            s.relres = s.absres / s.r0;
+            if (float_less(s.absres, s.absTol) || float_less(s.relres, s.relTol)) s.done = 1;
+        }
+        if (s.done == 0) {
+            s.iter += 1;
+            if (s.iter >= s.maxIter) s.done = 2;
+        }
+        s.chunkIter += 1;
+        c.go = s.done == 0 && s.chunkIter < s.chunkLimit;
+        c.first = 0;
+        c.parity = static_cast<int>(s.iter & 1);
+    }
+};
+
+template <int ND, bool SYM, bool RESIDENT, bool PRECOND>
+__global__ void __launch_bounds__(dp_threads<RESIDENT>(), 1) pcg_dia_persistent_kernel(const __grid_constant__ DpArgs<double> P,
+                                                                           PcgScalars* s) {
+    dp_solve<double, ND, SYM, RESIDENT, PRECOND, PcgCtl>(P, s);
+}
+
 __global__ void fill_ones_kernel(long n, double* __restrict__ v) {
     const long stride = static_cast<long>(gridDim.x) * blockDim.x;
     for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) v[i] = 1.0;
@@ -630,6 +685,12 @@ struct ciecu_pcg_s {
     long long waitNs = 2000000000LL;  // bound of one grid-wide exchange wait (global timer)
     long long withholdExchange = 0;   // test hook of the timeout path (ciecu_pcg_debug_exchange)
     bool pinned = false;              // K1 schedule pinned by ciecu_pcg_set_schedule
+    // Single launch over the DIA copy (dia_persistent.cuh).
+    bool dp = false;                  // the last solve ran that way
+    int dpState = 0;                  // 0 not planned, 1 planned, 2 its windows do not fit
+    ciecu::DpArgs<double> dpArgs{};
+    ciecu::DpPlan dpPlan{};
+    ciecu::DpSlot* dpSlots = nullptr;
 };
 
 namespace ciecu {
@@ -780,17 +841,76 @@ int ensure_persistent_buffers(ciecu_pcg_s* S) {
     cudaError_t e = pool_alloc(&S->z, bytes, st);
     if (e == cudaSuccess) e = pool_alloc(&S->p2, bytes, st);
     if (e == cudaSuccess) e = pool_alloc(&S->slots, slotBytes, st);
+    if (e == cudaSuccess) e = pool_alloc(&S->dpSlots, kDpSlotBytes, st);
     if (e == cudaSuccess) e = pool_alloc(&S->abortFlag, sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(S->slots, 0, slotBytes, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S->dpSlots, 0, kDpSlotBytes, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(S->abortFlag, 0, sizeof(int), st);
     if (e != cudaSuccess) {
-        pool_release({S->z, S->p2, S->slots, S->abortFlag});
+        pool_release({S->z, S->p2, S->slots, S->dpSlots, S->abortFlag});
         S->z = S->p2 = nullptr;
         S->slots = nullptr;
+        S->dpSlots = nullptr;
         S->abortFlag = nullptr;
         return cuda_fail(e, "pcg: single-launch buffers");
     }
     S->epoch = 1;
+    return CIECU_OK;
+}
+
+// The single launch over the DIA copy, where its windows and the vectors q, r and x
+// of a block fit in shared memory (dp_plan): 3D Q1 up to about 88^3, 2D Q1 to 1,400^2.
+// Per iteration on B200 against the graph of three kernels (or, where it fitted, the
+// single launch over CSR rows): 2D Q1 256^2 8.0 against 12.9 us, 3D Q1 64^3 15.2
+// against 33 us.  Larger systems keep the graph: with the vectors in global memory a
+// single launch measured 119 against 113 us at 128^3.
+int plan_dia_persistent(ciecu_pcg_s* S) {
+    if (S->dpState != 0) return CIECU_OK;
+    int device = 0, optin = 0;
+    CIECU_CUDA(cudaGetDevice(&device));
+    CIECU_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    S->dpArgs = DpArgs<double>{};
+    S->dpArgs.A = S->dia;
+    S->dpPlan = dp_plan(S->dpArgs, sm_count(), static_cast<size_t>(optin));
+    S->dpState = S->dpPlan.grid > 0 ? 1 : 2;
+    return CIECU_OK;
+}
+
+int launch_dia_persistent(ciecu_pcg_s* S, cudaStream_t st) {
+    DpArgs<double> a = S->dpArgs;
+    a.A = S->dia;
+    a.dinv = S->dinv;
+    a.x = S->x;
+    a.r = S->r;
+    a.q = S->q;
+    a.z = S->z;
+    a.p0 = S->p;
+    a.p1 = S->p2;
+    a.slots = S->dpSlots;
+    a.abortFlag = S->abortFlag;
+    a.epoch0 = S->epoch;
+    a.waitNs = S->waitNs;
+    a.withholdEpoch = S->withholdExchange > 0 ? S->epoch + static_cast<unsigned long long>(S->withholdExchange) : 0ULL;
+    const DpPlan& plan = S->dpPlan;
+    CIECU_TRY(with_diagonals(S->dia.ndiag, [&](auto nd) -> int {
+        constexpr int ND = decltype(nd)::value;
+        auto pick = [&](auto resident, auto pre) {
+            constexpr bool RES = decltype(resident)::value, PRE = decltype(pre)::value;
+            return S->diaSym ? pcg_dia_persistent_kernel<ND, true, RES, PRE>
+                             : pcg_dia_persistent_kernel<ND, false, RES, PRE>;
+        };
+        using std::false_type;
+        using std::true_type;
+        auto* kernel = plan.resident ? (S->dinv ? pick(true_type{}, true_type{}) : pick(true_type{}, false_type{}))
+                                     : (S->dinv ? pick(false_type{}, true_type{}) : pick(false_type{}, false_type{}));
+        CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(plan.smem)));
+        void* params[] = {&a, &S->d_s};
+        CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(plan.grid),
+                                               dim3(plan.threads), params, plan.smem, st));
+        return CIECU_OK;
+    }));
+    count_launch();
     return CIECU_OK;
 }
 
@@ -846,7 +966,7 @@ int run_persistent(ciecu_pcg_s* S, cudaStream_t st) {
         S->h_s->chunkLimit = kLimit;
         CIECU_CUDA(cudaMemcpyAsync(&S->d_s->chunkIter, &S->h_s->chunkIter, 2 * sizeof(long long),
                                    cudaMemcpyHostToDevice, st));
-        CIECU_TRY(launch_persistent_any(S, st));
+        CIECU_TRY(S->dp ? launch_dia_persistent(S, st) : launch_persistent_any(S, st));
         S->epoch += 2 * kLimit + 2;  // exchanges of one launch never reuse an epoch
         int aborted = 0;
         CIECU_CUDA(cudaMemcpyAsync(&aborted, S->abortFlag, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1023,7 +1143,7 @@ int ciecu_pcg_destroy(ciecu_pcg S) {
     // synchronises the device before releasing memory.
     if (S->graph) cudaGraphExecDestroy(S->graph);
     pool_release({S->x, S->r, S->p, S->q, S->d_s, S->d_partials, S->d_counter, S->diaBuf, S->z, S->p2, S->slots,
-                  S->abortFlag, S->split});
+                  S->dpSlots, S->abortFlag, S->split});
     delete S->h_s;
     delete S;
     return CIECU_OK;
@@ -1031,7 +1151,7 @@ int ciecu_pcg_destroy(ciecu_pcg S) {
 
 int ciecu_pcg_info(ciecu_pcg S, int* spmvSchedule, int* deviceLoop) {
     CIECU_REQUIRE(S, "pcg_info: null solver");
-    if (spmvSchedule) *spmvSchedule = S->kernel;
+    if (spmvSchedule) *spmvSchedule = S->persistent && S->dp ? kDiaSchedule : S->kernel;
     if (deviceLoop) *deviceLoop = S->persistent ? 2 : (S->deviceLoop ? 1 : 0);
     return CIECU_OK;
 }
@@ -1094,11 +1214,22 @@ int ciecu_pcg_product(ciecu_pcg S, double inScale, const double* d_in, double ou
     }
     CIECU_TRY(ensure_tuned(A));
     bool persistent = false;
-    CIECU_TRY(use_persistent(S, &persistent));
+    S->dp = false;
+    const bool automatic = S->loopMode == 0 && !S->pinned;
+    if (!automatic) CIECU_TRY(use_persistent(S, &persistent));
+    if (automatic || persistent) {
+        CIECU_TRY(refresh_dia(S, st));
+        if (S->diaBuf) {
+            CIECU_TRY(plan_dia_persistent(S));
+            S->dp = S->dpState == 1;
+        }
+        if (S->dp) persistent = true;
+        else if (automatic) CIECU_TRY(use_persistent(S, &persistent));
+    }
     if (persistent) {
         CIECU_TRY(ensure_persistent_buffers(S));
     } else {
-        CIECU_TRY(refresh_dia(S, st));
+        if (!automatic) CIECU_TRY(refresh_dia(S, st));
         CIECU_TRY(tune_solver_spmv(S));
     }
     S->persistent = persistent;

@@ -17,6 +17,7 @@
 // single-system solver; K3 ends the loop when every system is finished.
 #include "graph.cuh"
 #include "pcg.cuh"
+#include "sell_persistent.cuh"
 #include "ciecu_batch.h"
 
 #include <algorithm>
@@ -45,6 +46,7 @@ struct BatchScalars {
     int updateX;
     int restart;  // an FP32 breakdown: no step, direction restarted after the replacement
     int breakdowns;
+    long long launchIter;  // iterations in the current single launch
 };
 
 struct BatchGlobal {
@@ -327,6 +329,69 @@ __global__ void __launch_bounds__(kT) batch_direction_kernel(const Tile* __restr
         for (int i = t.rowBegin + threadIdx.x; i < t.rowEnd; i += kT)
             p[i] = add_rn(mul_rn(p[i], beta), mul_rn(r[i], dinv[i]));
     }
+}
+
+// ---- single launch over sliced rows (sell_persistent.cuh) ---------------------
+//
+// The decisions of K1 and K2 for one system; a launch runs at most `limit`
+// iterations of each, so that the wait of a block for one still busy with an earlier
+// system stays short.
+struct BatchCtl {
+    using Scalars = BatchScalars;
+    struct Shared {
+        BatchGlobal* g;
+        long long maxIter, limit;
+        double absTol, relTol;
+    };
+    static __device__ bool start(BatchScalars& s, DpCommand& c, const Shared&) {
+        c.go = c.step = 1;
+        c.beta = s.beta;
+        c.first = s.iter == 0;
+        c.parity = static_cast<int>(s.iter & 1);
+        s.launchIter = 0;
+        return s.done == 0;
+    }
+    static __device__ void afterProduct(BatchScalars& s, DpCommand& c, const Shared&, double pq) {
+        s.pq = pq;
+        if (!(0.0 < pq)) {
+            s.done = 3;
+            s.errorKind = 2;
+            s.errorIter = s.iter;
+            s.absres = sqrt(s.rr);
+            s.relres = s.absres / s.r0;
+            c.go = 0;
+        } else {
+            c.alpha = s.alpha = s.rz / pq;
+        }
+    }
+    static __device__ void afterUpdate(BatchScalars& s, DpCommand& c, const Shared& g, double rr, double rz) {
+        s.rr = rr;
+        c.beta = s.beta = rz / s.rz;
+        s.rz = rz;
+        s.launchIter += 1;
+        const double target = fmax(g.absTol, g.relTol * s.r0);  // the norms only near the threshold
+        if (!(rr > 1.01 * target * target) || s.iter + 1 >= g.maxIter || s.launchIter >= g.limit) {
+            s.absres = sqrt(rr);
+            s.relres = s.absres / s.r0;
+            if (float_less(s.absres, g.absTol) || float_less(s.relres, g.relTol)) s.done = 1;
+        }
+        if (s.done == 0) {
+            s.iter += 1;
+            if (s.iter >= g.maxIter) s.done = 2;
+        }
+        c.go = s.done == 0 && s.launchIter < g.limit;
+        c.first = 0;
+        c.parity = static_cast<int>(s.iter & 1);
+    }
+    static __device__ void finish(BatchScalars& s, const Shared& g) {
+        if (s.done) atomicAdd(&g.g->finished, 1u);
+    }
+};
+
+__global__ void __launch_bounds__(kSpThreads, 1) batch_sliced_persistent_kernel(const __grid_constant__ SpArgs P,
+                                                                                BatchScalars* s,
+                                                                                BatchCtl::Shared shared) {
+    sp_solve<true, BatchCtl>(P, s, shared);
 }
 
 // ---- reliable-update form: FP32 iterations, FP64 residual replacements ------
@@ -656,6 +721,12 @@ struct ciecu_batch_s {
     unsigned* d_counter = nullptr;
     int chunk = 16;
     int grid = 1;
+    // Single launch over sliced rows (FP64).
+    std::vector<long long> rowOffsets;
+    ciecu::SpPlan sp{};
+    double* p1 = nullptr;
+    int* abortFlag = nullptr;
+    unsigned long long epoch = 1;
 };
 
 namespace ciecu {
@@ -791,6 +862,66 @@ int run_level(ciecu_batch_s* B, Level<T>& L, const BatchGlobal& g0, unsigned pre
         if (B->h_g->finished >= static_cast<unsigned>(B->systems)) break;
     }
     return CIECU_OK;
+}
+
+constexpr long long kBatchLaunchIterations = 4096;
+constexpr long long kBatchWaitNs = 20000000000LL;
+
+// The FP64 solve as single launches; *used = false when the matrix does not suit
+// (sp_build).  The right-hand side is in L.r on entry.  64 uneven Q2 systems of 16 to
+// 128 cells a side: 68 ms, by the graph of three kernels 137 ms.
+int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
+    *used = false;
+    cudaStream_t st = B->A->space->stream;
+    Level<double>& L = B->f64;
+    CIECU_TRY(sp_build(B->sp, B->A, B->rowOffsets, kSpRows, st));
+    if (B->sp.state != 1) return CIECU_OK;
+    if (!B->p1) {
+        cudaError_t e = pool_alloc(&B->p1, sizeof(double) * static_cast<size_t>(std::max<long>(1, B->n)), st);
+        if (e == cudaSuccess) e = pool_alloc(&B->abortFlag, sizeof(int), st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(B->abortFlag, 0, sizeof(int), st);
+        if (e != cudaSuccess) return cuda_fail(e, "batched pcg: single-launch buffers");
+    }
+    *used = true;
+    CIECU_TRY(sp_fill(B->sp, B->A, st));
+    *B->h_g = g0;
+    B->h_g->finished = 0;
+    CIECU_CUDA(cudaMemcpyAsync(B->d_g, B->h_g, sizeof(BatchGlobal), cudaMemcpyHostToDevice, st));
+    batch_init_kernel<double><<<B->grid, kT, 0, st>>>(B->d_tiles, B->ntiles, B->d_tileBegin, B->d_tileCount, L.r, L.dinv,
+                                                      L.p, B->d_s, B->d_g, B->d_partials, B->d_counter);
+    count_launch();
+    CIECU_CHECK_LAUNCH("batch_init_kernel");
+    SpArgs a = B->sp.args;
+    a.dinv = L.dinv;
+    a.x = L.x;
+    a.r = L.r;
+    a.z = L.p;  // z_0, from the set-up kernel
+    a.p0 = L.q;
+    a.p1 = B->p1;
+    a.abortFlag = B->abortFlag;
+    a.waitNs = kBatchWaitNs;
+    a.withholdEpoch = 0;
+    BatchCtl::Shared shared{B->d_g, g0.maxIter, kBatchLaunchIterations, g0.absTol, g0.relTol};
+    CIECU_CUDA(cudaFuncSetAttribute(batch_sliced_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(B->sp.smem)));
+    for (;;) {
+        int aborted = 0;
+        CIECU_CUDA(cudaMemcpyAsync(B->h_g, B->d_g, sizeof(BatchGlobal), cudaMemcpyDeviceToHost, st));
+        CIECU_CUDA(cudaMemcpyAsync(&aborted, B->abortFlag, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CIECU_CUDA(cudaStreamSynchronize(st));
+        if (aborted) {
+            CIECU_CUDA(cudaMemsetAsync(B->abortFlag, 0, sizeof(int), st));
+            CIECU_CUDA(cudaStreamSynchronize(st));
+            return fail(CIECU_ERR_TIMEOUT, "batched pcg: an exchange of the single-launch solve gave up waiting");
+        }
+        if (B->h_g->finished >= static_cast<unsigned>(B->systems)) return CIECU_OK;
+        a.epoch0 = B->epoch;
+        B->epoch += 2 * kBatchLaunchIterations + 2;
+        void* params[] = {&a, &B->d_s, &shared};
+        CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_sliced_persistent_kernel),
+                                               dim3(B->sp.grid), dim3(B->sp.threads), params, B->sp.smem, st));
+        count_launch();
+    }
 }
 
 // FP32 copies of the matrix values and of D^-1 and the FP32 vectors (first use),
@@ -963,6 +1094,7 @@ int ciecu_batch_create(ciecu_csr lhs, int64_t systems, const int64_t* h_rowOffse
     B->f64.A = lhs->args<double>();
     B->settings = settings;
     B->n = lhs->rows;
+    B->rowOffsets.assign(h_rowOffsets, h_rowOffsets + systems + 1);
     B->systems = static_cast<int>(systems);
     B->ntiles = static_cast<int>(tiles.size());
     cudaStream_t st = lhs->space->stream;
@@ -1031,6 +1163,8 @@ int ciecu_batch_destroy(ciecu_batch B) {
     if (B->f32.graph) cudaGraphExecDestroy(B->f32.graph);
     if (B->relGraph) cudaGraphExecDestroy(B->relGraph);
     if (B->side) cudaStreamDestroy(B->side);
+    sp_destroy(B->sp);
+    pool_release({B->p1, B->abortFlag});
     cudaFree(B->d_tiles);
     cudaFree(B->d_tileBegin);
     cudaFree(B->d_tileCount);
@@ -1057,7 +1191,8 @@ int ciecu_batch_info(ciecu_batch B, int* lanesPerRow, int* deviceLoop, int64_t* 
     const bool f32 = reliable || B->innerTolerance > 0.0;
     if (lanesPerRow) *lanesPerRow = f32 ? B->f32.lanes : B->f64.lanes;
     if (deviceLoop)
-        *deviceLoop = (reliable ? B->relDeviceLoop : (f32 ? B->f32.deviceLoop : B->f64.deviceLoop)) ? 1 : 0;
+        *deviceLoop =
+            (reliable ? B->relDeviceLoop : (f32 ? B->f32.deviceLoop : B->f64.deviceLoop || B->sp.state == 1)) ? 1 : 0;
     if (tiles) *tiles = B->ntiles;
     return CIECU_OK;
 }
@@ -1123,7 +1258,9 @@ int ciecu_batch_product(ciecu_batch B, double inScale, const double* d_in, doubl
         } else if (B->innerTolerance == 0.0) {
             // FP64: every system runs ConjugateGradients_impl.hpp:49-201 as it is
             CIECU_CUDA(cudaMemsetAsync(B->d_s, 0, sizeof(BatchScalars) * B->systems, st));
-            CIECU_TRY(run_level(B, L, g, 0u));
+            bool sliced = false;
+            CIECU_TRY(run_sliced(B, g, &sliced));
+            if (!sliced) CIECU_TRY(run_level(B, L, g, 0u));
             CIECU_CUDA(cudaMemcpyAsync(s.data(), B->d_s, sizeof(BatchScalars) * B->systems, cudaMemcpyDeviceToHost,
                                        st));
             CIECU_CUDA(cudaStreamSynchronize(st));

@@ -68,6 +68,17 @@ constexpr size_t kDpSlotBytes = sizeof(DpSlot) * 2 * 2 * kDpCopies * kDpMaxBlock
 
 enum DpHome { kDpQ = 1, kDpR = 2, kDpX = 4, kDpP = 8, kDpD = 16 };  // vectors kept in shared memory
 
+// The blocks that take part in an exchange and their words: value k of copy c of
+// block b in set s at words[s * setStride + k * valueStride + c * count + b].
+struct DpGroup {
+    DpSlot* words;
+    int setStride, valueStride;
+    int count, me;
+    int* abortFlag;
+    long long waitNs;
+    unsigned long long withholdEpoch;  // test hook: the last block never publishes this epoch (0: none)
+};
+
 template <typename V>
 struct DpArgs {
     DiaArgs<V> A;
@@ -119,15 +130,15 @@ __device__ __forceinline__ void dp_load(const DpSlot* s, double& v, unsigned lon
 
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-// Sums `mine` over the grid and runs decide(sums) in lane 0 of warp 0 of every
+// Sums `mine` over the group and runs decide(sums) in lane 0 of warp 0 of every
 // block; the command it leaves in shared memory is valid for the whole block on
 // return.  ORDER: the other blocks' stores before their publication are visible
 // afterwards.  (The exchange after S needs no such order: the stores of p_k become
 // visible with the exchange after U, and the published sum depends on every entry
 // the block has read, so no block can overwrite an entry before it was read.)  False when a wait gave up or another block aborted.
-template <int K, bool ORDER, typename V, typename Decide>
+template <int K, bool ORDER, typename Decide>
 __device__ __forceinline__ bool dp_exchange(const double (&mine)[K], int set, unsigned long long epoch,
-                                            const DpArgs<V>& P, double* s_red, int* s_ok, Decide&& decide) {
+                                            const DpGroup& P, double* s_red, int* s_ok, Decide&& decide) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -139,15 +150,15 @@ __device__ __forceinline__ bool dp_exchange(const double (&mine)[K], int set, un
         double sum[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) sum[k] = warp_sum(lane < warps ? s_red[k * 32 + lane] : 0.0);
-        const int G = gridDim.x;
-        DpSlot* words = P.slots + static_cast<size_t>(set) * 2 * kDpCopies * kDpMaxBlocks;
+        const int G = P.count;
+        DpSlot* words = P.words + static_cast<size_t>(set) * P.setStride;
         if (ORDER) fence_gpu();  // the block's stores, ordered before the barrier above, precede its words
-        if (lane < kDpCopies && !(epoch == P.withholdEpoch && blockIdx.x == G - 1)) {
+        if (lane < kDpCopies && !(epoch == P.withholdEpoch && P.me == G - 1)) {
 #pragma unroll
             for (int k = 0; k < K; ++k)
-                dp_store(words + (k * kDpCopies + lane) * kDpMaxBlocks + blockIdx.x, sum[k], epoch);
+                dp_store(words + k * P.valueStride + lane * G + P.me, sum[k], epoch);
         }
-        const DpSlot* mineCopy = words + (blockIdx.x % kDpCopies) * kDpMaxBlocks;
+        const DpSlot* mineCopy = words + (P.me % kDpCopies) * G;
         constexpr int N = kDpMaxBlocks / 32;
         double got[K][N];
 #pragma unroll
@@ -171,12 +182,12 @@ __device__ __forceinline__ bool dp_exchange(const double (&mine)[K], int set, un
             for (int k = 0; k < K; ++k)
 #pragma unroll
                 for (int j = 0; j < N; ++j)
-                    dp_load(mineCopy + k * kDpCopies * kDpMaxBlocks + lane + 32 * j, v[k][j], e[k][j]);
+                    if (32 * j < G) dp_load(mineCopy + k * P.valueStride + min(lane + 32 * j, G - 1), v[k][j], e[k][j]);
 #pragma unroll
             for (int k = 0; k < K; ++k)
 #pragma unroll
                 for (int j = 0; j < N; ++j)
-                    if (e[k][j] == epoch && (need & (1u << (k * N + j)))) {
+                    if (32 * j < G && e[k][j] == epoch && (need & (1u << (k * N + j)))) {
                         got[k][j] = v[k][j];
                         need &= ~(1u << (k * N + j));
                     }
@@ -272,6 +283,8 @@ __device__ __forceinline__ void dp_solve(const DpArgs<V>& P, typename Ctl::Scala
                 s_mat[d * R + i] = inside(rb + i + P.A.off[d]) ? entry(d, rb + i) : V(0);
     const bool edge = rb + P.minOff < 0 || rb + R - 1 + P.maxOff >= n;  // some operand lies outside the matrix
     __syncthreads();
+    const DpGroup group{P.slots, 2 * kDpCopies * kDpMaxBlocks, kDpCopies * kDpMaxBlocks, static_cast<int>(gridDim.x),
+                        static_cast<int>(blockIdx.x), P.abortFlag, P.waitNs, P.withholdEpoch};
     unsigned long long epoch = P.epoch0;
     bool aborted = false;
     while (true) {
@@ -347,7 +360,7 @@ __device__ __forceinline__ void dp_solve(const DpArgs<V>& P, typename Ctl::Scala
         else rows(std::false_type{});
         {
             const double mine[1] = {pq};
-            if (!dp_exchange<1, false>(mine, 0, ++epoch, P, s_red, &s_ok,
+            if (!dp_exchange<1, false>(mine, 0, ++epoch, group, s_red, &s_ok,
                                        [&](const double (&tot)[1]) { Ctl::afterProduct(s_scalars, s_cmd, tot[0]); })) {
                 aborted = true;
                 break;
@@ -389,7 +402,7 @@ __device__ __forceinline__ void dp_solve(const DpArgs<V>& P, typename Ctl::Scala
         }
         {
             const double mine[2] = {rr, rz};
-            if (!dp_exchange<2, true>(mine, 1, ++epoch, P, s_red, &s_ok, [&](const double (&tot)[2]) {
+            if (!dp_exchange<2, true>(mine, 1, ++epoch, group, s_red, &s_ok, [&](const double (&tot)[2]) {
                     Ctl::afterUpdate(s_scalars, s_cmd, tot[0], PRECOND ? tot[1] : tot[0]);
                 })) {
                 aborted = true;

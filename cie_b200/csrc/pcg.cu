@@ -15,7 +15,9 @@
 #include "dia.cuh"
 #include "dia_persistent.cuh"
 #include "pcg.cuh"
+#include "sell_persistent.cuh"
 
+#include <climits>
 #include <string>
 #include <tuple>
 #include <mutex>
@@ -613,6 +615,25 @@ __global__ void __launch_bounds__(dp_threads<RESIDENT>(), 1) pcg_dia_persistent_
     dp_solve<double, ND, SYM, RESIDENT, PRECOND, PcgCtl>(P, s);
 }
 
+struct SpPcgCtl {
+    using Scalars = PcgScalars;
+    struct Shared {};
+    static __device__ bool start(PcgScalars& s, DpCommand& c, Shared) { return PcgCtl::start(s, c); }
+    static __device__ void afterProduct(PcgScalars& s, DpCommand& c, Shared, double pq) {
+        PcgCtl::afterProduct(s, c, pq);
+    }
+    static __device__ void afterUpdate(PcgScalars& s, DpCommand& c, Shared, double rr, double rz) {
+        PcgCtl::afterUpdate(s, c, rr, rz);
+    }
+    static __device__ void finish(PcgScalars&, Shared) {}
+};
+
+template <bool PRECOND>
+__global__ void __launch_bounds__(kSpThreads, 1) pcg_sliced_persistent_kernel(const __grid_constant__ SpArgs P,
+                                                                              PcgScalars* s) {
+    sp_solve<PRECOND, SpPcgCtl>(P, s, SpPcgCtl::Shared{});
+}
+
 __global__ void fill_ones_kernel(long n, double* __restrict__ v) {
     const long stride = static_cast<long>(gridDim.x) * blockDim.x;
     for (long i = static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) v[i] = 1.0;
@@ -691,6 +712,9 @@ struct ciecu_pcg_s {
     ciecu::DpArgs<double> dpArgs{};
     ciecu::DpPlan dpPlan{};
     ciecu::DpSlot* dpSlots = nullptr;
+    // Single launch over sliced rows (sell_persistent.cuh), for matrices without a DIA copy.
+    bool sliced = false;              // the last solve ran that way
+    ciecu::SpPlan sp{};
 };
 
 namespace ciecu {
@@ -934,6 +958,27 @@ int launch_persistent(ciecu_pcg_s* S, cudaStream_t st) {
     return CIECU_OK;
 }
 
+int launch_sliced_persistent(ciecu_pcg_s* S, cudaStream_t st) {
+    SpArgs a = S->sp.args;
+    a.dinv = S->dinv;
+    a.x = S->x;
+    a.r = S->r;
+    a.z = S->z;
+    a.p0 = S->p;
+    a.p1 = S->p2;
+    a.abortFlag = S->abortFlag;
+    a.epoch0 = S->epoch;
+    a.waitNs = S->waitNs;
+    a.withholdEpoch = S->withholdExchange > 0 ? S->epoch + static_cast<unsigned long long>(S->withholdExchange) : 0ULL;
+    auto* kernel = S->dinv ? pcg_sliced_persistent_kernel<true> : pcg_sliced_persistent_kernel<false>;
+    CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(S->sp.smem)));
+    void* params[] = {&a, &S->d_s};
+    CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(S->sp.grid), dim3(S->sp.threads),
+                                           params, S->sp.smem, st));
+    count_launch();
+    return CIECU_OK;
+}
+
 // Lanes per row: as many as leave one lane group per row of the largest block,
 // and no more than the average row needs.
 template <bool PRE>
@@ -966,7 +1011,8 @@ int run_persistent(ciecu_pcg_s* S, cudaStream_t st) {
         S->h_s->chunkLimit = kLimit;
         CIECU_CUDA(cudaMemcpyAsync(&S->d_s->chunkIter, &S->h_s->chunkIter, 2 * sizeof(long long),
                                    cudaMemcpyHostToDevice, st));
-        CIECU_TRY(S->dp ? launch_dia_persistent(S, st) : launch_persistent_any(S, st));
+        CIECU_TRY(S->dp ? launch_dia_persistent(S, st)
+                  : S->sliced ? launch_sliced_persistent(S, st) : launch_persistent_any(S, st));
         S->epoch += 2 * kLimit + 2;  // exchanges of one launch never reuse an epoch
         int aborted = 0;
         CIECU_CUDA(cudaMemcpyAsync(&aborted, S->abortFlag, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1142,6 +1188,7 @@ int ciecu_pcg_destroy(ciecu_pcg S) {
     // No access to S->A: the matrix handle may already be gone.  pool_release
     // synchronises the device before releasing memory.
     if (S->graph) cudaGraphExecDestroy(S->graph);
+    sp_destroy(S->sp);
     pool_release({S->x, S->r, S->p, S->q, S->d_s, S->d_partials, S->d_counter, S->diaBuf, S->z, S->p2, S->slots,
                   S->dpSlots, S->abortFlag, S->split});
     delete S->h_s;
@@ -1214,7 +1261,7 @@ int ciecu_pcg_product(ciecu_pcg S, double inScale, const double* d_in, double ou
     }
     CIECU_TRY(ensure_tuned(A));
     bool persistent = false;
-    S->dp = false;
+    S->dp = S->sliced = false;
     const bool automatic = S->loopMode == 0 && !S->pinned;
     if (!automatic) CIECU_TRY(use_persistent(S, &persistent));
     if (automatic || persistent) {
@@ -1223,7 +1270,12 @@ int ciecu_pcg_product(ciecu_pcg S, double inScale, const double* d_in, double ou
             CIECU_TRY(plan_dia_persistent(S));
             S->dp = S->dpState == 1;
         }
-        if (S->dp) persistent = true;
+        if (!S->dp) {
+            CIECU_TRY(sp_build(S->sp, A, {0, n}, LONG_MAX, st));
+            S->sliced = S->sp.state == 1;
+            if (S->sliced) CIECU_TRY(sp_fill(S->sp, A, st));
+        }
+        if (S->dp || S->sliced) persistent = true;
         else if (automatic) CIECU_TRY(use_persistent(S, &persistent));
     }
     if (persistent) {

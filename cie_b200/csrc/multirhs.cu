@@ -19,6 +19,7 @@
 #include "dia.cuh"
 #include "graph.cuh"
 #include "pcg.cuh"
+#include "sell_tma.cuh"
 #include "ciecu_multi.h"
 
 #include <algorithm>
@@ -48,6 +49,7 @@ struct ColumnScalars {
     int updateX;  // ... and it folds the FP32 solution into the FP64 one
     int restart;  // an FP32 breakdown: no step, direction restarted after the replacement
     int breakdowns;
+    int moved;    // k = 32, FP64: K3 owes x this iteration's step
 };
 
 struct MultiGlobal {
@@ -57,6 +59,8 @@ struct MultiGlobal {
     double absTol, relTol;
     double delta;  // FP32-refined form: replacement trigger
     long long replacements;  // FP32-refined form: residual recomputations (launches of T)
+    int timeout;             // a bounded wait for a copy gave up
+    int pad;
 };
 
 // FP32 breakdowns (p^T A p <= 0 in single precision) a column may recover from
@@ -71,10 +75,10 @@ __device__ __forceinline__ void set_loop(cudaGraphConditionalHandle cond, unsign
 // Per-column sums of NV values over the grid.  Every thread holds the values of
 // its column (lane % KP); the CTA holding the last block gets the totals of
 // column c in thread c (c < k) and returns true.  partials: NV x grid x 32.
-template <int KP, int NV>
+template <int KP, int NV, int THREADS = kT>
 __device__ __forceinline__ bool column_reduce_last(const double (&mine)[NV], int k, double* partials,
                                                    unsigned* counter, double (&out)[NV]) {
-    __shared__ double s_red[NV][kT];
+    __shared__ double s_red[NV][THREADS];
     __shared__ bool s_last;
 #pragma unroll
     for (int v = 0; v < NV; ++v) s_red[v][threadIdx.x] = mine[v];
@@ -84,7 +88,7 @@ __device__ __forceinline__ bool column_reduce_last(const double (&mine)[NV], int
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             double acc = 0.0;
-            for (int t = c; t < kT; t += KP) acc += s_red[v][t];  // fixed order: warps, then slots
+            for (int t = c; t < THREADS; t += KP) acc += s_red[v][t];  // fixed order: warps, then slots
             partials[(static_cast<long>(v) * gridDim.x + blockIdx.x) * 32 + c] = acc;
         }
     }
@@ -101,13 +105,13 @@ __device__ __forceinline__ bool column_reduce_last(const double (&mine)[NV], int
         double acc = 0.0;
         const volatile double* p = partials + static_cast<long>(v) * gridDim.x * 32;
         if (c < k)
-            for (unsigned b = part; b < gridDim.x; b += kWarps) acc += p[static_cast<long>(b) * 32 + c];
+            for (unsigned b = part; b < gridDim.x; b += THREADS / 32) acc += p[static_cast<long>(b) * 32 + c];
         __syncthreads();
         s_red[v][threadIdx.x] = acc;
         __syncthreads();
         if (threadIdx.x < k) {
             double tot = 0.0;
-            for (int w = 0; w < kWarps; ++w) tot += s_red[v][w * 32 + threadIdx.x];
+            for (int w = 0; w < THREADS / 32; ++w) tot += s_red[v][w * 32 + threadIdx.x];
             out[v] = tot;
         }
     }
@@ -363,6 +367,25 @@ __global__ void __launch_bounds__(kT) multi_spmv_dia_kernel(DiaArgs<double> D, i
     }
 }
 
+// K2's decisions for one column: beta and the stopping test.
+__device__ __forceinline__ void column_update(ColumnScalars& s, const double (&tot)[2], MultiGlobal* g) {
+    s.moved = s.done ? 0 : 1;  // x still lacks this iteration's step where K3 takes it
+    if (!s.done) {
+        s.rr = tot[0];
+        s.beta = tot[1] / s.rz;
+        s.rz = tot[1];
+        s.absres = sqrt(tot[0]);
+        s.relres = s.absres / s.r0;
+        if (float_less(s.absres, g->absTol) || float_less(s.relres, g->relTol)) {
+            s.done = 1;
+        } else {
+            s.iter += 1;
+            if (s.iter >= g->maxIter) s.done = 2;
+        }
+        if (s.done) atomicAdd(&g->finished, 1u);
+    }
+}
+
 // K2: X += alpha P; R -= alpha Q; rr, rz; beta and the stopping test per column.
 template <int KP>
 __global__ void __launch_bounds__(kT) multi_update_kernel(long n, int k, double* __restrict__ X,
@@ -389,23 +412,8 @@ __global__ void __launch_bounds__(kT) multi_update_kernel(long n, int k, double*
         }
     }
     double mine[2] = {rr, rz}, tot[2];
-    if (column_reduce_last<KP, 2>(mine, k, partials, counter, tot) && threadIdx.x < k) {
-        ColumnScalars& s = S[threadIdx.x];
-        if (!s.done) {
-            s.rr = tot[0];
-            s.beta = tot[1] / s.rz;
-            s.rz = tot[1];
-            s.absres = sqrt(tot[0]);
-            s.relres = s.absres / s.r0;
-            if (float_less(s.absres, g->absTol) || float_less(s.relres, g->relTol)) {
-                s.done = 1;
-            } else {
-                s.iter += 1;
-                if (s.iter >= g->maxIter) s.done = 2;
-            }
-            if (s.done) atomicAdd(&g->finished, 1u);
-        }
-    }
+    if (column_reduce_last<KP, 2>(mine, k, partials, counter, tot) && threadIdx.x < k)
+        column_update(S[threadIdx.x], tot, g);
 }
 
 // K3: P = beta P + D^-1 R per running column; ends the loop when all are done.
@@ -505,45 +513,13 @@ __global__ void __launch_bounds__(kT) multi_spmv32_dia_kernel(DiaArgs<float> D, 
         column_pq(S[threadIdx.x], tot[0], g);
 }
 
-// K2 of the refined form.  IF: the handle of the replacement (set when any column
-// asks for one).
-template <int KP, bool COND>
-__global__ void __launch_bounds__(kT) multi_update32_kernel(long n, int k, float* __restrict__ X,
-                                                            float* __restrict__ R, const float* __restrict__ P,
-                                                            const float* __restrict__ Q,
-                                                            const float* __restrict__ dinv, ColumnScalars* S,
-                                                            MultiGlobal* g, double* partials, unsigned* counter,
-                                                            cudaGraphConditionalHandle replace) {
-    if (*reinterpret_cast<volatile unsigned*>(&g->finished) >= static_cast<unsigned>(k)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) set_loop<COND>(replace, 0);
-        return;
-    }
-    constexpr int RPW = 32 / KP;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int slot = lane / KP, c = lane % KP;
-    double rr = 0.0, rz = 0.0;
-    if (c < k && !S[c].done) {
-        const bool step = !S[c].restart;
-        const float alpha = static_cast<float>(S[c].alpha), malpha = -alpha;
-        const long stride = static_cast<long>(gridDim.x) * kWarps * RPW;
-#pragma unroll 4
-        for (long i = (static_cast<long>(blockIdx.x) * kWarps + warp) * RPW + slot; i < n; i += stride) {
-            const long e = i * k + c;
-            float ri = R[e];
-            if (step) {
-                X[e] = fmaf(alpha, P[e], X[e]);
-                ri = fmaf(malpha, Q[e], ri);
-                R[e] = ri;
-            }
-            rr = fma(static_cast<double>(ri), static_cast<double>(ri), rr);
-            rz = fma(static_cast<double>(ri), static_cast<double>(ri * dinv[i]), rz);
-        }
-    }
-    double mine[2] = {rr, rz}, tot[2];
+// K2's decisions in the last block: every running column's FP32 recursion and whether
+// the columns' residuals are replaced.
+template <bool COND>
+__device__ __forceinline__ void decide_replacement(const double (&tot)[2], int k, ColumnScalars* S, MultiGlobal* g,
+                                                   cudaGraphConditionalHandle replace) {
     __shared__ unsigned s_any;
     if (threadIdx.x == 0) s_any = 0u;
-    const bool last = column_reduce_last<KP, 2>(mine, k, partials, counter, tot);
-    if (!last) return;
     __syncthreads();
     // The replacement recomputes B - A X for all columns in one FP64 SpMM, so it is
     // taken by every running column at once, and only when it is due for the batch:
@@ -590,6 +566,44 @@ __global__ void __launch_bounds__(kT) multi_update32_kernel(long n, int k, float
         g->anyPending = s_any;
         set_loop<COND>(replace, s_any);
     }
+}
+
+// K2 of the refined form.  IF: the handle of the replacement (set when any column
+// asks for one).
+template <int KP, bool COND>
+__global__ void __launch_bounds__(kT) multi_update32_kernel(long n, int k, float* __restrict__ X,
+                                                            float* __restrict__ R, const float* __restrict__ P,
+                                                            const float* __restrict__ Q,
+                                                            const float* __restrict__ dinv, ColumnScalars* S,
+                                                            MultiGlobal* g, double* partials, unsigned* counter,
+                                                            cudaGraphConditionalHandle replace) {
+    if (*reinterpret_cast<volatile unsigned*>(&g->finished) >= static_cast<unsigned>(k)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) set_loop<COND>(replace, 0);
+        return;
+    }
+    constexpr int RPW = 32 / KP;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = lane / KP, c = lane % KP;
+    double rr = 0.0, rz = 0.0;
+    if (c < k && !S[c].done) {
+        const bool step = !S[c].restart;
+        const float alpha = static_cast<float>(S[c].alpha), malpha = -alpha;
+        const long stride = static_cast<long>(gridDim.x) * kWarps * RPW;
+#pragma unroll 4
+        for (long i = (static_cast<long>(blockIdx.x) * kWarps + warp) * RPW + slot; i < n; i += stride) {
+            const long e = i * k + c;
+            float ri = R[e];
+            if (step) {
+                X[e] = fmaf(alpha, P[e], X[e]);
+                ri = fmaf(malpha, Q[e], ri);
+                R[e] = ri;
+            }
+            rr = fma(static_cast<double>(ri), static_cast<double>(ri), rr);
+            rz = fma(static_cast<double>(ri), static_cast<double>(ri * dinv[i]), rz);
+        }
+    }
+    double mine[2] = {rr, rz}, tot[2];
+    if (column_reduce_last<KP, 2>(mine, k, partials, counter, tot)) decide_replacement<COND>(tot, k, S, g, replace);
 }
 
 // F: X64 += X32, X32 = 0 for the columns with a replacement due.
@@ -656,6 +670,7 @@ __device__ __forceinline__ void column_replace(ColumnScalars& s, const double (&
     }
     if (s.done || !s.pending) return;
     s.pending = 0;
+    s.alpha = 0.0;  // the fold took the step that K3 owes x (k = 32)
     s.refinements += 1;
     s.rr = tot[0];
     s.absres = rnorm;
@@ -946,6 +961,123 @@ __device__ __forceinline__ void quad_rows_dia3(const DiaArgs<V>& D, const T* __r
     }
 }
 
+// The triple pass in FP32 with the operand rows staged. What bounds the pass that
+// gathers its rows through L1 is L2: each of a row's 27 operand rows is wanted again
+// one line and one plane of the grid later, by other CTAs (1.2 KB from L2 for a row's
+// 128 bytes of result; 128^3, 32 columns: 378 us; staging 128 rows' operands one triple
+// at a time, as often read, 387 us; walking eight lines of the grid at a time for L1's
+// sake 441 us). Here a CTA takes kPlaneRows rows, and the operand rows of all triples
+// whose offsets lie close together (the three lines of a plane) are one run of
+// kPlaneRows + span rows, consecutive in memory: one bulk copy to shared memory, one more
+// for each of the triples' diagonals, the next plane's while this one is summed; 0.6 KB
+// a row from L2. (The same copies as 16-byte cp.async took 389 us: they fill the queue
+// that the sums' shared-memory reads go through.) Sums in the order of quad_rows_dia3.
+constexpr int kPlaneThreads = 768;
+constexpr int kPlaneRows = kPlaneThreads / 32 * 16;
+
+struct PlaneArgs {
+    int runs;                 // groups of triples
+    int first[12], count[12]; // triples of a run
+    int lo[12], rows[12];     // smallest middle offset; operand rows: kPlaneRows + span + 2
+    int xFloats, stageFloats; // a stage: operand rows, then the diagonals
+};
+
+template <typename Op>
+__device__ __forceinline__ void quad_rows_dia3_planes(const DiaArgs<float>& D, const PlaneArgs& A,
+                                                      const float* __restrict__ X, Op& op, int* timeout) {
+    extern __shared__ __align__(128) float s_planes[];
+    __shared__ uint64_t s_full[2];
+    __shared__ int s_late;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = lane / kQuadLanes, c0 = (lane % kQuadLanes) * 4;
+    const int n = D.nrows;
+    const int local = warp * 16 + 4 * slot;
+    if (threadIdx.x == 0) {
+        s_late = 0;
+        mbar_init(&s_full[0], 1);
+        mbar_init(&s_full[1], 1);
+        fence_mbarrier_init();
+    }
+    __syncthreads();
+    // Run g of the rows from `base` into buffer `buf`, which nobody reads any more: lane 0
+    // of warp 0 the operand rows, its next lanes a diagonal each; operand rows outside
+    // the matrix are zeroed by all threads.
+    auto issue = [&](long base, int g, int buf) {
+        float* xs = s_planes + buf * A.stageFloats;
+        const long first = base + A.lo[g] - 1, end = first + A.rows[g];
+        const long from = max(first, 0L), to = max(from, min(end, static_cast<long>(n)));
+        if (warp == 0) {
+            unsigned bytes = 0;
+            const float* src = nullptr;
+            float* dst = nullptr;
+            if (lane == 0) {
+                bytes = static_cast<unsigned>((to - from) * 128);
+                src = X + from * 32;
+                dst = xs + (from - first) * 32;
+            } else if (lane <= 3 * A.count[g]) {
+                bytes = static_cast<unsigned>(min(static_cast<long>(kPlaneRows), D.ld - base) * 4);
+                src = D.val + static_cast<long>(3 * A.first[g] + lane - 1) * D.ld + base;
+                dst = xs + A.xFloats + (lane - 1) * kPlaneRows;
+            }
+            const unsigned total = __reduce_add_sync(0xffffffffu, bytes);
+            if (lane == 0) mbar_arrive_expect_tx(&s_full[buf], total);
+            __syncwarp();
+            if (bytes) bulk_copy_g2s(dst, src, bytes, &s_full[buf]);
+        }
+        if (first < 0 || end > n) {
+            for (long u = threadIdx.x; u < A.rows[g] * 32L; u += kPlaneThreads) {
+                const long row = first + (u >> 5);
+                if (row < from || row >= to) xs[u] = 0.0f;
+            }
+            fence_proxy_async_smem();  // a later copy may write these places
+        }
+    };
+    const long stride = static_cast<long>(gridDim.x) * kPlaneRows;
+    long base = static_cast<long>(blockIdx.x) * kPlaneRows;
+    unsigned turn = 0;  // runs done: buffer turn mod 2
+    if (base < n) issue(base, 0, 0);
+    for (; base < n; base += stride) {
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) acc[i][u] = 0.0f;
+#pragma unroll 1
+        for (int g = 0; g < A.runs; ++g, ++turn) {
+            const int buf = turn & 1;
+            if (!mbar_wait_bounded(&s_full[buf], (turn >> 1) & 1)) s_late = 1;
+            __syncthreads();  // this run is complete, its zeros are written, and the other buffer is free
+            if (s_late) {     // the one copy in flight is this run's: waited for once more, then left
+                mbar_wait_bounded(&s_full[buf], (turn >> 1) & 1);
+                if (threadIdx.x == 0) atomicExch(timeout, 1);
+                return;
+            }
+            if (g + 1 < A.runs) issue(base, g + 1, buf ^ 1);
+            else if (base + stride < n) issue(base + stride, 0, buf ^ 1);
+            const float* xs = s_planes + buf * A.stageFloats;
+            const float* vs = xs + A.xFloats;
+            for (int t = 0; t < A.count[g]; ++t) {
+                const float* x0 = xs + (D.off[3 * (A.first[g] + t) + 1] - A.lo[g] + local) * 32 + c0;
+                float xr[6][4];
+#pragma unroll
+                for (int j = 0; j < 6; ++j) Quad<float>::load_plain(x0 + j * 32, xr[j]);
+#pragma unroll
+                for (int e = 0; e < 3; ++e) {
+                    float v[4];
+                    Quad<float>::load_plain(vs + (3 * t + e) * kPlaneRows + local, v);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) acc[i][u] = fmaf(v[i], xr[i + e][u], acc[i][u]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (base + local + i < n) op.quad(base + local + i, c0, acc[i]);
+    }
+}
+
 // The DIA pass of the k = 32 kernels: triples when the stencil has them.
 template <bool TRIPLES, typename V, typename T, typename Op>
 __device__ __forceinline__ void quad_rows_dia(const DiaArgs<V>& D, const T* __restrict__ X, Op& op) {
@@ -967,7 +1099,7 @@ __device__ __forceinline__ void quad_pass(const DiaArgs<V>& D, const T* __restri
 // Per-column totals of four-column partial sums (thread: columns c0 .. c0+3 of
 // its rows): summed over the warp's four row slots, then lane c takes column c,
 // and the column reduction of the row-per-warp kernels finishes the job.
-template <int NV>
+template <int NV, int THREADS = kT>
 __device__ __forceinline__ bool quad_reduce_last(double (&part)[NV][4], double* partials, unsigned* counter,
                                                  double (&out)[NV]) {
     const int lane = threadIdx.x & 31;
@@ -985,7 +1117,7 @@ __device__ __forceinline__ bool quad_reduce_last(double (&part)[NV][4], double* 
         const int u = lane & 3;
         mine[v] = u == 0 ? t[0] : u == 1 ? t[1] : u == 2 ? t[2] : t[3];
     }
-    return column_reduce_last<32, NV>(mine, 32, partials, counter, out);
+    return column_reduce_last<32, NV, THREADS>(mine, 32, partials, counter, out);
 }
 
 template <typename T>
@@ -1001,6 +1133,232 @@ struct PqQuad {
         for (int u = 0; u < 4; ++u) acc[0][u] = fma(static_cast<double>(pv[u]), static_cast<double>(sum[u]), acc[0][u]);
     }
 };
+
+// K2 and K3 for k = 32 with four columns per lane.  x is updated in K3, which reads the
+// old direction anyway, instead of in K2: ten instead of nine vector passes shrink to
+// eight (R, Q in, R out; X, P, R in, X, P out), in 16-byte accesses.  FP32, 128^3: the
+// row-per-warp pair took 410 + 156 us.
+constexpr int kVecRows = 2;  // rows a thread has in flight
+
+template <typename T, typename F>
+__device__ __forceinline__ void quad_vector_rows(long n, F&& f) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int perWarp = 32 / kQuadLanes;
+    const long stride = static_cast<long>(gridDim.x) * kWarps * perWarp;
+    for (long i = (static_cast<long>(blockIdx.x) * kWarps + warp) * perWarp + lane / kQuadLanes; i < n;
+         i += kVecRows * stride)
+        f(i, stride);
+}
+
+// Steps of this iteration's columns: whether and by how much x and r move.
+template <typename T>
+__device__ __forceinline__ void quad_steps(const ColumnScalars* S, int c0, bool (&run)[4], bool (&step)[4], T (&alpha)[4]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        run[u] = !S[c0 + u].done;
+        step[u] = run[u] && !S[c0 + u].restart;
+        alpha[u] = step[u] ? static_cast<T>(S[c0 + u].alpha) : T(0);
+    }
+}
+
+// R -= alpha Q; per column r^T r and r^T D^-1 r (FP64 sums).
+template <typename T>
+__device__ __forceinline__ void quad_residual_step(long n, T* __restrict__ R, const T* __restrict__ Q,
+                                                   const T* __restrict__ dinv, const ColumnScalars* S,
+                                                   double (&sums)[2][4]) {
+    const int c0 = (threadIdx.x & 31) % kQuadLanes * 4;
+    bool run[4], step[4];
+    T alpha[4];
+    quad_steps(S, c0, run, step, alpha);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) sums[0][u] = sums[1][u] = 0.0;
+    if (!(run[0] || run[1] || run[2] || run[3])) return;
+    const bool all = step[0] && step[1] && step[2] && step[3];
+    quad_vector_rows<T>(n, [&](long i0, long stride) {
+        T r[kVecRows][4], q[kVecRows][4], d[kVecRows];
+#pragma unroll
+        for (int v = 0; v < kVecRows; ++v) {
+            const long i = i0 + v * stride;
+            if (i >= n) continue;
+            Quad<T>::load_plain(R + i * 32 + c0, r[v]);
+            Quad<T>::load(Q + i * 32 + c0, q[v]);
+            d[v] = __ldg(dinv + i);
+        }
+#pragma unroll
+        for (int v = 0; v < kVecRows; ++v) {
+            const long i = i0 + v * stride;
+            if (i >= n) continue;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (all || step[u]) r[v][u] = fma(-alpha[u], q[v][u], r[v][u]);
+                if (run[u]) {
+                    const double ri = static_cast<double>(r[v][u]);
+                    sums[0][u] = fma(ri, ri, sums[0][u]);
+                    sums[1][u] = fma(ri, static_cast<double>(r[v][u] * d[v]), sums[1][u]);
+                }
+            }
+            Quad<T>::store(R + i * 32 + c0, r[v]);
+        }
+    });
+}
+
+// X += alpha P, then P = D^-1 R + beta P (P = D^-1 R when FRESH and beta is 0: after a
+// breakdown the old direction may not be finite) in the precision's rounding.
+template <typename T>
+__device__ __forceinline__ T quad_direction(T z, T beta, T p) {
+    if constexpr (sizeof(T) == 8) return __dadd_rn(__dmul_rn(p, beta), z);
+    else return fmaf(beta, p, z);
+}
+
+template <typename T, typename Moves>
+__device__ __forceinline__ void quad_direction_step(long n, T* __restrict__ X, T* __restrict__ P,
+                                                    const T* __restrict__ R, const T* __restrict__ dinv,
+                                                    const ColumnScalars* S, bool fresh, Moves&& moves) {
+    const int c0 = (threadIdx.x & 31) % kQuadLanes * 4;
+    bool turn[4], move[4];
+    T alpha[4], beta[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const ColumnScalars& s = S[c0 + u];
+        turn[u] = !s.done;
+        move[u] = moves(s);
+        alpha[u] = move[u] ? static_cast<T>(s.alpha) : T(0);
+        beta[u] = turn[u] ? static_cast<T>(s.beta) : T(0);
+    }
+    const bool anyTurn = turn[0] || turn[1] || turn[2] || turn[3], anyMove = move[0] || move[1] || move[2] || move[3];
+    if (!anyTurn && !anyMove) return;
+    quad_vector_rows<T>(n, [&](long i0, long stride) {
+        T x[kVecRows][4], p[kVecRows][4], r[kVecRows][4], d[kVecRows];
+#pragma unroll
+        for (int v = 0; v < kVecRows; ++v) {
+            const long i = i0 + v * stride;
+            if (i >= n) continue;
+            Quad<T>::load_plain(P + i * 32 + c0, p[v]);
+            if (anyMove) Quad<T>::load_plain(X + i * 32 + c0, x[v]);
+            if (anyTurn) Quad<T>::load(R + i * 32 + c0, r[v]);
+            d[v] = __ldg(dinv + i);
+        }
+#pragma unroll
+        for (int v = 0; v < kVecRows; ++v) {
+            const long i = i0 + v * stride;
+            if (i >= n) continue;
+            if (anyMove) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (move[u]) x[v][u] = fma(alpha[u], p[v][u], x[v][u]);
+                Quad<T>::store(X + i * 32 + c0, x[v]);
+            }
+            if (anyTurn) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (turn[u]) {
+                        const T z = sizeof(T) == 8 ? static_cast<T>(__dmul_rn(r[v][u], d[v])) : r[v][u] * d[v];
+                        p[v][u] = fresh && beta[u] == T(0) ? z : quad_direction<T>(z, beta[u], p[v][u]);
+                    }
+                Quad<T>::store(P + i * 32 + c0, p[v]);
+            }
+        }
+    });
+}
+
+// K2 (FP64): R -= alpha Q, the sums and the decisions; K3 takes the step of x.
+__global__ void __launch_bounds__(kT) multi_update_quad_kernel(long n, double* __restrict__ R,
+                                                               const double* __restrict__ Q,
+                                                               const double* __restrict__ dinv, ColumnScalars* S,
+                                                               MultiGlobal* g, double* partials, unsigned* counter) {
+    if (*reinterpret_cast<volatile unsigned*>(&g->finished) >= 32u) {  // an iteration past the last: x is complete
+        if (blockIdx.x == 0 && threadIdx.x < 32) S[threadIdx.x].moved = 0;
+        return;
+    }
+    double sums[2][4], tot[2];
+    quad_residual_step<double>(n, R, Q, dinv, S, sums);
+    if (quad_reduce_last<2>(sums, partials, counter, tot) && threadIdx.x < 32) column_update(S[threadIdx.x], tot, g);
+}
+
+template <bool COND>
+__global__ void __launch_bounds__(kT) multi_direction_quad_kernel(long n, double* __restrict__ X,
+                                                                  double* __restrict__ P,
+                                                                  const double* __restrict__ R,
+                                                                  const double* __restrict__ dinv,
+                                                                  const ColumnScalars* S, MultiGlobal* g,
+                                                                  cudaGraphConditionalHandle cond) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        g->chunkIter += 1;
+        const bool more = *reinterpret_cast<volatile unsigned*>(&g->finished) < 32u;
+        set_loop<COND>(cond, (more && g->chunkIter < g->chunkLimit) ? 1u : 0u);
+    }
+    quad_direction_step<double>(n, X, P, R, dinv, S, false, [](const ColumnScalars& s) { return s.moved != 0; });
+}
+
+// K2 of the refined form; the replacement's fold, or K3, takes the step of x.
+template <bool COND>
+__global__ void __launch_bounds__(kT) multi_update32_quad_kernel(long n, float* __restrict__ R,
+                                                                 const float* __restrict__ Q,
+                                                                 const float* __restrict__ dinv, ColumnScalars* S,
+                                                                 MultiGlobal* g, double* partials, unsigned* counter,
+                                                                 cudaGraphConditionalHandle replace) {
+    if (*reinterpret_cast<volatile unsigned*>(&g->finished) >= 32u) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) set_loop<COND>(replace, 0);
+        return;
+    }
+    double sums[2][4], tot[2];
+    quad_residual_step<float>(n, R, Q, dinv, S, sums);
+    if (quad_reduce_last<2>(sums, partials, counter, tot)) decide_replacement<COND>(tot, 32, S, g, replace);
+}
+
+// F for k = 32: X64 += X32 + alpha P, X32 = 0 for the columns with a replacement due.
+__global__ void __launch_bounds__(kT) multi_fold32_quad_kernel(long n, double* __restrict__ X64,
+                                                               float* __restrict__ X32, const float* __restrict__ P,
+                                                               const ColumnScalars* S, const MultiGlobal* g) {
+    if (!*reinterpret_cast<const volatile unsigned*>(&g->anyPending)) return;
+    const int c0 = (threadIdx.x & 31) % kQuadLanes * 4;
+    bool due[4], step[4];
+    float alpha[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const ColumnScalars& s = S[c0 + u];
+        due[u] = s.pending != 0;
+        step[u] = due[u] && !s.restart;
+        alpha[u] = step[u] ? static_cast<float>(s.alpha) : 0.0f;
+    }
+    if (!(due[0] || due[1] || due[2] || due[3])) return;
+    quad_vector_rows<float>(n, [&](long i0, long stride) {
+#pragma unroll
+        for (int v = 0; v < kVecRows; ++v) {
+            const long i = i0 + v * stride;
+            if (i >= n) continue;
+            float x[4], p[4];
+            double x64[4];
+            Quad<float>::load_plain(X32 + i * 32 + c0, x);
+            Quad<float>::load(P + i * 32 + c0, p);
+            Quad<double>::load_plain(X64 + i * 32 + c0, x64);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (due[u]) {
+                    x64[u] += static_cast<double>(step[u] ? fmaf(alpha[u], p[u], x[u]) : x[u]);
+                    x[u] = 0.0f;
+                }
+            Quad<double>::store(X64 + i * 32 + c0, x64);
+            Quad<float>::store(X32 + i * 32 + c0, x);
+        }
+    });
+}
+
+template <bool COND>
+__global__ void __launch_bounds__(kT) multi_direction32_quad_kernel(long n, float* __restrict__ X,
+                                                                    float* __restrict__ P,
+                                                                    const float* __restrict__ R,
+                                                                    const float* __restrict__ dinv,
+                                                                    const ColumnScalars* S, MultiGlobal* g,
+                                                                    cudaGraphConditionalHandle cond) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        g->chunkIter += 1;
+        const bool more = *reinterpret_cast<volatile unsigned*>(&g->finished) < 32u;
+        set_loop<COND>(cond, (more && g->chunkIter < g->chunkLimit) ? 1u : 0u);
+    }
+    quad_direction_step<float>(n, X, P, R, dinv, S, true,
+                               [](const ColumnScalars& s) { return !s.done && s.alpha != 0.0; });
+}
 
 struct ResidualQuad {  // R = B - A X
     const double* __restrict__ b;
@@ -1044,18 +1402,19 @@ struct TrueResidualQuad {
 
 // K1 for k = 32 over either format; FP64 (the plain form) or FP32 (the refined
 // form, whose breakdowns restart).
-template <typename MA, typename T, bool COND, bool TRIPLES>
+template <typename MA, typename T, bool COND, bool TRIPLES, int THREADS = kT>
 __device__ __forceinline__ void multi_spmv_quad(MA A, const T* __restrict__ P, T* __restrict__ Q, ColumnScalars* S,
                                                 MultiGlobal* g, double* partials, unsigned* counter,
-                                                cudaGraphConditionalHandle cond) {
+                                                cudaGraphConditionalHandle cond, const PlaneArgs* planes = nullptr) {
     if (*reinterpret_cast<volatile unsigned*>(&g->finished) >= 32u) {
         if (blockIdx.x == 0 && threadIdx.x == 0) set_loop<COND>(cond, 0);
         return;
     }
     PqQuad<T> op{P, Q, {{0.0, 0.0, 0.0, 0.0}}};
-    quad_pass<TRIPLES>(A, P, op);
+    if constexpr (THREADS != kT) quad_rows_dia3_planes(A, *planes, P, op, &g->timeout);
+    else quad_pass<TRIPLES>(A, P, op);
     double tot[1];
-    if (quad_reduce_last<1>(op.acc, partials, counter, tot) && threadIdx.x < 32) {
+    if (quad_reduce_last<1, THREADS>(op.acc, partials, counter, tot) && threadIdx.x < 32) {
         ColumnScalars& s = S[threadIdx.x];
         if (std::is_same<T, float>::value) {
             column_pq(s, tot[0], g);
@@ -1090,6 +1449,16 @@ __global__ void __launch_bounds__(kT, 3) multi_spmv_quad3_f32_kernel(DiaArgs<flo
                                                                      unsigned* counter,
                                                                      cudaGraphConditionalHandle cond) {
     multi_spmv_quad<DiaArgs<float>, float, COND, true>(A, P, Q, S, g, partials, counter, cond);
+}
+
+// ... and the staged one, one CTA per SM, where two stages fit in shared memory (planes
+// of up to about 190 nodes a line).
+template <bool COND>
+__global__ void __launch_bounds__(kPlaneThreads, 1)
+    multi_spmv_planes_f32_kernel(DiaArgs<float> A, const __grid_constant__ PlaneArgs planes,
+                                 const float* __restrict__ P, float* __restrict__ Q, ColumnScalars* S, MultiGlobal* g,
+                                 double* partials, unsigned* counter, cudaGraphConditionalHandle cond) {
+    multi_spmv_quad<DiaArgs<float>, float, COND, true, kPlaneThreads>(A, P, Q, S, g, partials, counter, cond, &planes);
 }
 
 template <typename MA, bool TRIPLES = false>
@@ -1202,6 +1571,8 @@ struct ciecu_multi_s {
     bool triples = false;  // the DIA offsets come in consecutive triples: the reuse pass (quad_rows_dia3)
     int formatPin = -1;    // -1: SpMM format by timing, 0: CSR, 1: the DIA copy (ciecu_multi_set_format)
     int gridQD3 = 1, gridQ32D3 = 1;
+    ciecu::PlaneArgs planes{};  // the staged FP32 triple pass
+    size_t planesSmem = 0;      // its shared memory; 0: its stages do not fit
 };
 
 namespace ciecu {
@@ -1214,6 +1585,14 @@ bool quad_enabled() {
         return !(v && v[0] == '0');
     }();
     return enabled;
+}
+
+// Resident blocks of a k = 32 vector kernel, or fewer when the rows are few; never more
+// than the partial sums of the reductions hold.
+template <typename K>
+int quad_grid(K* kernel, long n) {
+    const long rowsPerBlock = kWarps * (32 / kQuadLanes) * kVecRows;
+    return fit_grid(kernel, kT, (n + rowsPerBlock - 1) / rowsPerBlock);
 }
 
 template <bool COND>
@@ -1243,6 +1622,13 @@ int launch_multi_iteration(ciecu_multi_s* M, cudaStream_t st, cudaGraphCondition
             multi_spmv_kernel<KP, false, COND><<<M->grid, kT, 0, st>>>(M->A->args<double>(), M->k, M->p, M->q,
                                                                        M->d_s, M->d_g, M->d_partials, M->d_counter,
                                                                        cond);
+        if (M->quad) {
+            multi_update_quad_kernel<<<quad_grid(multi_update_quad_kernel, M->n), kT, 0, st>>>(
+                M->n, M->r, M->q, M->dinv, M->d_s, M->d_g, M->d_partials, M->d_counter);
+            multi_direction_quad_kernel<COND><<<quad_grid(multi_direction_quad_kernel<COND>, M->n), kT, 0, st>>>(
+                M->n, M->x, M->p, M->r, M->dinv, M->d_s, M->d_g, cond);
+            return CIECU_OK;
+        }
         multi_update_kernel<KP><<<M->gridV, kT, 0, st>>>(M->n, M->k, M->x, M->r, M->p, M->q, M->dinv, M->d_s,
                                                          M->d_g, M->d_partials, M->d_counter);
         multi_direction_kernel<KP, COND><<<M->gridV, kT, 0, st>>>(M->n, M->k, M->p, M->r, M->dinv, M->d_s, M->d_g,
@@ -1411,8 +1797,16 @@ int launch_multi_iteration32(ciecu_multi_s* M, cudaStream_t st, cudaGraph_t root
     CIECU_TRY(with_group(M->kp, [&](auto kk) -> int {
         constexpr int KP = decltype(kk)::value;
         if (M->quad && M->useDia && M->triples)
-            multi_spmv_quad3_f32_kernel<COND><<<M->gridQ32D3, kT, 0, st>>>(
-                M->diaF, M->p32, M->q32, M->d_s, M->d_g, M->d_partials, M->d_counter, cond);
+        {
+            if (M->planesSmem > 0)
+                multi_spmv_planes_f32_kernel<COND><<<fit_grid(multi_spmv_planes_f32_kernel<COND>, kPlaneThreads,
+                                                              (M->n + kPlaneRows - 1) / kPlaneRows, M->planesSmem),
+                                                     kPlaneThreads, M->planesSmem, st>>>(
+                    M->diaF, M->planes, M->p32, M->q32, M->d_s, M->d_g, M->d_partials, M->d_counter, cond);
+            else
+                multi_spmv_quad3_f32_kernel<COND><<<M->gridQ32D3, kT, 0, st>>>(
+                    M->diaF, M->p32, M->q32, M->d_s, M->d_g, M->d_partials, M->d_counter, cond);
+        }
         else if (M->quad && M->useDia)
             multi_spmv_quad_kernel<DiaArgs<float>, float, COND><<<M->gridQ32D, kT, 0, st>>>(
                 M->diaF, M->p32, M->q32, M->d_s, M->d_g, M->d_partials, M->d_counter, cond);
@@ -1431,7 +1825,11 @@ int launch_multi_iteration32(ciecu_multi_s* M, cudaStream_t st, cudaGraph_t root
         else
             multi_spmv32_kernel<KP, false, COND><<<M->grid32, kT, 0, st>>>(
                 args32(M), M->k, M->p32, M->q32, M->d_s, M->d_g, M->d_partials, M->d_counter, cond);
-        multi_update32_kernel<KP, COND><<<M->gridV, kT, 0, st>>>(M->n, M->k, M->x32, M->r32, M->p32, M->q32,
+        if (M->quad)
+            multi_update32_quad_kernel<COND><<<quad_grid(multi_update32_quad_kernel<COND>, M->n), kT, 0, st>>>(
+                M->n, M->r32, M->q32, M->dinv32, M->d_s, M->d_g, M->d_partials, M->d_counter, replace);
+        else
+            multi_update32_kernel<KP, COND><<<M->gridV, kT, 0, st>>>(M->n, M->k, M->x32, M->r32, M->p32, M->q32,
                                                                   M->dinv32, M->d_s, M->d_g, M->d_partials,
                                                                   M->d_counter, replace);
         return CIECU_OK;
@@ -1439,7 +1837,11 @@ int launch_multi_iteration32(ciecu_multi_s* M, cudaStream_t st, cudaGraph_t root
     auto replacement = [&](cudaStream_t s2) -> int {
         CIECU_TRY(with_group(M->kp, [&](auto kk) -> int {
             constexpr int KP = decltype(kk)::value;
-            multi_fold32_kernel<KP><<<M->gridV, kT, 0, s2>>>(M->n, M->k, M->x, M->x32, M->d_s, M->d_g);
+            if (M->quad)
+                multi_fold32_quad_kernel<<<quad_grid(multi_fold32_quad_kernel, M->n), kT, 0, s2>>>(
+                    M->n, M->x, M->x32, M->p32, M->d_s, M->d_g);
+            else
+                multi_fold32_kernel<KP><<<M->gridV, kT, 0, s2>>>(M->n, M->k, M->x, M->x32, M->d_s, M->d_g);
             return CIECU_OK;
         }));
         return launch_true_residual<false>(M, s2, M->graphB);
@@ -1450,11 +1852,53 @@ int launch_multi_iteration32(ciecu_multi_s* M, cudaStream_t st, cudaGraph_t root
         CIECU_TRY(replacement(st));
     CIECU_TRY(with_group(M->kp, [&](auto kk) -> int {
         constexpr int KP = decltype(kk)::value;
+        if (M->quad) {
+            multi_direction32_quad_kernel<COND><<<quad_grid(multi_direction32_quad_kernel<COND>, M->n), kT, 0, st>>>(
+                M->n, M->x32, M->p32, M->r32, M->dinv32, M->d_s, M->d_g, cond);
+            return CIECU_OK;
+        }
         multi_direction32_kernel<KP, COND><<<M->gridV, kT, 0, st>>>(M->n, M->k, M->p32, M->r32, M->dinv32, M->d_s,
                                                                     M->d_g, cond);
         return CIECU_OK;
     }));
     CIECU_CHECK_LAUNCH("multi-rhs refined iteration");
+    return CIECU_OK;
+}
+
+// Groups the triples into runs whose middle offsets lie within kPlaneRows of their
+// neighbours and sizes the stages.
+int plan_planes(ciecu_multi_s* M) {
+    M->planesSmem = 0;
+    const DiaArgs<float>& D = M->diaF;
+    if (!M->quad || !M->triples || D.ndiag < 3) return CIECU_OK;
+    int device = 0, optin = 0;
+    CIECU_CUDA(cudaGetDevice(&device));
+    CIECU_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    PlaneArgs A{};
+    int rows = 0, most = 0;
+    for (int t = 0; t < D.ndiag / 3; ++t) {
+        const int o = D.off[3 * t + 1];
+        if (A.runs == 0 || o - D.off[3 * (t - 1) + 1] > kPlaneRows) {
+            A.first[A.runs] = t;
+            A.lo[A.runs] = o;
+            ++A.runs;  // at most ndiag / 3 = 10 runs
+        }
+        const int g = A.runs - 1;
+        A.count[g] += 1;
+        A.rows[g] = kPlaneRows + (o - A.lo[g]) + 2;
+        rows = std::max(rows, A.rows[g]);
+        most = std::max(most, A.count[g]);
+    }
+    A.xFloats = rows * 32;
+    A.stageFloats = A.xFloats + 3 * most * kPlaneRows;
+    const size_t smem = 2 * sizeof(float) * static_cast<size_t>(A.stageFloats);
+    if (smem + 16 * 1024 > static_cast<size_t>(optin)) return CIECU_OK;  // static: the reductions
+    CIECU_CUDA(cudaFuncSetAttribute(multi_spmv_planes_f32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(smem)));
+    CIECU_CUDA(cudaFuncSetAttribute(multi_spmv_planes_f32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(smem)));
+    M->planes = A;
+    M->planesSmem = smem;
     return CIECU_OK;
 }
 
@@ -1499,6 +1943,7 @@ int prepare32(ciecu_multi_s* M, cudaStream_t st) {
             if (e != cudaSuccess) return cuda_fail(e, "multi: FP32 diagonal copy");
             a.val = M->dia32;
             M->diaF = a;
+            CIECU_TRY(plan_planes(M));
         }
         CIECU_TRY(dia_fill_f32(M->A, M->diaF, M->dia32, nullptr, st));
     } else {
@@ -1581,7 +2026,7 @@ int refined_solve(ciecu_multi_s* M, const double* B, std::vector<ColumnScalars>&
     for (;;) {
         CIECU_CUDA(cudaMemcpyAsync(M->h_g, M->d_g, sizeof(MultiGlobal), cudaMemcpyDeviceToHost, st));
         CIECU_CUDA(cudaStreamSynchronize(st));
-        if (M->h_g->finished >= static_cast<unsigned>(M->k)) break;
+        if (M->h_g->finished >= static_cast<unsigned>(M->k) || M->h_g->timeout) break;
         const long long before = M->h_g->replacements;
         M->h_g->chunkIter = 0;
         M->h_g->chunkLimit = limit;
@@ -1592,8 +2037,9 @@ int refined_solve(ciecu_multi_s* M, const double* B, std::vector<ColumnScalars>&
         CIECU_CUDA(cudaStreamSynchronize(st));
         count_launch(M->deviceLoop32 ? 3LL * M->h_g->chunkIter + 2LL * (M->h_g->replacements - before)
                                      : 5LL * M->chunk);
-        if (M->h_g->finished >= static_cast<unsigned>(M->k)) break;
+        if (M->h_g->finished >= static_cast<unsigned>(M->k) || M->h_g->timeout) break;
     }
+    if (M->h_g->timeout) return fail(CIECU_ERR_TIMEOUT, "multi: a bounded wait for a copy gave up");
     CIECU_CUDA(cudaMemcpyAsync(s.data(), M->d_s, sizeof(ColumnScalars) * M->k, cudaMemcpyDeviceToHost, st));
     CIECU_CUDA(cudaStreamSynchronize(st));
     return CIECU_OK;
@@ -1658,6 +2104,10 @@ int ciecu_multi_create(ciecu_csr lhs, int rhsCount, const double* d_inverseDiago
     }
     int widest = std::max({M->grid, M->gridV, M->gridQ, M->gridQD, M->gridQ32, M->gridQ32D, M->gridQD3,
                            M->gridQ32D3});
+    for (const void* k : {reinterpret_cast<const void*>(multi_update_quad_kernel),
+                          reinterpret_cast<const void*>(multi_update32_quad_kernel<true>),
+                          reinterpret_cast<const void*>(multi_update32_quad_kernel<false>)})
+        widest = std::max(widest, resident_blocks(k, kT, 0));
     with_group(M->kp, [&](auto kk) -> int {
         constexpr int KP = decltype(kk)::value;
         for (const void* k : {reinterpret_cast<const void*>(multi_spmv_dia_kernel<KP, true, true>),

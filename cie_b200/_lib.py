@@ -46,6 +46,9 @@ SIGNATURES = {
     "ciecu_space_destroy": (c_int, [P]),
     "ciecu_space_synchronize": (c_int, [P]),
     "ciecu_space_stream": (P, [P]),
+    "ciecu_space_enter": (c_int, [P, P]),
+    "ciecu_space_leave": (c_int, [P, P]),
+    "ciecu_csr_product": (c_int, [P, P, c_double, P, c_double, P]),
     "ciecu_alloc": (c_int, [P, ctypes.c_size_t, P]),
     "ciecu_free": (c_int, [P, P]),
     "ciecu_memcpy_h2d": (c_int, [P, P, P, ctypes.c_size_t]),

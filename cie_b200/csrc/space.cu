@@ -235,6 +235,8 @@ int ciecu_space_create(void* cudaStream, ciecu_space* out) {
             if (e != cudaSuccess) { status = cuda_fail(e, "cudaStreamCreate"); break; }
             space->ownsStream = true;
         }
+        e = cudaEventCreateWithFlags(&space->order, cudaEventDisableTiming);
+        if (e != cudaSuccess) { status = cuda_fail(e, "cudaEventCreate(order)"); break; }
         e = cudaMalloc(&space->d_partials, sizeof(double) * kMaxPartials * 4);
         if (e != cudaSuccess) { status = cuda_fail(e, "cudaMalloc(partials)"); break; }
         e = cudaMalloc(&space->d_counter, sizeof(unsigned) * 8);
@@ -256,11 +258,32 @@ int ciecu_space_create(void* cudaStream, ciecu_space* out) {
     return CIECU_OK;
 }
 
+int ciecu_space_enter(ciecu_space space, void* callerStream) {
+    CIECU_REQUIRE(space, "space_enter: null space");
+    const cudaStream_t caller = static_cast<cudaStream_t>(callerStream);
+    if (caller == space->stream) return CIECU_OK;
+    std::lock_guard<std::mutex> lock(space->orderMutex);
+    CIECU_CUDA(cudaEventRecord(space->order, caller));
+    CIECU_CUDA(cudaStreamWaitEvent(space->stream, space->order, 0));
+    return CIECU_OK;
+}
+
+int ciecu_space_leave(ciecu_space space, void* callerStream) {
+    CIECU_REQUIRE(space, "space_leave: null space");
+    const cudaStream_t caller = static_cast<cudaStream_t>(callerStream);
+    if (caller == space->stream) return CIECU_OK;
+    std::lock_guard<std::mutex> lock(space->orderMutex);
+    CIECU_CUDA(cudaEventRecord(space->order, space->stream));
+    CIECU_CUDA(cudaStreamWaitEvent(caller, space->order, 0));
+    return CIECU_OK;
+}
+
 int ciecu_space_destroy(ciecu_space space) {
     if (!space) return CIECU_OK;
     // Only a stream this space created is touched (a borrowed one may already be
     // gone); cudaFree synchronises the device.
     if (space->ownsStream && space->stream) cudaStreamSynchronize(space->stream);
+    if (space->order) cudaEventDestroy(space->order);
     cudaFree(space->d_partials);
     cudaFree(space->d_counter);
     cudaFree(space->d_result);

@@ -5,6 +5,7 @@
 #include "common.cuh"
 
 #include <atomic>
+#include <mutex>
 
 struct ciecu_space_s {
     cudaStream_t stream = nullptr;
@@ -16,6 +17,10 @@ struct ciecu_space_s {
     unsigned* d_counter = nullptr;
     double* d_result = nullptr;
     double* h_result = nullptr;
+    // Orders the space's stream with a caller's (ciecu_space_enter / leave): an event that is
+    // recorded and waited for under the lock, so that threads may share it.
+    cudaEvent_t order = nullptr;
+    std::mutex orderMutex;
 };
 
 namespace ciecu {

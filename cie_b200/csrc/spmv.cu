@@ -337,6 +337,19 @@ int ciecu_csr_spmv_f32(ciecu_csr csr, float inScale, const float* d_in, float ou
     return launch_spmv<float>(csr, csr->kernel, nullptr, 0, inScale, d_in, outScale, d_out);
 }
 
+int ciecu_csr_product(ciecu_csr csr, void* callerStream, double inScale, const void* d_in, double outScale,
+                      void* d_out) {
+    CIECU_REQUIRE(csr, "csr_product: null matrix");
+    CIECU_TRY(ciecu_space_enter(csr->space, callerStream));
+    const int status =
+        csr->valueType == CIECU_F64
+            ? ciecu_csr_spmv_f64(csr, inScale, static_cast<const double*>(d_in), outScale, static_cast<double*>(d_out))
+            : ciecu_csr_spmv_f32(csr, static_cast<float>(inScale), static_cast<const float*>(d_in),
+                                 static_cast<float>(outScale), static_cast<float*>(d_out));
+    if (status != CIECU_OK) return status;
+    return ciecu_space_leave(csr->space, callerStream);
+}
+
 int ciecu_csr_masked_spmv_f64(ciecu_csr csr, const uint16_t* d_mask, uint16_t threshold, double inScale,
                               const double* d_in, double outScale, double* d_out) {
     CIECU_TRY(spmv_checks(csr, d_in, d_out, CIECU_F64));

@@ -68,6 +68,11 @@ int ciecu_space_create(void* cudaStream, ciecu_space* out);
 int ciecu_space_destroy(ciecu_space space);
 int ciecu_space_synchronize(ciecu_space space);
 void* ciecu_space_stream(ciecu_space space);
+/* Order with a caller's stream: work submitted to the space after `enter` follows what
+ * the caller's stream holds, work submitted there after `leave` follows the space's.
+ * Callable from several threads. */
+int ciecu_space_enter(ciecu_space space, void* callerStream);
+int ciecu_space_leave(ciecu_space space, void* callerStream);
 
 /* SYCLSpace::makeVector / DeviceMemory (cieutils/packages/concurrency/inc/sycl.hpp:33-71) */
 int ciecu_alloc(ciecu_space space, size_t bytes, void** d_out);
@@ -126,6 +131,9 @@ int ciecu_csr_spmv_f32(ciecu_csr csr, float inScale, const float* d_in, float ou
 /* MaskedCSROperator<int,double,double,uint16_t>::product (MaskedCSROperator.cpp:37-118):
  * rows/columns with mask >= threshold are excluded; masked rows receive
  * combine(inScale, out, outScale, 0) (CPU semantics, :51-66). */
+/* enter, ciecu_csr_spmv_f64 or _f32 by the matrix's value type, and leave. */
+int ciecu_csr_product(ciecu_csr csr, void* callerStream, double inScale, const void* d_in, double outScale,
+                      void* d_out);
 int ciecu_csr_masked_spmv_f64(ciecu_csr csr, const uint16_t* d_mask, uint16_t threshold,
                               double inScale, const double* d_in, double outScale, double* d_out);
 

@@ -17,6 +17,7 @@
 #include "dia.cuh"
 #include "graph.cuh"
 #include "pcg.cuh"
+#include "smoother_slices.cuh"
 
 #include <cooperative_groups.h>
 
@@ -251,15 +252,116 @@ __global__ void __launch_bounds__(kVectorThreads)
     vector_rows<float, float, short, VS, kVectorThreads, false>(A, z, op);
 }
 
-// 16-bit offsets col - row of every entry; bad[0] counts offsets outside int16.
+// ---- the FP32 smoother over the sliced copy (smoother_slices.cuh) --------------
+//
+// A sweep of degree k is its start (fused into the pass before it) and k - 1 of these.
+
+struct SlExpired {  // a bounded wait gave up: ends the solve
+    MgScalars* s;
+    __device__ __forceinline__ void expired() const {
+        s->done = 3;
+        s->error = CIECU_ERR_TIMEOUT;
+        s->errorKind = 3;
+        s->errorIter = s->iter;
+    }
+};
+
+// A Chebyshev step.  The last step of the sweep leaves out = x (AFTER = 1), or ends the
+// cycle with z = out + x in FP64 (AFTER = 2), instead of the sweep's own vectors.
+template <int AFTER>
+struct SlChebStep : SlExpired {
+    struct Pre {
+        float r, dinv, x, z;
+    };
+    const float* __restrict__ dinv;
+    float c1, c2;
+    float* __restrict__ r;
+    float* __restrict__ dnew;
+    float* __restrict__ x;
+    float* __restrict__ out;
+    double* __restrict__ z;
+    __device__ __forceinline__ Pre pre(int i) const { return Pre{r[i], dinv[i], x[i], AFTER == 2 ? out[i] : 0.f}; }
+    __device__ __forceinline__ void post(int i, const Pre& p, float sum, float d) const {
+        const float ri = p.r - sum;
+        const float di = c1 * d + c2 * p.dinv * ri;
+        const float xi = p.x + di;
+        if (AFTER == 0) {
+            r[i] = ri;
+            dnew[i] = di;
+            x[i] = xi;
+        } else if (AFTER == 1) {
+            out[i] = xi;
+        } else {
+            z[i] = static_cast<double>(p.z + xi);
+        }
+    }
+};
+
+// in - A z: in FP64 for the restriction, or as the start of the second sweep.
+template <bool START>
+struct SlResidual : SlExpired {
+    struct Pre {
+        float in, dinv;
+    };
+    const float* __restrict__ in;
+    const float* __restrict__ dinv;
+    float theta;
+    double* __restrict__ t;
+    float* __restrict__ r;
+    float* __restrict__ d;
+    float* __restrict__ x;
+    __device__ __forceinline__ Pre pre(int i) const { return Pre{in[i], START ? dinv[i] : 0.f}; }
+    __device__ __forceinline__ void post(int i, const Pre& p, float sum, float) const {
+        const float ri = p.in - sum;
+        if (START) {
+            r[i] = ri;
+            const float di = p.dinv * ri / theta;
+            d[i] = di;
+            x[i] = di;
+        } else {
+            t[i] = static_cast<double>(ri);
+        }
+    }
+};
+
+template <typename Op>
+__global__ void __launch_bounds__(kSlThreads) sl_kernel(SlArgs A, const float* __restrict__ v, Op op) {
+    sl_rows(A, v, op);
+}
+
+// The cycle's residual in FP32 and the start of its first sweep.
+__global__ void sl_start_kernel(long n, const double* __restrict__ in, const float* __restrict__ dinv, float theta,
+                                float* __restrict__ r32, float* __restrict__ r, float* __restrict__ d,
+                                float* __restrict__ x) {
+    for (long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<long>(gridDim.x) * blockDim.x) {
+        const float ri = static_cast<float>(in[i]);
+        r32[i] = ri;
+        r[i] = ri;
+        const float di = dinv[i] * ri / theta;
+        d[i] = di;
+        x[i] = di;
+    }
+}
+
+// 16-bit offsets col - row of every entry, and the smallest and largest of them and of 0
+// (range[0], range[1], started at 0); offsets outside int16 show there.
 __global__ void offsets16_kernel(int n, const int* __restrict__ rowptr, const int* __restrict__ col,
-                                 short* __restrict__ out, unsigned* bad) {
+                                 short* __restrict__ out, int* range) {
+    int lo = 0, hi = 0;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
         for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) {
             const int d = col[k] - r;
-            if (d < -32768 || d > 32767) atomicAdd(bad, 1u);
+            lo = min(lo, d);
+            hi = max(hi, d);
             out[k] = static_cast<short>(d);
         }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(range, lo);
+        atomicMax(range + 1, hi);
+    }
 }
 
 // Calls f(std::integral_constant<int, VS>) for VS in {4, 8, 16, 32}.
@@ -691,6 +793,7 @@ struct ciecu_mgcg_s {
     float *dinv32 = nullptr, *r32 = nullptr, *z32 = nullptr, *t32 = nullptr, *cheb32 = nullptr;  // FP32 smoothing
     short* col16 = nullptr;  // 16-bit column offsets of the FP32 smoother matrix (when its bandwidth allows)
     int lanes16 = 8;         // lanes per row of the 16-bit-offset smoother kernels (timed at creation)
+    ciecu::SlPlan slices;    // the sliced copy of the smoother matrix (blocks = 0: the CSR kernels)
     double *rc = nullptr, *cx = nullptr, *cr = nullptr, *cz = nullptr, *cp = nullptr, *cq = nullptr;
     double *cu = nullptr, *cw = nullptr, *cs = nullptr, *cm0 = nullptr, *cm1 = nullptr;
     ciecu::MgScalars* d_s = nullptr;
@@ -743,15 +846,70 @@ int residual32(ciecu_mgcg_s* M, const float* z, float* t, cudaStream_t st) {
     return CIECU_OK;
 }
 
+int coarse_solve(ciecu_mgcg_s* M, cudaStream_t st);
+
+template <typename Op>
+int sl_launch(const ciecu_mgcg_s* M, const float* v, const Op& op, cudaStream_t st) {
+    sl_kernel<Op><<<M->slices.blocks, kSlThreads, M->slices.smem, st>>>(M->slices.args, v, op);
+    count_launch();
+    return CIECU_OK;
+}
+
+// The vectors' entries in the work arrays: n rounded up to 16 bytes of floats.
+long padded(long n) { return (n + 3) / 4 * 4; }
+
+// The steps of a sweep whose start is in M->cheb32; the last one leaves z32 = x, or
+// z = z32 + x (END).
+template <bool END>
+int sl_sweep(ciecu_mgcg_s* M, cudaStream_t st) {
+    const long ld = padded(M->n);
+    float *r = M->cheb32, *da = r + ld, *db = r + 2 * ld, *x = r + 3 * ld;
+    const double theta = 0.5 * (M->lambdaMax + M->lambdaMin);
+    const double delta = 0.5 * (M->lambdaMax - M->lambdaMin);
+    const double sigma = theta / delta;
+    double rho = 1.0 / sigma;
+    for (int k = 1; k < M->options.degree; ++k) {
+        const double rhoNew = 1.0 / (2.0 * sigma - rho);
+        const float c1 = static_cast<float>(rhoNew * rho), c2 = static_cast<float>(2.0 * rhoNew / delta);
+        if (k + 1 < M->options.degree)
+            CIECU_TRY(sl_launch(M, da, SlChebStep<0>{{M->d_s}, M->dinv32, c1, c2, r, db, x, nullptr, nullptr}, st));
+        else
+            CIECU_TRY(sl_launch(M, da, SlChebStep<END ? 2 : 1>{{M->d_s}, M->dinv32, c1, c2, r, db, x, M->z32, M->z},
+                                st));
+        std::swap(da, db);
+        rho = rhoNew;
+    }
+    return CIECU_OK;
+}
+
+// The FP32 cycle over the sliced copy: 5 vector passes and conversions fewer than over CSR.
+int sl_cycle(ciecu_mgcg_s* M, cudaStream_t st) {
+    const long n = M->n, ld = padded(n);
+    float *r = M->cheb32, *d = r + ld, *x = r + 3 * ld;
+    const float theta = static_cast<float>(0.5 * (M->lambdaMax + M->lambdaMin));
+    sl_start_kernel<<<grid_of(n), kT, 0, st>>>(n, M->r, M->dinv32, theta, M->r32, r, d, x);
+    count_launch();
+    CIECU_TRY(sl_sweep<false>(M, st));
+    CIECU_TRY(sl_launch(M, M->z32, SlResidual<false>{{M->d_s}, M->r32, nullptr, theta, M->t, nullptr, nullptr, nullptr},
+                        st));
+    CIECU_TRY(ciecu_csr_spmv_f64(M->R, 0.0, M->t, 1.0, M->rc));
+    CIECU_TRY(coarse_solve(M, st));
+    CIECU_TRY(ciecu_csr_spmv_f64(M->P, 0.0, M->cx, 1.0, M->t));  // t = P ec
+    convert_kernel<double, float><<<grid_of(n), kT, 0, st>>>(n, M->t, M->z32, 1);
+    count_launch();
+    CIECU_TRY(sl_launch(M, M->z32, SlResidual<true>{{M->d_s}, M->r32, M->dinv32, theta, nullptr, r, d, x}, st));
+    return sl_sweep<true>(M, st);
+}
+
 // out (+)= S in: Chebyshev polynomial of degree `degree` in D^-1 A applied to in.
 template <typename T>
 int chebyshev(ciecu_mgcg_s* M, ciecu_csr_s* A, const T* dinv, const T* in, T* out, bool accumulate, T* work,
               cudaStream_t st) {
     const long n = M->n;
     T* r = work;
-    T* da = work + n;
-    T* db = work + 2 * n;
-    T* x = work + 3 * n;
+    T* da = work + padded(n);
+    T* db = work + 2 * padded(n);
+    T* x = work + 3 * padded(n);
     const double theta = 0.5 * (M->lambdaMax + M->lambdaMin);
     const double delta = 0.5 * (M->lambdaMax - M->lambdaMin);
     const double sigma = theta / delta;
@@ -975,6 +1133,8 @@ int cycle(ciecu_mgcg_s* M, cudaStream_t st) {
         CIECU_CUDA(cudaMemcpyAsync(M->t, M->r, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
         CIECU_TRY(ciecu_csr_spmv_f64(A, 1.0, M->z, -1.0, M->t));
         CIECU_TRY(chebyshev<double>(M, A, M->dinv, M->t, M->z, true, M->cheb, st));
+    } else if (M->slices.blocks) {
+        CIECU_TRY(sl_cycle(M, st));
     } else {
         ciecu_csr_s* S = M->S32;
         convert_kernel<double, float><<<grid_of(n), kT, 0, st>>>(n, M->r, M->r32, 0);
@@ -1060,31 +1220,105 @@ __global__ void to_f32_kernel(long n, const double* __restrict__ a, float* __res
         b[i] = static_cast<float>(a[i]);
 }
 
+// The sliced copy of the FP32 smoother matrix (its layout; refresh_slices fills it at every
+// solve), where sl_layout finds that it pays.  A sweep of one step has no row pass to gain.
+// Q3, 117,649 rows: 15 us a step against 31.4 by the CSR kernel of 8 lanes a row.
+int prepare_slices(ciecu_mgcg_s* M, int lo, int hi, cudaStream_t st) {
+    ciecu_csr_s* S = M->S32;
+    if (M->options.degree < 2) return CIECU_OK;
+    int dev = 0, optin = 0;
+    CIECU_CUDA(cudaGetDevice(&dev));
+    CIECU_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const int n = static_cast<int>(M->n);
+    std::vector<int> rowptr(static_cast<size_t>(n) + 1), sliceEnd;
+    std::vector<short> row;
+    std::vector<SlBlock> blocks;
+    CIECU_CUDA(cudaMemcpyAsync(rowptr.data(), S->rowptr, sizeof(int) * rowptr.size(), cudaMemcpyDeviceToHost, st));
+    CIECU_CUDA(cudaStreamSynchronize(st));
+    SlPlan plan;
+    if (!sl_layout(n, rowptr.data(), lo, hi, sm_count(), static_cast<size_t>(std::max(optin - 2048, 0)), blocks,
+                   sliceEnd, row, plan.args.winLen, plan.smem, plan.steps))
+        return CIECU_OK;
+    using First = SlResidual<false>;
+    using Second = SlResidual<true>;
+    for (const void* kernel :
+         {reinterpret_cast<const void*>(sl_kernel<SlChebStep<0>>), reinterpret_cast<const void*>(sl_kernel<SlChebStep<1>>),
+          reinterpret_cast<const void*>(sl_kernel<SlChebStep<2>>), reinterpret_cast<const void*>(sl_kernel<First>),
+          reinterpret_cast<const void*>(sl_kernel<Second>)})
+        CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 2048));
+    size_t at = 0;
+    auto part = [&](size_t bytes) {
+        const size_t begin = at;
+        at = (at + bytes + 255) / 256 * 256;
+        return begin;
+    };
+    const size_t val = part(sizeof(float4) * 32 * static_cast<size_t>(plan.steps));
+    const size_t off = part(sizeof(short4) * 32 * static_cast<size_t>(plan.steps));
+    const size_t blk = part(sizeof(SlBlock) * blocks.size()), ends = part(sizeof(int) * sliceEnd.size());
+    const size_t rows = part(sizeof(short) * row.size());
+    if (pool_alloc(&plan.memory, at, st) != cudaSuccess) {
+        cudaGetLastError();  // no room: the CSR kernels stay
+        return CIECU_OK;
+    }
+    M->slices = plan;
+    char* base = static_cast<char*>(plan.memory);
+    CIECU_CUDA(cudaMemcpyAsync(base + blk, blocks.data(), sizeof(SlBlock) * blocks.size(), cudaMemcpyHostToDevice, st));
+    CIECU_CUDA(cudaMemcpyAsync(base + ends, sliceEnd.data(), sizeof(int) * sliceEnd.size(), cudaMemcpyHostToDevice, st));
+    CIECU_CUDA(cudaMemcpyAsync(base + rows, row.data(), sizeof(short) * row.size(), cudaMemcpyHostToDevice, st));
+    CIECU_CUDA(cudaStreamSynchronize(st));  // the host arrays end here
+    SlArgs& a = M->slices.args;
+    a.val = reinterpret_cast<float4*>(base + val);
+    a.off = reinterpret_cast<short4*>(base + off);
+    a.blocks = reinterpret_cast<SlBlock*>(base + blk);
+    a.sliceEnd = reinterpret_cast<int*>(base + ends);
+    a.row = reinterpret_cast<short*>(base + rows);
+    a.n = n;
+    a.lo = lo;
+    a.hi = hi;
+    M->slices.blocks = static_cast<int>(blocks.size());
+    M->lanes16 = 4;
+    return CIECU_OK;
+}
+
+// At every solve: the smoother matrix's values into the sliced copy.
+int refresh_slices(ciecu_mgcg_s* M, cudaStream_t st) {
+    if (!M->slices.blocks) return CIECU_OK;
+    const SlArgs& a = M->slices.args;
+    const CsrArgs<float> csr = M->S32->args<float>();
+    sl_fill_kernel<<<grid_for(static_cast<long>(M->slices.blocks) * 256, 256, 8), 256, 0, st>>>(
+        a, M->slices.blocks, csr.rowptr, M->col16, csr.val, const_cast<float4*>(a.val), const_cast<short4*>(a.off));
+    count_launch();
+    CIECU_CHECK_LAUNCH("sl_fill_kernel");
+    return CIECU_OK;
+}
+
 // 16-bit column offsets of the FP32 smoother matrix when every |col - row| fits,
 // and the lanes per row of its kernels (the residual kernel timed, best of
 // three, on scratch vectors); otherwise the smoother keeps the int32 columns.
 int prepare_offsets16(ciecu_mgcg_s* M, cudaStream_t st) {
     ciecu_csr_s* S = M->S32;
     if (S->nnz <= 0) return CIECU_OK;
-    unsigned* d_bad = reinterpret_cast<unsigned*>(S->space->d_result);
-    unsigned bad = 0;
+    int* d_range = reinterpret_cast<int*>(S->space->d_result);
+    int range[2] = {0, 0};
     if (cudaMalloc(&M->col16, sizeof(short) * static_cast<size_t>(S->nnz)) != cudaSuccess) {
         cudaGetLastError();  // no room: int32 columns
         M->col16 = nullptr;
         return CIECU_OK;
     }
-    CIECU_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(unsigned), st));
+    CIECU_CUDA(cudaMemsetAsync(d_range, 0, sizeof(range), st));
     offsets16_kernel<<<grid_for(M->n, 256, 8), 256, 0, st>>>(static_cast<int>(M->n), S->rowptr, S->col, M->col16,
-                                                             d_bad);
+                                                             d_range);
     count_launch();
     CIECU_CHECK_LAUNCH("offsets16_kernel");
-    CIECU_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    CIECU_CUDA(cudaMemcpyAsync(range, d_range, sizeof(range), cudaMemcpyDeviceToHost, st));
     CIECU_CUDA(cudaStreamSynchronize(st));
-    if (bad) {
+    if (range[0] < -32768 || range[1] > 32767) {
         cudaFree(M->col16);
         M->col16 = nullptr;
         return CIECU_OK;
     }
+    CIECU_TRY(prepare_slices(M, range[0], range[1], st));
+    if (M->slices.blocks) return CIECU_OK;
     // t32 / z32 as scratch (the solve overwrites both)
     CIECU_CUDA(cudaMemsetAsync(M->z32, 0, sizeof(float) * M->n, st));
     cudaEvent_t e0, e1;
@@ -1129,6 +1363,7 @@ int ciecu_mgcg_destroy(ciecu_mgcg M) {
                       M->cu, M->cw, M->cs, M->cm0, M->cm1, M->partials})
         cudaFree(v);
     for (float* v : {M->dinv32, M->r32, M->z32, M->t32, M->cheb32}) cudaFree(v);
+    if (M->slices.memory) pool_release({M->slices.memory});
     cudaFree(M->col16);
     cudaFree(M->coarse32);
     cudaFree(M->d_s);
@@ -1188,11 +1423,11 @@ int ciecu_mgcg_create(ciecu_csr fine, const double* d_fineInverseDiagonal, ciecu
         if (e == cudaSuccess) e = cudaMalloc(v, sizeof(double) * n);
     for (double** v : {&M->rc, &M->cx, &M->cr, &M->cz, &M->cp, &M->cq, &M->cu, &M->cw, &M->cs, &M->cm0, &M->cm1})
         if (e == cudaSuccess) e = cudaMalloc(v, sizeof(double) * m);
-    if (e == cudaSuccess && !smoother32) e = cudaMalloc(&M->cheb, sizeof(double) * 4 * n);
+    if (e == cudaSuccess && !smoother32) e = cudaMalloc(&M->cheb, sizeof(double) * 4 * padded(n));
     if (e == cudaSuccess && smoother32) {
         for (float** v : {&M->dinv32, &M->r32, &M->z32, &M->t32})
-            if (e == cudaSuccess) e = cudaMalloc(v, sizeof(float) * n);
-        if (e == cudaSuccess) e = cudaMalloc(&M->cheb32, sizeof(float) * 4 * n);
+            if (e == cudaSuccess) e = cudaMalloc(v, sizeof(float) * padded(n));
+        if (e == cudaSuccess) e = cudaMalloc(&M->cheb32, sizeof(float) * 4 * padded(n));
     }
     if (e == cudaSuccess) e = cudaMalloc(&M->partials, sizeof(double) * 2 * kMaxPartials);
     if (e == cudaSuccess) e = cudaMalloc(&M->counter, sizeof(unsigned) * 4);
@@ -1250,6 +1485,7 @@ int ciecu_mgcg_product(ciecu_mgcg M, double inScale, const double* d_in, double 
     CIECU_CUDA(cudaMemcpyAsync(M->x, d_out, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
     if (M->settings.iterationCount > 0) {
         CIECU_TRY(refresh_cluster(M, st));
+        CIECU_TRY(refresh_slices(M, st));
         if (M->graph && M->graphCluster != M->clusterActive) {  // the coarse form changed: capture again
             cudaGraphExecDestroy(M->graph);
             M->graph = nullptr;
@@ -1285,6 +1521,7 @@ int ciecu_mgcg_product(ciecu_mgcg M, double inScale, const double* d_in, double 
         const MgScalars& s = *M->h_s;
         if (s.error) {
             if (h_stats) *h_stats = ciecu_statistics{s.errorIter, s.absres, s.relres};
+            if (s.errorKind == 3) return fail(CIECU_ERR_TIMEOUT, "mgcg: a bounded wait for a copy gave up");
             if (s.errorKind == 1)
                 return fail(CIECU_ERR_BREAKDOWN, "preconditioned norm vanished in iteration " +
                                                      std::to_string(s.errorIter) + " (r^T @ z <= 0)");

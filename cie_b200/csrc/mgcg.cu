@@ -586,8 +586,14 @@ __global__ void __launch_bounds__(csr_threads<K>())
 // iteration come from the same vectors and are reduced together, and
 //   beta = gamma / gamma_old, alpha = gamma / (delta - beta gamma / alpha_old),
 //   p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = D^-1 r;
-// so an iteration costs one row pass over shared memory and two cluster barriers
-// (the reduction, the publication of u).  Its iterates are those of the pipelined
+// so an iteration costs one row pass over shared memory and two exchanges (the
+// reduction, the publication of u).  An exchange is a remote store that completes
+// bytes at the receiver's mbarrier (st.async): a CTA waits for the data it needs, the
+// sums of all CTAs or the halo of its neighbours, and for no one else.  With one row
+// per thread the row's coefficients stay in registers.
+// What bounds it: latency.  17^3 rows in 7 CTAs: 2.0 us an iteration; 3.55 with cluster
+// barriers, remote reads of the sums and the coefficients in shared memory, 2.55 with
+// the sums and the step formed by every warp.  Its iterates are those of the pipelined
 // kernels above in exact arithmetic; the matrix is read in FP32 (the solve is a
 // preconditioner), everything else is FP64.  Every CTA forms the cluster-wide
 // sums from the per-CTA sums in rank order with the same butterfly, so all
@@ -605,6 +611,7 @@ struct ClusterCoarse {
     const double* __restrict__ b;
     const double* __restrict__ dinv;
     double* __restrict__ x;
+    MgScalars* scalars;  // told when a bounded wait gives up
     int m, rowsPerCta, halo, iterations;
     int center[kClusterMaxTriples];  // triple centres, ascending, centre[NT / 2] = 0
 };
@@ -618,66 +625,144 @@ constexpr int cluster_upper_diagonals() {
 
 __host__ __device__ constexpr long cluster_align16(long bytes) { return (bytes + 15) / 16 * 16; }
 
-// Shared-memory bytes of a CTA: U rows, operand rows, 32 warp sums x 2 and 2 CTA sums.
+// Shared-memory bytes of a CTA: U rows, operand rows, 32 warp sums x 2, the sums that the
+// CTAs send (2 sets of 2 each, kClusterMaxCtas CTAs) and 3 barriers.
 __host__ __device__ constexpr long cluster_smem_bytes(int nu, int rowsPerCta, int halo) {
-    return cluster_align16(4L * nu * (rowsPerCta + halo)) + 8L * (rowsPerCta + 2L * halo) + 8L * 66;
+    return cluster_align16(cluster_align16(4L * nu * (rowsPerCta + halo)) + 8L * (rowsPerCta + 2L * halo)) +
+           8L * (64 + 4 * kClusterMaxCtas + 3);
 }
 
-__device__ __forceinline__ double warp_sum_all(double v) {
-#pragma unroll
-    for (int k = 16; k >= 1; k >>= 1) v += __shfl_xor_sync(0xffffffffu, v, k);
-    return v;  // the same bits in every lane: each step adds the same pair in both lanes
+// ---- remote stores that complete bytes at the receiver's barrier ----
+
+__device__ __forceinline__ unsigned cluster_address(const void* shared, int rank) {
+    unsigned out;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(out)
+        : "r"(static_cast<unsigned>(__cvta_generic_to_shared(shared))), "r"(rank));
+    return out;
 }
 
-// Cluster-wide sums of two values, bitwise equal in every thread of every CTA.
-__device__ __forceinline__ void cluster_sum2(cooperative_groups::cluster_group& cluster, double v0, double v1,
-                                             double* warpSums, double* ctaSums, int nctas, double& t0, double& t1) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v0 = warp_sum_all(v0);
-    v1 = warp_sum_all(v1);
-    if (lane == 0) {
-        warpSums[warp] = v0;
-        warpSums[32 + warp] = v1;
+__device__ __forceinline__ void cluster_send(unsigned to, unsigned bar, double v) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(to),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+
+// The bytes of the barrier's next phase (its one arrival).
+__device__ __forceinline__ void cluster_expect(const unsigned long long* bar, int bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(bar))),
+                 "r"(bytes)
+                 : "memory");
+}
+
+// False: the phase did not end within about a second.
+__device__ __forceinline__ bool cluster_wait(const unsigned long long* bar, unsigned parity) {
+    unsigned ok = 0;
+    for (long long begun = clock64(); !ok;) {
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))), "r"(parity)
+            : "memory");
+        if (!ok && clock64() - begun > (1LL << 31)) return false;
     }
+    return true;
+}
+
+// Sums of two values over 16-lane halves: v0's in the lower half, v1's in the upper one,
+// the same bits in every lane of a half.
+__device__ __forceinline__ double half_sum(double v) {
+#pragma unroll
+    for (int k = 8; k >= 1; k >>= 1) v += __shfl_xor_sync(0xffffffffu, v, k);
+    return v;
+}
+
+__device__ __forceinline__ double half_sum2(double v0, double v1) {
+    const bool upper = threadIdx.x & 16;
+    const double give = upper ? v0 : v1;
+    return half_sum((upper ? v1 : v0) + __shfl_xor_sync(0xffffffffu, give, 16));
+}
+
+// The step of one iteration, the same bits in every CTA.
+struct ClusterStep {
+    double alpha, beta;
+    int state;  // 0: go on, 1: no further steps, 2: a wait gave up
+};
+
+// From the threads' shares of (r, u) and (w, u): warp 0 sends the CTA's sums to every
+// CTA's box of this turn (two boxes, two barriers: a CTA may be one exchange ahead of
+// another, never two, since it needs that one's sums), adds what arrives in rank order
+// of a butterfly and forms the step; the other warps wait for its result, and spend
+// neither shuffles nor divisions on it.
+__device__ __forceinline__ void cluster_step(double g, double dl, double* warpSums, double* box,
+                                             unsigned long long* bars, int it, int rank, int nctas, double& gammaOld,
+                                             double& alphaOld, ClusterStep* step) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane & 15, upper = lane >> 4;
+    constexpr int kWarps = kClusterThreads / 32;
+    static_assert(kWarps > 16 && kWarps <= 32 && kClusterMaxCtas == 16, "two halves of 16 lanes");
+    const double v = half_sum2(g, dl);
+    if (half == 0) warpSums[32 * upper + warp] = v;
     __syncthreads();
     if (warp == 0) {
-        constexpr int kWarps = kClusterThreads / 32;
-        const double a = warp_sum_all(lane < kWarps ? warpSums[lane] : 0.0);
-        const double b = warp_sum_all(lane < kWarps ? warpSums[32 + lane] : 0.0);
-        if (lane == 0) {
-            ctaSums[0] = a;
-            ctaSums[1] = b;
+        double* mine = box + (it & 1) * 2 * kClusterMaxCtas;  // (r, u) of every CTA, then (w, u)
+        unsigned long long* bar = bars + (it & 1);
+        const double* sums = warpSums + 32 * upper;
+        const double cta = half_sum(sums[half] + (half + 16 < kWarps ? sums[half + 16] : 0.0));
+        if (half < nctas)
+            cluster_send(cluster_address(mine + kClusterMaxCtas * upper + rank, half), cluster_address(bar, half), cta);
+        ClusterStep s{0.0, 0.0, 2};
+        if (cluster_wait(bar, (it >> 1) & 1)) {
+            if (lane == 0) cluster_expect(bar, 16 * nctas);
+            const double all = half_sum(half < nctas ? mine[kClusterMaxCtas * upper + half] : 0.0);
+            const double gamma = __shfl_sync(0xffffffffu, all, 0), delta = __shfl_sync(0xffffffffu, all, 16);
+            s.beta = it == 0 ? 0.0 : gamma / gammaOld;
+            const double den = it == 0 ? delta : delta - s.beta * gamma / alphaOld;
+            s.state = !(0.0 < gamma) || !(0.0 < den);  // converged to rounding or broken down
+            s.alpha = gamma / den;
+            gammaOld = gamma;
+            alphaOld = s.alpha;
         }
+        if (lane == 0) *step = s;
     }
-    cluster.sync();
-    const double a = lane < nctas ? *cluster.map_shared_rank(ctaSums, lane) : 0.0;
-    const double b = lane < nctas ? *cluster.map_shared_rank(ctaSums + 1, lane) : 0.0;
-    t0 = warp_sum_all(a);
-    t1 = warp_sum_all(b);
+    __syncthreads();
 }
 
 // u of the own rows into the CTA's operand, and into the halo of the neighbours
-// whose rows reach them (rows within H of either end of the block).
+// whose rows reach them (rows within H of either end of the block).  They have read
+// their halo: their sums, which this CTA has, came after it.
 template <int R>
-__device__ __forceinline__ void cluster_publish(cooperative_groups::cluster_group& cluster, double* pe,
-                                                const double (&u)[R], int li0, int C, int H, int rank, int nctas) {
-    double* prev = rank > 0 ? cluster.map_shared_rank(pe, rank - 1) : nullptr;
-    double* next = rank + 1 < nctas ? cluster.map_shared_rank(pe, rank + 1) : nullptr;
+__device__ __forceinline__ void cluster_publish(double* pe, const unsigned long long* bar, const double (&u)[R],
+                                                int li0, int C, int H, int rank, int nctas) {
+    const bool prev = rank > 0, next = rank + 1 < nctas;
 #pragma unroll
     for (int j = 0; j < R; ++j) {
         const int li = li0 + j;
         pe[H + li] = u[j];
-        if (prev && li < H) prev[C + H + li] = u[j];            // the previous CTA's right halo
-        if (next && li >= C - H) next[li - C + H] = u[j];       // the next CTA's left halo
+        if (prev && li < H)  // the previous CTA's right halo
+            cluster_send(cluster_address(pe + C + H + li, rank - 1), cluster_address(bar, rank - 1), u[j]);
+        if (next && li >= C - H)  // the next CTA's left halo
+            cluster_send(cluster_address(pe + li - C + H, rank + 1), cluster_address(bar, rank + 1), u[j]);
     }
+}
+
+// Coefficient of offset c - 1 + k (c the centre of triple t) in the row of U index e.
+// Lower entries are read from U at row r + o: A[r][r + o] = U_{-o}[r + o], where -o is
+// the mirrored centre + 1 - k.
+template <int NT>
+__device__ __forceinline__ float cluster_coefficient(const float* U, int lu, int e, int c, int t, int k) {
+    if (t < NT / 2) return U[(2 + 3 * (NT / 2 - 1 - t) + (2 - k)) * lu + e + c - 1 + k];
+    if (t == NT / 2) return k == 0 ? U[lu + e - 1] : (k == 1 ? U[e] : U[lu + e]);
+    return U[(2 + 3 * (t - NT / 2 - 1) + k) * lu + e];
 }
 
 // w = A u for the R consecutive own rows starting at operand index e0 (= H + li0;
 // U index of those rows is the same): per triple of diagonals the R + 2 operand
-// entries are loaded once.  Lower entries are read from U at row r + o.
+// entries are loaded once.  R = 1: the coefficients are the registers `own`.
 template <int NT, int R>
-__device__ __forceinline__ void cluster_rows(const float* U, int lu, const double* pe, int e0, const int* center,
-                                             double (&w)[R]) {
+__device__ __forceinline__ void cluster_rows(const float* U, const float (&own)[R == 1 ? 3 * NT : 1], int lu,
+                                             const double* pe, int e0, const int* center, double (&w)[R]) {
 #pragma unroll
     for (int j = 0; j < R; ++j) w[j] = 0.0;
 #pragma unroll
@@ -691,12 +776,8 @@ __device__ __forceinline__ void cluster_rows(const float* U, int lu, const doubl
 #pragma unroll
             for (int j = 0; j < R; ++j) {
                 float a;
-                if (t < NT / 2)  // o < 0: A[r][r + o] = U_{-o}[r + o], -o = c_mirror + 1 - k
-                    a = U[(2 + 3 * (NT / 2 - 1 - t) + (2 - k)) * lu + e0 + j + c - 1 + k];
-                else if (t == NT / 2)
-                    a = k == 0 ? U[lu + e0 + j - 1] : (k == 1 ? U[e0 + j] : U[lu + e0 + j]);
-                else
-                    a = U[(2 + 3 * (t - NT / 2 - 1) + k) * lu + e0 + j];
+                if constexpr (R == 1) a = own[3 * t + k];
+                else a = cluster_coefficient<NT>(U, lu, e0 + j, c, t, k);
                 w[j] = fma(static_cast<double>(a), xv[j + k], w[j]);
             }
         }
@@ -715,8 +796,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1) coarse_cluster_kernel(Clus
     const long start = static_cast<long>(rank) * C;
     float* U = reinterpret_cast<float*>(smem);
     double* pe = reinterpret_cast<double*>(smem + cluster_align16(4L * NU * lu));
-    double* warpSums = pe + pl;
-    double* ctaSums = warpSums + 64;
+    double* warpSums = reinterpret_cast<double*>(
+        smem + cluster_align16(cluster_align16(4L * NU * lu) + 8L * pl));  // the boxes after it: 16 bytes
+    double* box = warpSums + 64;
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(box + 4 * kClusterMaxCtas);  // sums x 2, halo
+    const int haloBytes = 8 * H * ((rank > 0) + (rank + 1 < nctas));
 
     for (int d = 0; d < NU; ++d)
         for (int e = threadIdx.x; e < lu; e += kClusterThreads) {
@@ -724,7 +808,17 @@ __global__ void __launch_bounds__(kClusterThreads, 1) coarse_cluster_kernel(Clus
             U[d * lu + e] = (r >= 0 && r < a.m) ? __ldg(a.upper + d * a.ld + r) : 0.0f;
         }
     for (int e = threadIdx.x; e < pl; e += kClusterThreads) pe[e] = 0.0;
-    cluster.sync();  // every CTA has zeroed its operand before any halo is pushed
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 3; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                             static_cast<unsigned>(__cvta_generic_to_shared(bars + k)))
+                         : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        cluster_expect(bars, 16 * nctas);
+        cluster_expect(bars + 1, 16 * nctas);
+        cluster_expect(bars + 2, haloBytes);
+    }
+    cluster.sync();  // every CTA has zeroed its operand and its barriers stand before anything is sent
 
     const int li0 = R * static_cast<int>(threadIdx.x);
     double xs[R], rs[R], ps[R], ss[R], ds[R], us[R];
@@ -737,23 +831,34 @@ __global__ void __launch_bounds__(kClusterThreads, 1) coarse_cluster_kernel(Clus
         us[j] = ds[j] * rs[j];
         xs[j] = ps[j] = ss[j] = 0.0;
     }
-    cluster_publish<R>(cluster, pe, us, li0, C, H, rank, nctas);
-    cluster.sync();
-    double gammaOld = 0.0, alphaOld = 0.0;
+    __shared__ ClusterStep s_step;
+    float own[R == 1 ? 3 * NT : 1];
+    if constexpr (R == 1) {
+#pragma unroll
+        for (int k = 0; k < 3 * NT; ++k) own[k] = cluster_coefficient<NT>(U, lu, H + li0, a.center[k / 3], k / 3, k % 3);
+    }
+    cluster_publish<R>(pe, bars + 2, us, li0, C, H, rank, nctas);
+    double gammaOld = 0.0, alphaOld = 0.0;  // warp 0's
+    bool ok = true;
     for (int it = 0; it < a.iterations; ++it) {
+        __syncthreads();  // the own rows of u
+        if (nctas > 1) {
+            ok = cluster_wait(bars + 2, it & 1);
+            if (!ok) break;
+            if (threadIdx.x == 0) cluster_expect(bars + 2, haloBytes);
+        }
         double w[R];
-        cluster_rows<NT, R>(U, lu, pe, H + li0, a.center, w);
+        cluster_rows<NT, R>(U, own, lu, pe, H + li0, a.center, w);
         double g = 0.0, dl = 0.0;
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             g = fma(rs[j], us[j], g);
             dl = fma(w[j], us[j], dl);
         }
-        cluster_sum2(cluster, g, dl, warpSums, ctaSums, nctas, g, dl);
-        const double beta = it == 0 ? 0.0 : g / gammaOld;
-        const double den = it == 0 ? dl : dl - beta * g / alphaOld;
-        if (!(0.0 < g) || !(0.0 < den)) break;  // converged to rounding or broken down: no further steps
-        const double alpha = g / den;
+        cluster_step(g, dl, warpSums, box, bars, it, rank, nctas, gammaOld, alphaOld, &s_step);
+        ok = s_step.state != 2;
+        if (s_step.state) break;
+        const double alpha = s_step.alpha, beta = s_step.beta;
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             ps[j] = fma(beta, ps[j], us[j]);
@@ -762,18 +867,21 @@ __global__ void __launch_bounds__(kClusterThreads, 1) coarse_cluster_kernel(Clus
             rs[j] = fma(-alpha, ss[j], rs[j]);
             us[j] = ds[j] * rs[j];
         }
-        gammaOld = g;
-        alphaOld = alpha;
         if (it + 1 == a.iterations) break;
-        cluster_publish<R>(cluster, pe, us, li0, C, H, rank, nctas);
-        cluster.sync();
+        cluster_publish<R>(pe, bars + 2, us, li0, C, H, rank, nctas);
+    }
+    if (!ok) {  // a bounded wait gave up
+        a.scalars->done = 3;
+        a.scalars->error = CIECU_ERR_TIMEOUT;
+        a.scalars->errorKind = 3;
+        a.scalars->errorIter = a.scalars->iter;
     }
 #pragma unroll
     for (int j = 0; j < R; ++j) {
         const long row = start + li0 + j;
         if (row < a.m) a.x[row] = xs[j];
     }
-    cluster.sync();  // no CTA leaves while another may still read its CTA sums
+    cluster.sync();  // no CTA leaves while another may still send to it
 }
 
 __global__ void count_cycle_kernel(MgScalars* s) { s->cycles += 1; }
@@ -1051,6 +1159,7 @@ int prepare_cluster(ciecu_mgcg_s* M, cudaStream_t st) {
     a.b = M->rc;
     a.dinv = M->dinvc;
     a.x = M->cx;
+    a.scalars = M->d_s;
     a.m = static_cast<int>(M->m);
     a.rowsPerCta = rows * kClusterThreads;
     a.halo = halo;
@@ -1433,6 +1542,7 @@ int ciecu_mgcg_create(ciecu_csr fine, const double* d_fineInverseDiagonal, ciecu
     if (e == cudaSuccess) e = cudaMalloc(&M->counter, sizeof(unsigned) * 4);
     if (e == cudaSuccess) e = cudaMemsetAsync(M->counter, 0, sizeof(unsigned) * 4, st);
     if (e == cudaSuccess) e = cudaMalloc(&M->d_s, sizeof(MgScalars));
+    if (e == cudaSuccess) e = cudaMemsetAsync(M->d_s, 0, sizeof(MgScalars), st);
     if (e == cudaSuccess) e = cudaMallocHost(&M->h_s, sizeof(MgScalars));
     if (e != cudaSuccess) {
         ciecu_mgcg_destroy(M);
@@ -1554,7 +1664,10 @@ int ciecu_mgcg_coarse_apply(ciecu_mgcg M, const double* d_in, double* d_out) {
     CIECU_TRY(coarse_solve(M, st));
     CIECU_CHECK_LAUNCH("coarse solve");
     CIECU_CUDA(cudaMemcpyAsync(d_out, M->cx, sizeof(double) * M->m, cudaMemcpyDeviceToDevice, st));
+    int kind = 0;
+    CIECU_CUDA(cudaMemcpyAsync(&kind, &M->d_s->errorKind, sizeof(int), cudaMemcpyDeviceToHost, st));
     CIECU_CUDA(cudaStreamSynchronize(st));
+    if (kind == 3) return fail(CIECU_ERR_TIMEOUT, "mgcg_coarse_apply: a bounded wait gave up");
     return CIECU_OK;
 }
 

@@ -21,6 +21,11 @@ inline bool device_loop_enabled() {
     return enabled;
 }
 
+// Iterations in the body of a solver's loop: a turn of the WHILE node costs 8 us beside
+// its kernels (3 with an IF node in the body as well, at 2.1 M rows; 4 at 262,144); the
+// kernels of the iterations after the last one return at once, about 2 us each.
+constexpr int kLoopUnroll = 8;
+
 template <typename F>
 int build_while_graph(cudaStream_t st, F&& body, cudaGraphExec_t* exec) {
     *exec = nullptr;

@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(kT) mixed_spmv_kernel(SellArgs<float, CI> A, c
         if (blockIdx.x == 0 && threadIdx.x == 0) set_cond<COND>(loop, 0);
         return;
     }
+    if (*reinterpret_cast<volatile int*>(&s->update)) return;  // until the refinement
     auto op = M1Op<FUSED>::make(x, p, q, s);
     sell_rows<U, float, float, CI>(A, x, op);
     double mine[1] = {op.acc}, tot[1];
@@ -276,6 +277,7 @@ __global__ void __launch_bounds__(kT, 3) mixed_spmv_dia_kernel(DiaArgs<float> A,
         if (blockIdx.x == 0 && threadIdx.x == 0) set_cond<COND>(loop, 0);
         return;
     }
+    if (*reinterpret_cast<volatile int*>(&s->update)) return;  // until the refinement
     auto op = M1Op<FUSED>::make(x, p, q, s);
     mixed_dia_rows<ND, TRIPLES>(A, x, op);
     double mine[1] = {op.acc}, tot[1];
@@ -560,6 +562,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32) mixed_spmv_tma_kernel(SellArgs
         if (blockIdx.x == 0 && threadIdx.x == 0) set_cond<COND>(loop, 0);
         return;
     }
+    if (*reinterpret_cast<volatile int*>(&s->update)) return;  // until the refinement
     auto op = M1Op<FUSED>::make(x, p, q, s);
     sell_rows_tma<CI>(A, x, op, tma_smem, &s->tmaError);
     double mine[1] = {op.acc}, tot[1];
@@ -603,6 +606,7 @@ __global__ void __launch_bounds__(kT, 3) mixed_update_kernel(long n, float* __re
         }
         return;
     }
+    if (*reinterpret_cast<volatile int*>(&s->update)) return;  // until the refinement, which is set
     const float alpha = static_cast<float>(s->alpha);
     const bool step = !s->restart;  // after an FP32 breakdown: no step (p may not be finite)
     double rr = 0.0, rz = 0.0;
@@ -977,7 +981,7 @@ int launch_single(ciecu_mixed_s* M, cudaStream_t st, cudaGraphConditionalHandle 
     return CIECU_OK;
 }
 
-// One inner iteration.  With conditional nodes (useCond) the refinement pair
+// Inner iterations.  With conditional nodes (useCond) the refinement pair
 // R1/R2 sits under IF(refine); otherwise it is launched unconditionally and
 // returns at once unless M2 requested a replacement.
 template <bool COND>
@@ -992,10 +996,15 @@ int launch_inner(ciecu_mixed_s* M, cudaStream_t st, cudaGraph_t root, cudaGraphC
     if (single) {
         CIECU_TRY(launch_single<COND>(M, st, loop, refine));
     } else {
-        CIECU_TRY(launch_inner_spmv<COND>(M, st, loop));
-        auto* kernel = M->z32 ? mixed_update_kernel<COND, true> : mixed_update_kernel<COND, false>;
-        kernel<<<fit_grid(kernel, kT, needV), kT, 0, st>>>(M->n, M->x32, M->r32, M->z32, M->p32, M->q32, M->dinv32,
-                                                           M->d_s, M->d_partials, M->d_counter, loop, refine);
+        // The fused form has several iterations before the refinement: once one asks for it,
+        // those after it return at once.  (The plain form's direction pass comes after it.)
+        for (int i = 0; i < (useCond && M->z32 ? kLoopUnroll : 1); ++i) {
+            CIECU_TRY(launch_inner_spmv<COND>(M, st, loop));
+            auto* kernel = M->z32 ? mixed_update_kernel<COND, true> : mixed_update_kernel<COND, false>;
+            kernel<<<fit_grid(kernel, kT, needV), kT, 0, st>>>(M->n, M->x32, M->r32, M->z32, M->p32, M->q32,
+                                                               M->dinv32, M->d_s, M->d_partials, M->d_counter, loop,
+                                                               refine);
+        }
     }
     auto refinement = [&](cudaStream_t s2) -> int {
         if (single)

@@ -1114,9 +1114,10 @@ int build_graph(ciecu_pcg_s* S) {
     }
     int status = CIECU_ERR_ARGUMENT;
     if (device_loop_enabled())
-        status = build_while_graph(st, [&](cudaGraph_t, cudaGraphConditionalHandle cond) {
-        return launch_iteration<true>(S, st, cond);
-    }, &S->graph);
+        status = build_while_graph(st, [&](cudaGraph_t, cudaGraphConditionalHandle cond) -> int {
+            for (int i = 0; i < kLoopUnroll; ++i) CIECU_TRY(launch_iteration<true>(S, st, cond));
+            return CIECU_OK;
+        }, &S->graph);
     if (status == CIECU_OK) {
         S->deviceLoop = true;
         S->graphKernel = S->kernel;

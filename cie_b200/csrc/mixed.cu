@@ -248,7 +248,8 @@ __global__ void __launch_bounds__(kT) mixed_spmv_kernel(SellArgs<float, CI> A, c
 // diagonals (dia.cuh): FP32 values only, no column indices.  The full copy is read
 // even when it is symmetric: reading the lower half back from the upper one (as
 // the FP64 PCG does) measured slower here, where every row pass is already a
-// four-row, 16-byte-load stream.
+// four-row, 16-byte-load stream; by marching tiles (dia_march.cuh) 47 us against 41 at
+// 2.1 M rows.
 // TRIPLES: the offsets come in consecutive triples (dia_rows4_triples).
 template <int ND, bool TRIPLES, typename Op>
 __device__ __forceinline__ void mixed_dia_rows(const DiaArgs<float>& A, const float* __restrict__ x, Op& op) {

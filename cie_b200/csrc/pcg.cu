@@ -13,6 +13,7 @@
 // fixed number of iterations can be replayed until the host sees the flag.
 #include "graph.cuh"
 #include "dia.cuh"
+#include "dia_march.cuh"
 #include "dia_persistent.cuh"
 #include "pcg.cuh"
 #include "sell_persistent.cuh"
@@ -131,6 +132,45 @@ __global__ void __launch_bounds__(kT) pcg_spmv_dia_sym_kernel(DiaArgs<double> U,
     dia_rows_sym<0, double, double>(U, p, op);
     double mine[1] = {op.acc}, tot[1];
     if (grid_reduce_last<1, kT>(mine, partials, counter, tot) && threadIdx.x == 0) {
+        s->pq = tot[0];
+        if (!(0.0 < tot[0])) {
+            s->done = 3;
+            s->error = CIECU_ERR_BREAKDOWN;
+            s->errorKind = 2;
+            s->errorIter = s->iter;
+            set_loop<COND>(cond, 0);
+        } else {
+            s->alpha = s->rz / tot[0];
+        }
+    }
+}
+
+// K1 by tiles that march through the planes of a 3D Q1 stencil (dia_march.cuh): the same
+// row sums again, each entry of the upper half read from memory once.
+struct MarchPqOp : PqOp {
+    PcgScalars* s;
+    __device__ __forceinline__ void expired() const {
+        s->done = 3;
+        s->error = CIECU_ERR_TIMEOUT;
+        s->errorKind = 3;
+        s->errorIter = s->iter;
+    }
+};
+
+template <bool COND>
+__global__ void __launch_bounds__(kDmThreads, 1)
+    pcg_spmv_march_kernel(const __grid_constant__ DmArgs A, const double* __restrict__ p,
+                          double* __restrict__ q, PcgScalars* s, double* partials, unsigned* counter,
+                          cudaGraphConditionalHandle cond) {
+    if (*reinterpret_cast<volatile int*>(&s->done)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) set_loop<COND>(cond, 0);
+        return;
+    }
+    MarchPqOp op{{p, q, 0.0}, s};
+    dm_rows(A, p, op);
+    double mine[1] = {op.acc}, tot[1];
+    if (grid_reduce_last<1, kDmThreads>(mine, partials, counter, tot) && threadIdx.x == 0) {
+        if (s->done) return;  // a wait gave up
         s->pq = tot[0];
         if (!(0.0 < tot[0])) {
             s->done = 3;
@@ -688,6 +728,9 @@ struct ciecu_pcg_s {
     double* diaBuf = nullptr;
     ciecu::DiaArgs<double> dia{};
     bool diaSym = false;           // the copy is bitwise symmetric: K1 reads diaU, its upper half
+    bool marchPlanned = false;
+    ciecu::DmPlan march{};  // ... by tiles marching through the planes (blocks = 0: not)
+    double* triples = nullptr;
     ciecu::DiaArgs<double> diaU{};
     // Single-launch solve (allocated at its first use).
     int loopMode = 0;     // 0 auto (single launch when the system fits in L2), 1 graph, 2 single launch
@@ -732,7 +775,10 @@ int launch_k1(ciecu_pcg_s* S, cudaStream_t st, int schedule, cudaGraphConditiona
         // Runtime diagonal count (9 loads in flight per row): a fully unrolled
         // 27-diagonal FP64 row needs 64 registers and halves the occupancy, which
         // measured 20 % slower at 128^3.
-        if (S->diaSym)
+        if (S->diaSym && S->march.blocks)
+            pcg_spmv_march_kernel<COND><<<S->march.blocks, kDmThreads, S->march.smem, st>>>(
+                S->march.args, S->p, S->q, S->d_s, S->d_partials, S->d_counter, cond);
+        else if (S->diaSym)
             pcg_spmv_dia_sym_kernel<COND><<<fit_grid(pcg_spmv_dia_sym_kernel<COND>, kT, (S->n + kT - 1) / kT), kT, 0,
                                             st>>>(S->diaU, S->p, S->q, S->d_s, S->d_partials, S->d_counter, cond);
         else
@@ -747,6 +793,23 @@ int launch_k1(ciecu_pcg_s* S, cudaStream_t st, int schedule, cudaGraphConditiona
                                    st>>>(A->args<double>(), S->p, S->q, S->d_s, S->d_partials, S->d_counter, cond);
         return CIECU_OK;
     });
+}
+
+// Least bytes of the upper half for which K1 marches: where the matrix no longer stays in
+// L2.  An iteration over 113^3 rows (162 MB): 66 us, 76 by dia_rows_sym; 97^3 (102 MB): 51 and
+// 52; 81^3 (60 MB): 41 and 34.
+constexpr long kMarchBytes = 112L << 20;
+
+// Plans the marching K1 once per solver; refills its copy of the triples at every solve.
+int refresh_march(ciecu_pcg_s* S, cudaStream_t st) {
+    if (!S->marchPlanned) {
+        S->marchPlanned = true;
+        CIECU_TRY(dm_prepare(S->diaU, kMarchBytes,
+                                     {reinterpret_cast<const void*>(pcg_spmv_march_kernel<true>),
+                                      reinterpret_cast<const void*>(pcg_spmv_march_kernel<false>)},
+                                     S->p, st, &S->march, &S->triples));
+    }
+    return S->march.blocks ? dm_fill(S->diaU, S->triples, st) : CIECU_OK;
 }
 
 // Finds the diagonals once per solver and refills the DIA copy from the CSR
@@ -779,6 +842,7 @@ int refresh_dia(ciecu_pcg_s* S, cudaStream_t st) {
             CIECU_TRY(dia_symmetric(S->dia, st, reinterpret_cast<unsigned*>(S->A->space->d_result), &sym));
         S->diaSym = sym;
         if (sym) S->diaU = dia_upper_view(S->dia);
+        if (sym) CIECU_TRY(refresh_march(S, st));
     }
     return CIECU_OK;
 }
@@ -1190,7 +1254,7 @@ int ciecu_pcg_destroy(ciecu_pcg S) {
     // synchronises the device before releasing memory.
     if (S->graph) cudaGraphExecDestroy(S->graph);
     sp_destroy(S->sp);
-    pool_release({S->x, S->r, S->p, S->q, S->d_s, S->d_partials, S->d_counter, S->diaBuf, S->z, S->p2, S->slots,
+    pool_release({S->x, S->r, S->p, S->q, S->d_s, S->d_partials, S->d_counter, S->diaBuf, S->triples, S->z, S->p2, S->slots,
                   S->dpSlots, S->abortFlag, S->split});
     delete S->h_s;
     delete S;
@@ -1338,6 +1402,7 @@ int ciecu_pcg_product(ciecu_pcg S, double inScale, const double* d_in, double ou
         const PcgScalars& s = *S->h_s;
         if (s.error) {
             if (h_stats) *h_stats = ciecu_statistics{s.errorIter, s.absres, s.relres};
+            if (s.errorKind == 3) return fail(CIECU_ERR_TIMEOUT, "pcg: a bounded wait for a copy gave up");
             if (s.errorKind == 1)
                 return fail(CIECU_ERR_BREAKDOWN, "preconditioned norm vanished in iteration 0 (r^T @ z = 0)");
             return fail(CIECU_ERR_BREAKDOWN, "p^T @ A @ p vanished in iteration " + std::to_string(s.errorIter));

@@ -1,6 +1,6 @@
 """Assembly path over the CUDA backend: structured Q_p meshes, the CSR pattern
 (Assembler::makeCSRMatrix), GPU element stiffness integration + atomic-free
-coloured scatter (IntegrandProcessor + Assembler::addContribution), symmetric
+row-wise gather (IntegrandProcessor + Assembler::addContribution), symmetric
 Dirichlet elimination, and the seeded synthetic Poisson problems.
 
 Seeded inputs (identical host arrays feed the GPU and the oracle):

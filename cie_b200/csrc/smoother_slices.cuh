@@ -9,7 +9,8 @@
 // length, longest first, to the warp with the least work, and lie in the order in which
 // their warp reads them: a warp reads ONE contiguous stream, kSlSteps steps ahead, across
 // the ends of its rows.  Padding has value 0 and offset 0.  A row's sum is kept in 16
-// partial sums, so no chain is longer than a sixteenth of the row.
+// partial sums, so no chain is longer than a sixteenth of the row, and they are added in the
+// order of the CSR kernel of 16 lanes a row: the same bits.
 //
 // What bounds it: a launch costs 7.5 us whatever the size (start, block, window, epilogue);
 // the copy then comes from L2 at the 11 TB/s that all SMs draw together.  117,649 rows of
@@ -147,9 +148,9 @@ __device__ __forceinline__ void sl_rows(const SlArgs& A, const float* __restrict
                     o[u] = __ldg(A.off + (t + u + kSlSteps) * 32L + lane);
                 }
                 if (t + u + 1 == stop) {
-                    float s = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-                    s += __shfl_xor_sync(0xffffffffu, s, 1);
+                    float s = (acc[0] + acc[2]) + (acc[1] + acc[3]);
                     s += __shfl_xor_sync(0xffffffffu, s, 2);
+                    s += __shfl_xor_sync(0xffffffffu, s, 1);
                     if ((lane & 3) == 0 && r >= 0) sum[r] = s;
                     acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
                     r = nextRow;

@@ -3,30 +3,42 @@
 // material scaling of ScaledMultiMaterialIntegrand (integrands/impl/
 // ScaledMultiMaterialIntegrand_impl.hpp:33-60) and the stiffness integrand
 // (LinearIsotropicStiffnessIntegrand_impl.hpp:62-75), load-balanced and with the
-// element matrices formed from moments.
+// element contraction on tensor cores.
 //
 // The element matrix of a cut cell is a Gram matrix over its kept quadrature
-// points, K = sum_{p,d} w_p s_p f_d G_p[d] G_p[d]^T.  Products of two basis
-// functions (or of two derivatives) of one axis are polynomials of degree 2 p, so
-//   phi_i phi_j = sum_a c0[ij][a] P_a,   phi_i' phi_j' = sum_a c1[ij][a] P_a
-// in Legendre polynomials, and the points enter only through the (2p + 1)^dim
-// moments of the cell, mu[abc] = sum_p w_p s_p P_a(x_p) P_b(y_p) P_c(z_p):
-//   K = sum_axis f_axis sum_abc mu[abc] c[..][a] c[..][b] c[..][c].
-// Three passes:
+// points: K = sum_{p,d} w_p s_p f_d G_p[d] G_p[d]^T = B^T W B, B of (points x dim)
+// rows and nb <= 64 columns.  It is computed in three passes:
 //   1. classify every cell by its base points (one warp per cell); a prefix sum
 //      numbers the cut cells in cell order;
-//   2. one CTA per cut cell (fc_cell_kernel): a warp per depth-1 tree node walks
-//      that node's subtree with the keep / refine rules and adds the kept points'
-//      moments, plane by plane and axis by axis; the warps' moments are summed in
-//      node order and contracted with c0 and c1 axis by axis;
-//   3. the row gather (assembly.cuh) adds every cell's matrix into the CSR values:
-//      regular cells s K1 (s = 1 inside, alpha outside, K1 the standard-rule
-//      matrix), cut cells their own, in colour order.
-// Everything is in FP64 (the FP32 copy for inner / preconditioner operators rounds
-// the finished FP64 element matrices), and no sum depends on the schedule.
+//   2. one CTA per (cut cell, depth-1 tree node) walks that node's subtree with
+//      the keep / refine rules, stages the basis gradients of 16 kept points at a
+//      time in shared memory and accumulates B^T W B with warp-level tensor-core
+//      MMAs into a partial element matrix -- eight CTAs per cut cell instead of
+//      one, so no SM waits for a few cut cells of a colour;
+//   3. the row gather (assembly.cuh) adds every cell's matrix into the CSR values, in
+//      colour order: regular cells s K1 (s = 1 inside, alpha outside, K1 the
+//      standard-rule matrix), cut cells the sum of their partials in node order.
+//      The result does not depend on the schedule.
+//
+// What bounds it: the walk's barriers and the staging of the gradients (tensor pipe 21 %
+// active), 18 ms of 19.3 at 32^3 Q3 with 2,528 cut cells.  The points enter an element matrix only
+// through their (2p + 1)^dim Legendre moments, and formed from those the same matrices take
+// 1.5 ms, 2.5e-16 from these in the 2-norm; but with alpha = 1e-6 the solution hears the
+// rounding of the matrix 1e7 times louder, and came out up to 1.5e-9 elsewhere.
+//
+// Two contractions:
+//   FP64 (the solver's matrix): mma.sync m8n8k4 f64 (DMMA) -- FP64 products and
+//     sums, the same accuracy as the scalar FP64 loop (parity 1e-12 with the
+//     restatement);
+//   FP32 (a single-precision copy for inner / preconditioner operators):
+//     mma.sync m16n8k16 bf16 with FP32 accumulation, each operand split into a
+//     high and a low bf16 part and the three significant products summed
+//     (hi*hi + hi*lo + lo*hi): about 16 significant bits per product, FP32 sums.
 #include "assembly.cuh"
 #include "sortscan.cuh"
 #include "space.cuh"
+
+#include <cuda_bf16.h>
 
 #include <algorithm>
 #include <string>
@@ -34,6 +46,13 @@
 
 namespace ciecu {
 namespace {
+
+constexpr int kFcWarps = 8;
+constexpr int kFcThreads = 32 * kFcWarps;
+constexpr int kFcPoints = 16;               // kept points staged per chunk
+constexpr int kFcRows = 3 * kFcPoints;      // rows (point, axis) of B per chunk
+constexpr int kFcStride = 72;               // doubles per staged row: 64 columns + 8 (spreads the banks)
+constexpr int kFcStack = 64;
 
 // One warp per cell: number of the cell's base points inside the domain.
 // cut[e] = 1 for a cell with points on both sides; side[e] = 1 for a cell fully
@@ -70,74 +89,152 @@ __global__ void fc_compact_kernel(long ncells, const int* __restrict__ cut, cons
         if (cut[e]) cutCells[index[e]] = static_cast<int>(e);
 }
 
-// Sizes of a cell's moment form: axis d < dim has q1 points, order + 1 functions,
-// m1 = 2 order + 1 Legendre polynomials and `pairs` unordered function pairs; an
-// absent axis has one of each.  DIM and ORDER are compile-time for the common
-// elements (0: taken from the arguments).
-template <int DIM, int ORDER>
-struct FcShape {
-    int dim, n1, m1, pairs, q1;
-    __device__ FcShape(const EmbeddedArgs& P) {
-        dim = DIM ? DIM : P.dim;
-        n1 = (ORDER ? ORDER : P.order) + 1;
-        m1 = 2 * n1 - 1;
-        pairs = n1 * (n1 + 1) / 2;
-        q1 = P.q1;
-    }
-    __device__ __forceinline__ int q(int d) const { return d < dim ? q1 : 1; }
-    __device__ __forceinline__ int m(int d) const { return d < dim ? m1 : 1; }
-    __device__ __forceinline__ int p(int d) const { return d < dim ? pairs : 1; }
-};
-
-constexpr int kFcMoments = 343;                      // most moments of a cell: 7^3 (nb <= 64)
-constexpr int kFcPerLane = (kFcMoments + 31) / 32;
-
-// Shared memory of a CTA in doubles: each warp's tables and planes, then the
-// moments and the arrays of the contraction (the warps' moments alias the latter).
-struct FcSmem {
-    int warp, moments, a, b, k, total;
-};
-__host__ __device__ inline FcSmem fc_smem(int dim, int order, int q1, int warps) {
-    const int m1 = 2 * order + 1, pairs = (order + 1) * (order + 2) / 2;
-    const int mx = m1, my = dim > 1 ? m1 : 1, mz = dim > 2 ? m1 : 1;
-    const int px = pairs, py = dim > 1 ? pairs : 1, pz = dim > 2 ? pairs : 1;
-    FcSmem s;
-    s.warp = 3 * q1 * m1 + q1 * q1 + m1 * q1 + m1 * m1;
-    s.moments = mx * my * mz;
-    s.a = mx * my * pz;
-    s.b = mx * py * pz;
-    s.k = px * py * pz;
-    const int contraction = 2 * s.a + 2 * s.b + s.k, partial = warps * s.moments;
-    s.total = warps * s.warp + s.moments + (contraction > partial ? contraction : partial);
-    return s;
+__device__ __forceinline__ void dmma_8x8x4(double& c0, double& c1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c0), "+d"(c1)
+                 : "d"(a), "d"(b));
 }
 
-// One CTA per cut cell, one warp per start node: the 2^dim children of the root
-// (depth 1) when maxDepth >= 1, else the root.  Each warp walks its subtree
-// depth-first with the rules of KDTreeQuadraturePointFactory.hpp:156-170.
-// pairTable: c0 then c1, [pair (i <= j) at j (j + 1) / 2 + i][m1].
-//   What bounds it: FP64 arithmetic and the latency of its short steps.  The
-// contraction of a cell is 36,000 FMAs (Q3) and a kept tree node 2,600, against
-// 8,192 FMAs for every kept point of the Gram form on the tensor cores (FP64 DMMA),
-// which took 17.7 ms of the 22 ms of the 32^3 Q3 sphere (2,528 cut cells); this
-// kernel takes 0.62 ms of 1.46 ms.  Against a 64-bit evaluation both are 4.1e-15
-// off (2-norm of the matrix).  The FP32 copy came from split-BF16 MMAs, 2.2e-6 off;
-// rounded from these matrices it is 2.9e-8 off.
-template <int DIM, int ORDER, typename V>
-__global__ void __launch_bounds__(256) fc_cell_kernel(EmbeddedArgs P, const int* __restrict__ cutCells, int first,
-                                                      const double* __restrict__ pairTable, V* __restrict__ out) {
-    extern __shared__ double fc_shared[];
-    const FcShape<DIM, ORDER> S(P);
-    const int dim = S.dim, m1 = S.m1, q1 = S.q1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    const FcSmem size = fc_smem(dim, S.n1 - 1, q1, warps);
-    double* s_tab = fc_shared + warp * size.warp;  // [axis][point][polynomial]
-    double* s_w = s_tab + 3 * q1 * m1;             // weights of a plane, x fastest
-    double* s_t1 = s_w + q1 * q1;                  // [y point][x polynomial]
-    double* s_t2 = s_t1 + m1 * q1;                 // [y polynomial][x polynomial]
-    double* s_mu = fc_shared + warps * size.warp;
-    double* s_part = s_mu + size.moments;          // the warps' moments, then the contraction's arrays
-    const int e = cutCells[first + blockIdx.x];
+__device__ __forceinline__ void bmma_16x8x16(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+        "{%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// (x0, x1) -> packed bf16 pairs of their high and low parts (x0 in the low half).
+__device__ __forceinline__ void split_bf16x2(float x0, float x1, unsigned& hi, unsigned& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(x0 - __low2float(h), x1 - __high2float(h));
+    hi = *reinterpret_cast<const unsigned*>(&h);
+    lo = *reinterpret_cast<const unsigned*>(&l);
+}
+
+// Tensor-core accumulator of one CTA's partial element matrix.
+//   FP64: warp w owns rows 8w..8w+7, all 8 column tiles of 8 (DMMA 8x8x4).
+//   FP32: warp w owns rows 16(w/2)..+15, column tiles 4(w%2)..+3 (BF16 16x8x16).
+template <bool F64>
+struct Accumulator;
+
+template <>
+struct Accumulator<true> {
+    double c[8][2];
+    __device__ void zero() {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j][0] = c[j][1] = 0.0;
+    }
+    // rows: staged rows (a multiple of 4, zero-filled); w: their weights.
+    __device__ void add(const double* G, const double* w, int rows, int nt) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (warp >= nt) return;
+        const int col = lane >> 2, kk = lane & 3;
+        for (int k0 = 0; k0 < rows; k0 += 4) {
+            const double* g = G + (k0 + kk) * kFcStride + col;
+            const double a = g[warp * 8] * w[k0 + kk];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j < nt) dmma_8x8x4(c[j][0], c[j][1], a, g[j * 8]);
+        }
+    }
+    __device__ void store(double* out, int nb) const {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int row = warp * 8 + (lane >> 2);
+        if (row >= nb) return;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int col = j * 8 + (lane & 3) * 2 + h;
+                if (col < nb) out[row * nb + col] = c[j][h];
+            }
+    }
+};
+
+template <>
+struct Accumulator<false> {
+    float c[4][4];
+    __device__ void zero() {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.0f;
+    }
+    // rows: staged rows (a multiple of 16, zero-filled).  nt16: row tiles of 16,
+    // nt8: column tiles of 8 in use.
+    __device__ void add(const double* G, const double* w, int rows, int nt16, int nt8) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int tr = warp >> 1, tc0 = (warp & 1) * 4;
+        if (tr >= nt16 || tc0 >= nt8) return;
+        const int g = lane >> 2, t = lane & 3;
+        for (int k0 = 0; k0 < rows; k0 += 16) {
+            // A[i][k] = w_k G[k][16 tr + i]: (g, 2t..2t+1), (g+8, ..), (g, 2t+8..), (g+8, 2t+8..)
+            unsigned ahi[4], alo[4];
+            const int ks[2] = {k0 + 2 * t, k0 + 2 * t + 8};
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int k = ks[half];
+                const double w0 = w[k], w1 = w[k + 1];
+#pragma unroll
+                for (int rr = 0; rr < 2; ++rr) {
+                    const int i = tr * 16 + g + rr * 8;
+                    split_bf16x2(static_cast<float>(w0 * G[k * kFcStride + i]),
+                                 static_cast<float>(w1 * G[(k + 1) * kFcStride + i]), ahi[half * 2 + rr],
+                                 alo[half * 2 + rr]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (tc0 + j >= nt8) break;
+                const int n = (tc0 + j) * 8 + g;
+                unsigned bhi[2], blo[2];
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int k = ks[half];
+                    split_bf16x2(static_cast<float>(G[k * kFcStride + n]), static_cast<float>(G[(k + 1) * kFcStride + n]),
+                                 bhi[half], blo[half]);
+                }
+                bmma_16x8x16(c[j], ahi, bhi);
+                bmma_16x8x16(c[j], ahi, blo);
+                bmma_16x8x16(c[j], alo, bhi);
+            }
+        }
+    }
+    __device__ void store(float* out, int nb) const {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int tr = warp >> 1, tc0 = (warp & 1) * 4;
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int row = tr * 16 + g + (h >> 1) * 8;
+                const int col = (tc0 + j) * 8 + t * 2 + (h & 1);
+                if (row < nb && col < nb) out[row * nb + col] = c[j][h];
+            }
+    }
+};
+
+// One CTA per (cut cell of the batch, start node).  Start nodes: the 2^dim
+// children of the root (depth 1) when maxDepth >= 1, else the root.  The CTA
+// walks the start node's subtree depth-first with the rules of
+// KDTreeQuadraturePointFactory.hpp:156-170 and adds the kept points' terms.
+template <bool F64>
+__global__ void __launch_bounds__(kFcThreads)
+    fc_partial_kernel(EmbeddedArgs P, const int* __restrict__ cutCells, int first, int nstart,
+                      typename std::conditional<F64, double, float>::type* __restrict__ partial) {
+    __shared__ double s_G[kFcRows * kFcStride];
+    __shared__ double s_w[kFcRows];
+    __shared__ double s_v[kFcPoints][3][16], s_dv[kFcPoints][3][16];
+    __shared__ double s_stack[kFcStack][4];  // base[3], length
+    __shared__ int s_stackDepth[kFcStack];
+    __shared__ int s_top;
+    __shared__ double s_node[4];
+    __shared__ int s_nodeDepth;
+    __shared__ int s_inside;
+    const int t = threadIdx.x;
+    const int dim = P.dim, nb = P.nb, nq = P.nq, n1 = P.order + 1;
+    const int item = blockIdx.x;
+    const int e = cutCells[first + item / nstart];
+    const int startChild = item % nstart;
     double corg[3] = {0.0, 0.0, 0.0};
     {
         long rest = e;
@@ -146,218 +243,120 @@ __global__ void __launch_bounds__(256) fc_cell_kernel(EmbeddedArgs P, const int*
             rest /= P.cells[d];
         }
     }
-    const int nq = P.nq;
-    const int qx = S.q(0), qy = S.q(1), qz = S.q(2), mx = S.m(0), my = S.m(1), mz = S.m(2);
-    const int mxy = mx * my;
-    double acc[kFcPerLane];
-#pragma unroll
-    for (int j = 0; j < kFcPerLane; ++j) acc[j] = 0.0;
-    const int d0 = P.maxDepth >= 1 ? 1 : 0, digit = (1 << dim) - 1;
-    int depth = d0, code = d0 ? warp : 0;  // `dim` bits of the child number a level below the root
-    for (;;) {
-        double base[3] = {-1.0, -1.0, -1.0};
-        double length = 2.0;
-        for (int level = 1; level <= depth; ++level) {
-            length *= 0.5;
-            const int child = (code >> (dim * (depth - level))) & digit;
-            for (int d = 0; d < dim; ++d)
-                if ((child >> d) & 1) base[d] += length;
+    Accumulator<F64> acc;
+    acc.zero();
+    const int nt8 = (nb + 7) / 8, nt16 = (nb + 15) / 16;
+    if (t == 0) {
+        s_top = 1;
+        if (nstart == 1) {
+            s_stack[0][0] = s_stack[0][1] = s_stack[0][2] = -1.0;
+            s_stack[0][3] = 2.0;
+            s_stackDepth[0] = 0;
+        } else {
+            for (int d = 0; d < 3; ++d) s_stack[0][d] = d < dim ? -1.0 + ((startChild >> d) & 1) : -1.0;
+            s_stack[0][3] = 1.0;
+            s_stackDepth[0] = 1;
         }
-        int inside = 0;
-        for (int q = lane; q < nq; q += 32) {
+    }
+    __syncthreads();
+    for (;;) {
+        const int top = s_top;  // every thread reads it before thread 0 pops
+        __syncthreads();
+        if (top == 0) break;
+        if (t == 0) {
+            const int k = --s_top;
+            for (int j = 0; j < 4; ++j) s_node[j] = s_stack[k][j];
+            s_nodeDepth = s_stackDepth[k];
+        }
+        __syncthreads();
+        const double base[3] = {s_node[0], s_node[1], s_node[2]};
+        const double length = s_node[3];
+        const int depth = s_nodeDepth;
+        int mine = 0;
+        for (int q = t; q < nq; q += kFcThreads) {
             double xi[3];
             embedded_point(P, base, length, q, xi);
-            inside += embedded_inside(P, corg, xi) ? 1 : 0;
+            mine += embedded_inside(P, corg, xi) ? 1 : 0;
         }
-        inside = __reduce_add_sync(0xffffffffu, inside);
-        const bool homogeneous = inside == 0 || inside == nq;
-        const bool keep = inside == nq || depth == P.maxDepth || (depth == 0 && homogeneous);
+        // number of inside points of the node
+        if (t == 0) s_inside = 0;
+        __syncthreads();
+        if (mine) atomicAdd(&s_inside, mine);
+        __syncthreads();
+        const int nin = s_inside;
+        const bool homogeneous = nin == 0 || nin == nq;
+        const bool keep = (homogeneous && nin == nq) || depth == P.maxDepth || (depth == 0 && homogeneous);
         if (keep) {
             double jac = 1.0;
             for (int d = 0; d < dim; ++d) jac *= 0.5 * length;
-            // P_a at the node's points of each axis, by the three-term recurrence
-            for (int t = lane; t < 3 * q1; t += 32) {
-                const int d = t / q1, i = t - d * q1;
-                double* tab = s_tab + t * m1;
-                const double x = base[d] + 0.5 * length * (P.gn[i] + 1.0);
-                double p0 = 1.0, p1 = x;
-                tab[0] = 1.0;
-                for (int k = 1; k < m1; ++k) {
-                    tab[k] = p1;
-                    const double p2 = ((2.0 * k + 1.0) * x * p1 - k * p0) / (k + 1.0);
-                    p0 = p1;
-                    p1 = p2;
-                }
-            }
-            __syncwarp();
-            for (int z = 0; z < qz; ++z) {
-                for (int t = lane; t < qx * qy; t += 32) {
+            for (int q0 = 0; q0 < nq; q0 += kFcPoints) {
+                const int np = min(kFcPoints, nq - q0);
+                const int rows = np * dim;
+                const int padded = F64 ? (rows + 3) & ~3 : (rows + 15) & ~15;
+                if (t < np * dim) {
+                    const int p = t / dim, d = t - (t / dim) * dim;
                     double xi[3];
-                    const double w = embedded_point(P, base, length, z * qx * qy + t, xi) * jac;
-                    s_w[t] = w * (embedded_inside(P, corg, xi) ? 1.0 : P.alpha);
+                    embedded_point(P, base, length, q0 + p, xi);
+                    lagrange(P.order, xi[d], s_v[p][d], s_dv[p][d]);
                 }
-                __syncwarp();
-                for (int t = lane; t < mx * qy; t += 32) {
-                    const int y = t / mx, a = t - y * mx;
-                    double s = 0.0;
-                    for (int x = 0; x < qx; ++x) s = fma(s_w[y * qx + x], s_tab[x * m1 + a], s);
-                    s_t1[t] = s;
+                if (t < np) {
+                    double xi[3];
+                    const double w = embedded_point(P, base, length, q0 + t, xi) * jac *
+                                     (embedded_inside(P, corg, xi) ? 1.0 : P.alpha);
+                    for (int d = 0; d < dim; ++d) s_w[t * dim + d] = w * P.f[d];
                 }
-                __syncwarp();
-                for (int t = lane; t < mxy; t += 32) {
-                    const int b = t / mx, a = t - b * mx;
-                    double s = 0.0;
-                    for (int y = 0; y < qy; ++y) s = fma(s_t1[y * mx + a], s_tab[(q1 + y) * m1 + b], s);
-                    s_t2[t] = s;
-                }
-                __syncwarp();
-                const double* pz = s_tab + (2 * q1 + z) * m1;
-#pragma unroll
-                for (int j = 0; j < kFcPerLane; ++j) {
-                    const int t = lane + 32 * j;
-                    if (t < size.moments) {
-                        const int c = t / mxy;
-                        acc[j] = fma(s_t2[t - c * mxy], pz[c], acc[j]);
+                for (int r = rows + t; r < padded; r += kFcThreads) s_w[r] = 0.0;
+                __syncthreads();
+                // B rows (point p, axis dd): G[a] = prod_d (d == dd ? dN : N)_{i_d(a)}; columns >= nb are 0
+                for (int idx = t; idx < padded * 64; idx += kFcThreads) {
+                    const int r = idx >> 6, a = idx & 63;
+                    double g = 0.0;
+                    if (r < rows && a < nb) {
+                        const int p = r / dim, dd = r - (r / dim) * dim;
+                        int ra = a;
+                        g = 1.0;
+                        for (int d = 0; d < dim; ++d) {
+                            const int i = ra % n1;
+                            ra /= n1;
+                            g *= (d == dd) ? s_dv[p][d][i] : s_v[p][d][i];
+                        }
                     }
+                    s_G[r * kFcStride + a] = g;
                 }
-                __syncwarp();
+                __syncthreads();
+                if constexpr (F64)
+                    acc.add(s_G, s_w, padded, nt8);
+                else
+                    acc.add(s_G, s_w, padded, nt16, nt8);
+                __syncthreads();
             }
         }
-        if (!homogeneous && depth < P.maxDepth) {
-            code <<= dim;
-            ++depth;
-            continue;
-        }
-        while (depth > d0 && (code & digit) == digit) {
-            code >>= dim;
-            --depth;
-        }
-        if (depth == d0) break;
-        ++code;
-    }
-#pragma unroll
-    for (int j = 0; j < kFcPerLane; ++j) {
-        const int t = lane + 32 * j;
-        if (t < size.moments) s_part[warp * size.moments + t] = acc[j];
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < size.moments; t += blockDim.x) {
-        double s = 0.0;
-        for (int w = 0; w < warps; ++w) s += s_part[w * size.moments + t];
-        s_mu[t] = s;
-    }
-    __syncthreads();
-    // Contraction, z then y then x.  Per axis only one of the three factors is a
-    // product of derivatives, so two arrays are carried: "0" without a derivative
-    // yet, "1" the sum of those with one (times their f).
-    const int px = S.p(0), py = S.p(1), pz = S.p(2);
-    double* s_a0 = s_part;
-    double* s_a1 = s_a0 + size.a;
-    double* s_b0 = s_a1 + size.a;
-    double* s_b1 = s_b0 + size.b;
-    double* s_k = s_b1 + size.b;
-    const double* c0 = pairTable;
-    const double* c1 = pairTable + S.pairs * m1;
-    for (int t = threadIdx.x; t < size.a; t += blockDim.x) {
-        const int p = t / mxy, ab = t - p * mxy;
-        double s0 = 0.0, s1 = 0.0;
-        if (dim > 2) {
-            for (int c = 0; c < mz; ++c) {
-                const double mu = s_mu[c * mxy + ab];
-                s0 = fma(mu, c0[p * m1 + c], s0);
-                s1 = fma(mu, c1[p * m1 + c], s1);
+        if (t == 0 && !homogeneous && depth < P.maxDepth) {
+            const double half = 0.5 * length;
+            const int children = 1 << dim;
+            for (int c = children - 1; c >= 0; --c) {  // pushed in reverse: child 0 is visited first
+                const int k = s_top++;
+                for (int d = 0; d < 3; ++d) s_stack[k][d] = d < dim ? base[d] + ((c >> d) & 1) * half : -1.0;
+                s_stack[k][3] = half;
+                s_stackDepth[k] = depth + 1;
             }
-        } else {
-            s0 = s_mu[ab];
         }
-        s_a0[t] = s0;
-        s_a1[t] = s1 * P.f[2];
+        __syncthreads();
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < size.b; t += blockDim.x) {
-        const int pp = t / mx, a = t - pp * mx;  // pp = (z pair, y pair), y fastest
-        const int pzi = pp / py, pyi = pp - pzi * py;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-        if (dim > 1) {
-            for (int b = 0; b < my; ++b) {
-                const double v0 = s_a0[pzi * mxy + b * mx + a], v1 = s_a1[pzi * mxy + b * mx + a];
-                s0 = fma(v0, c0[pyi * m1 + b], s0);
-                s1 = fma(v0, c1[pyi * m1 + b], s1);
-                s2 = fma(v1, c0[pyi * m1 + b], s2);
-            }
-        } else {
-            s0 = s_a0[a];
-        }
-        s_b0[t] = s0;
-        s_b1[t] = fma(s1, P.f[1], s2);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < size.k; t += blockDim.x) {
-        const int pp = t / px, pxi = t - pp * px;
-        double s0 = 0.0, s1 = 0.0;
-        for (int a = 0; a < mx; ++a) {
-            s0 = fma(s_b0[pp * mx + a], c1[pxi * m1 + a], s0);
-            s1 = fma(s_b1[pp * mx + a], c0[pxi * m1 + a], s1);
-        }
-        s_k[t] = fma(s0, P.f[0], s1);
-    }
-    __syncthreads();
-    const int n1 = S.n1;
-    int nb = 1;
-    for (int d = 0; d < dim; ++d) nb *= n1;
-    V* o = out + static_cast<long>(blockIdx.x) * nb * nb;
-    auto pair = [](int i, int j) { return i < j ? j * (j + 1) / 2 + i : i * (i + 1) / 2 + j; };
-    for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {
-        const int a = t / nb, b = t - a * nb;
-        int at = pair(a % n1, b % n1);
-        if (dim > 1) at += px * pair((a / n1) % n1, (b / n1) % n1);
-        if (dim > 2) at += px * py * pair(a / (n1 * n1), b / (n1 * n1));
-        o[t] = static_cast<V>(s_k[at]);
-    }
-    (void)pz;
+    acc.store(partial + static_cast<long>(item) * nb * nb, nb);
 }
 
-template <int DIM, int ORDER, typename V>
-int launch_cells(const EmbeddedArgs& A, const int* cutCells, long first, long count, const double* pairTable, V* out,
-                 cudaStream_t st) {
-    const int warps = A.maxDepth >= 1 ? (1 << A.dim) : 1;
-    const size_t smem = sizeof(double) * fc_smem(A.dim, A.order, A.q1, warps).total;
-    auto kernel = fc_cell_kernel<DIM, ORDER, V>;
-    CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    kernel<<<static_cast<unsigned>(count), 32 * warps, smem, st>>>(A, cutCells, static_cast<int>(first), pairTable, out);
-    count_launch();
-    CIECU_CHECK_LAUNCH("fc_cell_kernel");
-    return CIECU_OK;
-}
-
-// c0 and c1 of the 1-D basis: coefficients (2a + 1)/2 int f P_a of the products f,
-// by a Gauss rule that is exact for them (degree 4 order).
-std::vector<double> pair_table(int order) {
-    const int n1 = order + 1, m1 = 2 * order + 1, pairs = n1 * (n1 + 1) / 2;
-    std::vector<double> x, w, out(static_cast<size_t>(2 * pairs * m1), 0.0);
-    gauss_legendre(m1, x, w);
-    for (int a = 0; a < m1; ++a)
-        for (int j = 0, at = 0; j < n1; ++j)
-            for (int i = 0; i <= j; ++i, ++at) {
-                long double s0 = 0.0L, s1 = 0.0L;
-                for (int q = 0; q < m1; ++q) {
-                    double v[16], dv[16];
-                    lagrange(order, x[q], v, dv);
-                    long double p0 = 1.0L, p1 = x[q];
-                    for (int k = 1; k <= a; ++k) {
-                        const long double p2 = ((2 * k + 1) * static_cast<long double>(x[q]) * p1 - k * p0) / (k + 1);
-                        p0 = p1;
-                        p1 = p2;
-                    }
-                    s0 += static_cast<long double>(w[q]) * v[i] * v[j] * p0;
-                    s1 += static_cast<long double>(w[q]) * dv[i] * dv[j] * p0;
-                }
-                out[static_cast<size_t>(at) * m1 + a] = static_cast<double>((2 * a + 1) * s0 / 2);
-                // the products of derivatives have degree 2 order - 2
-                out[static_cast<size_t>(pairs + at) * m1 + a] =
-                    a <= 2 * order - 2 ? static_cast<double>((2 * a + 1) * s1 / 2) : 0.0;
-            }
-    return out;
+// A cut cell's matrix: its partial matrices in start-node order.
+template <typename V>
+__global__ void fc_sum_kernel(long total, int nb2, int nstart, const V* __restrict__ partial, V* __restrict__ matrix) {
+    for (long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; t < total;
+         t += static_cast<long>(gridDim.x) * blockDim.x) {
+        const long cell = t / nb2;
+        const V* part = partial + cell * nstart * nb2 + (t - cell * nb2);
+        V sum = V(0);
+        for (int j = 0; j < nstart; ++j) sum += part[static_cast<long>(j) * nb2];
+        matrix[t] = sum;
+    }
 }
 
 // The row gather's cells: regular cells kappa s K1 (first batch only), the cut
@@ -434,28 +433,27 @@ int assemble_finite_cell(ciecu_assembly_s* P, const double* d_kappa, const doubl
     double f[3];
     convention_factors(P->dim, h_cellSize, convention, A.scale, f);
     for (int d = 0; d < 3; ++d) A.f[d] = f[d];
-    // batches of cut cells whose matrices fit in 512 MB
-    const long perCut = nb2 * static_cast<long>(sizeof(V));
+    const int nstart = maxDepth >= 1 ? (1 << P->dim) : 1;
+    // batches of cut cells whose partial matrices fit in 512 MB
+    const long perCut = static_cast<long>(nstart) * nb2 * static_cast<long>(sizeof(V));
     const long batchCap = std::max<long>(1, (512L << 20) / perCut);
-    // work: K1 (FP64 and V), the pair table, cut flags, their prefix sum, cut list, sides, scan work
-    const std::vector<double> pairs = pair_table(P->order);
+    // work: K1 (FP64 and V), cut flags, their prefix sum, cut list, sides, scan work
     const long scanWork = scan_work(ncells);
-    const size_t bytes = sizeof(double) * (nb2 + pairs.size()) + sizeof(V) * nb2 +
+    const size_t bytes = sizeof(double) * nb2 + sizeof(V) * nb2 +
                          sizeof(int) * (3 * static_cast<size_t>(ncells) + 1 + static_cast<size_t>(scanWork)) +
                          static_cast<size_t>(ncells) + 256;
     unsigned char* work = nullptr;
     CIECU_CUDA(pool_alloc(&work, bytes, st));
-    V* matrices = nullptr;
+    V *partial = nullptr, *matrices = nullptr;
     auto done = [&](int status) {  // stream-ordered: the kernels that use them come first
+        if (partial) cudaFreeAsync(partial, st);
         if (matrices) cudaFreeAsync(matrices, st);
         cudaFreeAsync(work, st);
         return status;
     };
     double* K1 = reinterpret_cast<double*>(work);
-    double* pairTable = K1 + nb2;
-    V* K1v = reinterpret_cast<V*>(pairTable + pairs.size());
-    int* cut = reinterpret_cast<int*>(
-        work + ((sizeof(double) * (nb2 + pairs.size()) + sizeof(V) * nb2 + 15) & ~size_t(15)));
+    V* K1v = reinterpret_cast<V*>(K1 + nb2);
+    int* cut = reinterpret_cast<int*>(work + ((sizeof(double) * nb2 + sizeof(V) * nb2 + 15) & ~size_t(15)));
     int* index = cut + ncells;       // ncells + 1
     int* cutCells = index + ncells + 1;
     int* scan = cutCells + ncells;
@@ -475,32 +473,27 @@ int assemble_finite_cell(ciecu_assembly_s* P, const double* d_kappa, const doubl
     if (status != CIECU_OK) return done(status);
     fc_compact_kernel<<<grid_for(ncells, 256, 8), 256, 0, st>>>(ncells, cut, index, cutCells);
     count_launch();
-    cudaError_t e = cudaMemcpyAsync(pairTable, pairs.data(), sizeof(double) * pairs.size(), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return done(cuda_fail(e, "assemble_embedded: pair table"));
     int ncut = 0;
-    e = cudaMemcpyAsync(&ncut, index + ncells, sizeof(int), cudaMemcpyDeviceToHost, st);
+    cudaError_t e = cudaMemcpyAsync(&ncut, index + ncells, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return done(cuda_fail(e, "assemble_embedded: classification"));
     const long batch = std::min<long>(std::max(ncut, 1), batchCap);
     if (ncut > 0) {
-        e = pool_alloc(&matrices, static_cast<size_t>(batch * perCut), st);
+        e = pool_alloc(&partial, static_cast<size_t>(batch * perCut), st);
+        if (e == cudaSuccess) e = pool_alloc(&matrices, static_cast<size_t>(batch) * nb2 * sizeof(V), st);
         if (e != cudaSuccess) return done(cuda_fail(e, "assemble_embedded: cut-cell matrices"));
     }
     V* val = static_cast<V*>(d_entries);
     for (long b0 = 0; b0 < std::max<long>(ncut, 1); b0 += batch) {
         const long b1 = std::min<long>(ncut, b0 + batch);
         if (b1 > b0) {
-            const int shape = A.dim * 10 + A.order;
-            auto cells = [&](auto d, auto p) {
-                return launch_cells<decltype(d)::value, decltype(p)::value, V>(A, cutCells, b0, b1 - b0, pairTable,
-                                                                               matrices, st);
-            };
-            using std::integral_constant;
-            if (shape == 33) status = cells(integral_constant<int, 3>{}, integral_constant<int, 3>{});
-            else if (shape == 32) status = cells(integral_constant<int, 3>{}, integral_constant<int, 2>{});
-            else if (shape == 31) status = cells(integral_constant<int, 3>{}, integral_constant<int, 1>{});
-            else status = cells(integral_constant<int, 0>{}, integral_constant<int, 0>{});
-            if (status != CIECU_OK) return done(status);
+            fc_partial_kernel<F64><<<static_cast<unsigned>((b1 - b0) * nstart), kFcThreads, 0, st>>>(
+                A, cutCells, static_cast<int>(b0), nstart, partial);
+            const long entries = (b1 - b0) * nb2;
+            fc_sum_kernel<V><<<grid_for(entries, 256, 8), 256, 0, st>>>(entries, nb2, nstart, partial, matrices);
+            count_launch(2);
+            e = cudaGetLastError();
+            if (e != cudaSuccess) return done(cuda_fail(e, "assemble_embedded"));
         }
         status = launch_row_gather<V>(P,
                                       FiniteCellSource<V>{cut, index, side, matrices, d_kappa, alpha, A.scale, nb2,

@@ -219,7 +219,7 @@ def make_two_level_cg(space, problem, settings, center=None, radius=0.4, alpha=1
                       coarseIterations=8, ratio=30.0, flexible=True, precision="f64"):
     """The device two-level CG of a finite-cell problem made by
     make_embedded_poisson (same sphere, factor and tree).  precision "f32"
-    smooths on the FP32 copy of the finite-cell matrix
+    smooths on the FP32 matrix assembled with the tensor-core contraction
     (ciecu_assemble_embedded_f32) and eliminated like the FP64 one."""
     fine, fineD, mg = make_two_level(space, problem, center=center, radius=radius, alpha=alpha, depth=depth,
                                      degree=degree)

@@ -102,7 +102,7 @@ public:
                                       entries.data(), _work.get(), &cut));
         return cut;
     }
-    // The same matrix in FP32 (the FP64 element matrices rounded).
+    // The same matrix in FP32 with the contraction on the tensor cores.
     int64_t finiteCellF32(std::array<double, 3> center, double radius, double alpha, int maxDepth,
                           CUDAView<float> entries32, CUDAView<const double> kappa = {}, bool accumulate = false) {
         int64_t cut = 0;

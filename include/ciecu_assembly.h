@@ -51,8 +51,8 @@ int ciecu_assemble_stiffness(ciecu_assembly plan, const double* d_kappa, const d
  * homogeneous and inside, at the maximum depth, or homogeneous at depth 0, and
  * refined while not homogeneous.  K_e in FP64, convention as
  * ciecu_assemble_stiffness; d_kappa may be NULL (kappa = 1).  The plan's basis has
- * at most 64 functions.  The points of a cut cell enter through its Legendre
- * moments (one CTA per cut cell, FP64), and every CSR entry sums its cells in
+ * at most 64 functions.  The cut cells' Gram contractions run on the tensor cores
+ * in FP64 (one CTA per depth-1 tree node), and every CSR entry sums its cells in
  * colour order, so the result does not depend on the schedule.
  * d_work: nb*nb doubles (kept for the interface; the call allocates its own
  * work arrays).  h_cutCells (may be NULL): the number of cut cells.  The call
@@ -64,7 +64,10 @@ int ciecu_assemble_embedded(ciecu_assembly plan, const double* d_kappa, const do
 
 /* The same finite-cell matrix in single precision, for inner or preconditioner
  * operators: d_entries32 (FP32 values in the plan's CSR pattern) (+)= the element
- * matrices, computed in FP64 as above and rounded to FP32 before they are summed. */
+ * matrices with the Gram contraction B^T W B on the tensor cores in BF16 with
+ * FP32 accumulation, each operand split into a high and a low BF16 part and the
+ * three significant products summed (about 16 significant bits per product); the
+ * regular cells add the FP64 standard-rule matrix rounded to FP32. */
 int ciecu_assemble_embedded_f32(ciecu_assembly plan, const double* d_kappa, const double* h_cellSize,
                                 const int32_t* h_cells, const double* h_origin, const double* h_center, double radius,
                                 double alpha, int maxDepth, int convention, int accumulate, float* d_entries32,

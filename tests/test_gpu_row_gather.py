@@ -1,8 +1,8 @@
 """The row-gather assembly at the sizes where its paths change: element sizes with
 and without a compile-time kernel, more incident cells per row than a group of
 lanes holds, rows too long for shared memory, 16-bit positions; the elimination
-over column arrays that do not start on a 16-byte boundary; and the moment form
-of the cut cells at orders, rules and depths of its runtime-sized kernel.  All
+over column arrays that do not start on a 16-byte boundary; and cut cells
+at other orders, rules and depths.  All
 against the restatement, with the tolerances of the other assembly tests."""
 from types import SimpleNamespace
 

@@ -20,8 +20,10 @@
 //      standard-rule matrix), cut cells the sum of their partials in node order.
 //      The result does not depend on the schedule.
 //
-// What bounds it: the walk's barriers and the staging of the gradients (tensor pipe 21 %
-// active), 18 ms of 19.3 at 32^3 Q3 with 2,528 cut cells.  The points enter an element matrix only
+// What bounds it: the walk's barriers and the products, about 6 ms of FP64 MMAs of 9.8 ms at
+// 32^3 Q3 with 2,528 cut cells.  The basis is evaluated once a node and axis, and a thread
+// stages one column for all points, its functions known from the start (evaluated at every
+// point, with divisions for every staged value: 19.3 ms, the same bits).  The points enter an element matrix only
 // through their (2p + 1)^dim Legendre moments, and formed from those the same matrices take
 // 1.5 ms, 2.5e-16 from these in the 2-norm; but with alpha = 1e-6 the solution hears the
 // rounding of the matrix 1e7 times louder, and came out up to 1.5e-9 elsewhere.
@@ -223,7 +225,8 @@ __global__ void __launch_bounds__(kFcThreads)
                       typename std::conditional<F64, double, float>::type* __restrict__ partial) {
     __shared__ double s_G[kFcRows * kFcStride];
     __shared__ double s_w[kFcRows];
-    __shared__ double s_v[kFcPoints][3][16], s_dv[kFcPoints][3][16];
+    __shared__ double s_v[3][16][16], s_dv[3][16][16];  // of the node's 1D points: axis, point, function
+    __shared__ int s_at[kFcPoints][3];
     __shared__ double s_stack[kFcStack][4];  // base[3], length
     __shared__ int s_stackDepth[kFcStack];
     __shared__ int s_top;
@@ -246,6 +249,8 @@ __global__ void __launch_bounds__(kFcThreads)
     Accumulator<F64> acc;
     acc.zero();
     const int nt8 = (nb + 7) / 8, nt16 = (nb + 15) / 16;
+    const int column = t & 63;
+    int fn[3] = {column % n1, column / n1 % n1, column / (n1 * n1) % n1};  // the column's function on each axis
     if (t == 0) {
         s_top = 1;
         if (nstart == 1) {
@@ -289,40 +294,45 @@ __global__ void __launch_bounds__(kFcThreads)
         if (keep) {
             double jac = 1.0;
             for (int d = 0; d < dim; ++d) jac *= 0.5 * length;
+            if (t < dim * P.q1) {
+                const int d = t / P.q1, i = t - d * P.q1;
+                double xi[3];
+                embedded_point(P, base, length, d == 0 ? i : (d == 1 ? i * P.q1 : i * P.q1 * P.q1), xi);
+                lagrange(P.order, xi[d], s_v[d][i], s_dv[d][i]);
+            }
             for (int q0 = 0; q0 < nq; q0 += kFcPoints) {
                 const int np = min(kFcPoints, nq - q0);
                 const int rows = np * dim;
                 const int padded = F64 ? (rows + 3) & ~3 : (rows + 15) & ~15;
-                if (t < np * dim) {
-                    const int p = t / dim, d = t - (t / dim) * dim;
-                    double xi[3];
-                    embedded_point(P, base, length, q0 + p, xi);
-                    lagrange(P.order, xi[d], s_v[p][d], s_dv[p][d]);
-                }
                 if (t < np) {
                     double xi[3];
                     const double w = embedded_point(P, base, length, q0 + t, xi) * jac *
                                      (embedded_inside(P, corg, xi) ? 1.0 : P.alpha);
                     for (int d = 0; d < dim; ++d) s_w[t * dim + d] = w * P.f[d];
+                    int rest = q0 + t;
+                    for (int d = 0; d < 3; ++d) {
+                        s_at[t][d] = rest % P.q1;
+                        rest /= P.q1;
+                    }
                 }
                 for (int r = rows + t; r < padded; r += kFcThreads) s_w[r] = 0.0;
                 __syncthreads();
                 // B rows (point p, axis dd): G[a] = prod_d (d == dd ? dN : N)_{i_d(a)}; columns >= nb are 0
-                for (int idx = t; idx < padded * 64; idx += kFcThreads) {
-                    const int r = idx >> 6, a = idx & 63;
-                    double g = 0.0;
-                    if (r < rows && a < nb) {
-                        const int p = r / dim, dd = r - (r / dim) * dim;
-                        int ra = a;
-                        g = 1.0;
-                        for (int d = 0; d < dim; ++d) {
-                            const int i = ra % n1;
-                            ra /= n1;
-                            g *= (d == dd) ? s_dv[p][d][i] : s_v[p][d][i];
-                        }
+                // (a thread's column is the same for all rows)
+                for (int p = t >> 6; p < np; p += kFcThreads / 64) {
+                    double v[3], dv[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        v[d] = d < dim ? s_v[d][s_at[p][d]][fn[d]] : 1.0;
+                        dv[d] = d < dim ? s_dv[d][s_at[p][d]][fn[d]] : 1.0;
                     }
-                    s_G[r * kFcStride + a] = g;
+                    double* g = s_G + p * dim * kFcStride + column;
+                    const bool in = column < nb;
+                    g[0] = in ? dv[0] * v[1] * v[2] : 0.0;
+                    if (dim > 1) g[kFcStride] = in ? v[0] * dv[1] * v[2] : 0.0;
+                    if (dim > 2) g[2 * kFcStride] = in ? v[0] * v[1] * dv[2] : 0.0;
                 }
+                for (int r = rows + (t >> 6); r < padded; r += kFcThreads / 64) s_G[r * kFcStride + column] = 0.0;
                 __syncthreads();
                 if constexpr (F64)
                     acc.add(s_G, s_w, padded, nt8);

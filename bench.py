@@ -582,7 +582,7 @@ def profile_target(space, target, cells, schedule=0):
         solver.product(0.0, B, 1.0, X)
         info = solver.info()
     elif target == "embedded":
-        # the FP64 assembly inside the set-up, then the FP32 one
+        # the FP64 (DMMA) assembly inside the set-up, then the FP32 (split-BF16) one
         c = cells if cells <= 32 else 16
         prob = make_embedded_poisson(space, 3, 3, [c, c, c], radius=0.4, alpha=1e-6, depth=2)
         v32 = torch.zeros(prob.matrix.entries.numel(), dtype=torch.float32, device="cuda")

@@ -403,7 +403,6 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
         e = pool_alloc(&P->d_pos, std::max<size_t>(1, static_cast<size_t>(incidences) * nb * P->posBytes), st);
     if (e == cudaSuccess) e = pool_alloc(&P->d_gtab, sizeof(double) * gtab.size(), st);
     if (e == cudaSuccess) e = pool_alloc(&P->d_wq, sizeof(double) * wq.size(), st);
-    if (e == cudaSuccess) e = pool_alloc(&P->d_unit, sizeof(double) * nb * nb, st);
     if (e == cudaSuccess) e = pool_alloc(&scratch, sizeof(int) * scratchInts, st);
     int* d_order = scratch;
     int* d_count = scratch + ncells;
@@ -475,7 +474,7 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
 int ciecu_assembly_destroy(ciecu_assembly P) {
     if (!P) return CIECU_OK;
     // No access to P->csr (it may already be gone); pool_release synchronises the device.
-    pool_release({P->d_incStart, P->d_inc, P->d_pos, P->d_gtab, P->d_wq, P->d_unit});
+    pool_release({P->d_incStart, P->d_inc, P->d_pos, P->d_gtab, P->d_wq});
     delete P;
     return CIECU_OK;
 }
@@ -495,9 +494,17 @@ int ciecu_assemble_stiffness(ciecu_assembly P, const double* d_kappa, const doub
     convention_factors(P->dim, h_cellSize, convention, scale, f);
     // the reference element's sums, once per call: each contribution to an entry is
     // fma(kappa_e scale, S[a][b], entry), one rounding, so that the host restatement
-    // of this summation order reproduces the matrix bit for bit
-    CIECU_TRY(unit_element(P, 1.0, f, P->d_unit, st));
-    return launch_row_gather<double>(P, UniformSource{d_kappa, scale}, P->d_unit, accumulate ? 1 : 0, d_entries, st);
+    // of this summation order reproduces the matrix bit for bit.  The sums belong to
+    // the call, not to the plan: threads may assemble with one plan and different cell
+    // sizes or conventions, and a captured call may be replayed beside another.
+    double* unit = nullptr;
+    CIECU_CUDA(pool_alloc(&unit, sizeof(double) * P->nb * P->nb, st));
+    int status = unit_element(P, 1.0, f, unit, st);
+    if (status == CIECU_OK)
+        status = launch_row_gather<double>(P, UniformSource{d_kappa, scale}, unit, accumulate ? 1 : 0, d_entries, st);
+    const cudaError_t e = cudaFreeAsync(unit, st);  // stream-ordered: after the gather
+    if (status == CIECU_OK && e != cudaSuccess) return cuda_fail(e, "assemble_stiffness: free");
+    return status;
 }
 
 int ciecu_element_gradient(ciecu_assembly P, const double* h_cellSize, int convention, const double* d_lambda,

@@ -28,7 +28,6 @@ struct ciecu_assembly_s {
     int colors = 0;
     double* d_gtab = nullptr;         // nq * dim * nb parametric gradients
     double* d_wq = nullptr;           // nq weights
-    double* d_unit = nullptr;         // nb * nb: the reference element's sums of the current call
     int q1 = 0;                       // 1-D quadrature points (nq = q1^dim)
     std::vector<double> gn, gw;       // 1-D Gauss-Legendre rule on [-1, 1]
 };

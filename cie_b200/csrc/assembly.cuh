@@ -261,8 +261,7 @@ int launch_row_gather_nb(const ciecu_assembly_s* P, const SRC& src, const V* bas
     const size_t smem = (G.stagedBase ? baseBytes : 0) +
                         (G.rowStride ? sizeof(V) * static_cast<size_t>(rowsPerBlock) * G.rowStride : 0);
     auto kernel = row_gather_kernel<V, POS, NB, SRC>;
-    CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kGatherBaseBytes + kGatherRowBytes + 64)));
+    CIECU_TRY(allow_shared(kernel));
     const long blocks = (static_cast<long>(G.rows) + rowsPerBlock - 1) / rowsPerBlock;
     kernel<<<fit_grid(kernel, kGatherThreads, blocks, smem), kGatherThreads, smem, st>>>(G, src, base, val);
     count_launch();

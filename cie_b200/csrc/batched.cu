@@ -902,8 +902,7 @@ int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
     a.waitNs = kBatchWaitNs;
     a.withholdEpoch = 0;
     BatchCtl::Shared shared{B->d_g, g0.maxIter, kBatchLaunchIterations, g0.absTol, g0.relTol};
-    CIECU_CUDA(cudaFuncSetAttribute(batch_sliced_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(B->sp.smem)));
+    CIECU_TRY(allow_shared(batch_sliced_persistent_kernel));
     for (;;) {
         int aborted = 0;
         CIECU_CUDA(cudaMemcpyAsync(B->h_g, B->d_g, sizeof(BatchGlobal), cudaMemcpyDeviceToHost, st));

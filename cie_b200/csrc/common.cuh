@@ -159,6 +159,15 @@ __device__ __forceinline__ T combine(T inScale, T old, T outScale, T sum) {
     return inScale * old + outScale * sum;
 }
 
+// Opts `kernel` in to all the dynamic shared memory that fits beside its static one, so
+// that any launch may follow.  The limit belongs to the function in the whole process: set
+// to one caller's size, it would cut off a larger launch of another solver or thread.
+int allow_shared(const void* kernel);
+template <typename K>
+int allow_shared(K* kernel) {
+    return allow_shared(reinterpret_cast<const void*>(kernel));
+}
+
 // Largest grid of `kernel` whose blocks are all resident at once (one wave),
 // capped by the blocks the work needs; cached per kernel.
 int resident_blocks(const void* kernel, int threads, size_t smem);

@@ -320,7 +320,7 @@ inline int dm_prepare(const DiaArgs<double>& u, long leastBytes, std::initialize
     DmPlan plan = dm_plan(u, sm_count(), static_cast<size_t>(std::max(optin - 2048, 0)));
     if (!plan.blocks) return CIECU_OK;
     for (const void* kernel : kernels)
-        CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 2048));
+        CIECU_TRY(allow_shared(kernel));
     double* triples = nullptr;
     if (pool_alloc(&triples, sizeof(double) * 12 * static_cast<size_t>(u.ld), st) != cudaSuccess) {
         cudaGetLastError();

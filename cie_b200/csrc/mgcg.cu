@@ -1129,8 +1129,9 @@ int prepare_cluster(ciecu_mgcg_s* M, cudaStream_t st) {
     }
     if (!rows) return CIECU_OK;
     const ClusterKernel kern = cluster_kernel(nt, rows);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e == cudaSuccess && ctas > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    CIECU_TRY(allow_shared(kern));
+    cudaError_t e = cudaSuccess;
+    if (ctas > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     int clusters = 0;
     if (e == cudaSuccess) {
         M->clusterCtas = ctas;
@@ -1354,7 +1355,7 @@ int prepare_slices(ciecu_mgcg_s* M, int lo, int hi, cudaStream_t st) {
          {reinterpret_cast<const void*>(sl_kernel<SlChebStep<0>>), reinterpret_cast<const void*>(sl_kernel<SlChebStep<1>>),
           reinterpret_cast<const void*>(sl_kernel<SlChebStep<2>>), reinterpret_cast<const void*>(sl_kernel<First>),
           reinterpret_cast<const void*>(sl_kernel<Second>)})
-        CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 2048));
+        CIECU_TRY(allow_shared(kernel));
     size_t at = 0;
     auto part = [&](size_t bytes) {
         const size_t begin = at;

@@ -1893,10 +1893,8 @@ int plan_planes(ciecu_multi_s* M) {
     A.stageFloats = A.xFloats + 3 * most * kPlaneRows;
     const size_t smem = 2 * sizeof(float) * static_cast<size_t>(A.stageFloats);
     if (smem + 16 * 1024 > static_cast<size_t>(optin)) return CIECU_OK;  // static: the reductions
-    CIECU_CUDA(cudaFuncSetAttribute(multi_spmv_planes_f32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
-    CIECU_CUDA(cudaFuncSetAttribute(multi_spmv_planes_f32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
+    CIECU_TRY(allow_shared(multi_spmv_planes_f32_kernel<true>));
+    CIECU_TRY(allow_shared(multi_spmv_planes_f32_kernel<false>));
     M->planes = A;
     M->planesSmem = smem;
     return CIECU_OK;

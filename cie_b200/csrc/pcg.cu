@@ -991,8 +991,7 @@ int launch_dia_persistent(ciecu_pcg_s* S, cudaStream_t st) {
         using std::true_type;
         auto* kernel = plan.resident ? (S->dinv ? pick(true_type{}, true_type{}) : pick(true_type{}, false_type{}))
                                      : (S->dinv ? pick(false_type{}, true_type{}) : pick(false_type{}, false_type{}));
-        CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(plan.smem)));
+        CIECU_TRY(allow_shared(kernel));
         void* params[] = {&a, &S->d_s};
         CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(plan.grid),
                                                dim3(plan.threads), params, plan.smem, st));
@@ -1005,7 +1004,7 @@ int launch_dia_persistent(ciecu_pcg_s* S, cudaStream_t st) {
 template <int VS, bool PRE>
 int launch_persistent(ciecu_pcg_s* S, cudaStream_t st) {
     auto kernel = pcg_persistent_kernel<VS, PRE>;
-    CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(S->smem)));
+    CIECU_TRY(allow_shared(kernel));
     int occ = 0;
     CIECU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kPT, S->smem));
     if (occ < 1) return fail(CIECU_ERR_CUDA, "pcg: the single-launch kernel does not fit on an SM");
@@ -1035,7 +1034,7 @@ int launch_sliced_persistent(ciecu_pcg_s* S, cudaStream_t st) {
     a.waitNs = S->waitNs;
     a.withholdEpoch = S->withholdExchange > 0 ? S->epoch + static_cast<unsigned long long>(S->withholdExchange) : 0ULL;
     auto* kernel = S->dinv ? pcg_sliced_persistent_kernel<true> : pcg_sliced_persistent_kernel<false>;
-    CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(S->sp.smem)));
+    CIECU_TRY(allow_shared(kernel));
     void* params[] = {&a, &S->d_s};
     CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(S->sp.grid), dim3(S->sp.threads),
                                            params, S->sp.smem, st));

@@ -6,6 +6,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <string>
 
@@ -90,6 +91,23 @@ void pool_release(std::initializer_list<void*> ptrs) {
     for (void* p : ptrs)
         if (p) cudaFreeAsync(p, cudaStreamLegacy);
     cudaStreamSynchronize(cudaStreamLegacy);  // the blocks are free for any stream from here
+}
+
+int allow_shared(const void* kernel) {
+    static std::mutex mutex;
+    static std::set<std::pair<int, const void*>> done;  // per device: the attribute is
+    int device = 0, optin = 0;
+    CIECU_CUDA(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto key = std::make_pair(device, kernel);
+    if (done.count(key)) return CIECU_OK;
+    cudaFuncAttributes attributes{};
+    CIECU_CUDA(cudaFuncGetAttributes(&attributes, kernel));
+    CIECU_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    const int most = optin - static_cast<int>(attributes.sharedSizeBytes);
+    CIECU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    done.insert(key);
+    return CIECU_OK;
 }
 
 int resident_blocks(const void* kernel, int threads, size_t smem) {

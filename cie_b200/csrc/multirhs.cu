@@ -980,6 +980,8 @@ struct PlaneArgs {
     int first[12], count[12]; // triples of a run
     int lo[12], rows[12];     // smallest middle offset; operand rows: kPlaneRows + span + 2
     int xFloats, stageFloats; // a stage: operand rows, then the diagonals
+    unsigned long long waitNs;  // bound of a wait for a run's copies
+    int withholdRun;            // test hook: CTA 0 leaves out the copies of its run of this number, from 1 (0: none)
 };
 
 template <typename Op>
@@ -999,10 +1001,10 @@ __device__ __forceinline__ void quad_rows_dia3_planes(const DiaArgs<float>& D, c
         fence_mbarrier_init();
     }
     __syncthreads();
-    // Run g of the rows from `base` into buffer `buf`, which nobody reads any more: lane 0
-    // of warp 0 the operand rows, its next lanes a diagonal each; operand rows outside
-    // the matrix are zeroed by all threads.
-    auto issue = [&](long base, int g, int buf) {
+    // Run g of the rows from `base`, the CTA's run of that number, into buffer `buf`, which
+    // nobody reads any more: lane 0 of warp 0 the operand rows, its next lanes a diagonal
+    // each; operand rows outside the matrix are zeroed by all threads.
+    auto issue = [&](long base, int g, int buf, int number) {
         float* xs = s_planes + buf * A.stageFloats;
         const long first = base + A.lo[g] - 1, end = first + A.rows[g];
         const long from = max(first, 0L), to = max(from, min(end, static_cast<long>(n)));
@@ -1022,7 +1024,7 @@ __device__ __forceinline__ void quad_rows_dia3_planes(const DiaArgs<float>& D, c
             const unsigned total = __reduce_add_sync(0xffffffffu, bytes);
             if (lane == 0) mbar_arrive_expect_tx(&s_full[buf], total);
             __syncwarp();
-            if (bytes) bulk_copy_g2s(dst, src, bytes, &s_full[buf]);
+            if (bytes && (number != A.withholdRun || blockIdx.x > 0)) bulk_copy_g2s(dst, src, bytes, &s_full[buf]);
         }
         if (first < 0 || end > n) {
             for (long u = threadIdx.x; u < A.rows[g] * 32L; u += kPlaneThreads) {
@@ -1035,7 +1037,7 @@ __device__ __forceinline__ void quad_rows_dia3_planes(const DiaArgs<float>& D, c
     const long stride = static_cast<long>(gridDim.x) * kPlaneRows;
     long base = static_cast<long>(blockIdx.x) * kPlaneRows;
     unsigned turn = 0;  // runs done: buffer turn mod 2
-    if (base < n) issue(base, 0, 0);
+    if (base < n) issue(base, 0, 0, 1);
     for (; base < n; base += stride) {
         float acc[4][4];
 #pragma unroll
@@ -1045,15 +1047,15 @@ __device__ __forceinline__ void quad_rows_dia3_planes(const DiaArgs<float>& D, c
 #pragma unroll 1
         for (int g = 0; g < A.runs; ++g, ++turn) {
             const int buf = turn & 1;
-            if (!mbar_wait_bounded(&s_full[buf], (turn >> 1) & 1)) s_late = 1;
+            if (!mbar_wait_bounded(&s_full[buf], (turn >> 1) & 1, A.waitNs)) s_late = 1;
             __syncthreads();  // this run is complete, its zeros are written, and the other buffer is free
             if (s_late) {     // the one copy in flight is this run's: waited for once more, then left
-                mbar_wait_bounded(&s_full[buf], (turn >> 1) & 1);
+                mbar_wait_bounded(&s_full[buf], (turn >> 1) & 1, A.waitNs);
                 if (threadIdx.x == 0) atomicExch(timeout, 1);
                 return;
             }
-            if (g + 1 < A.runs) issue(base, g + 1, buf ^ 1);
-            else if (base + stride < n) issue(base + stride, 0, buf ^ 1);
+            if (g + 1 < A.runs) issue(base, g + 1, buf ^ 1, turn + 2);
+            else if (base + stride < n) issue(base + stride, 0, buf ^ 1, turn + 2);
             const float* xs = s_planes + buf * A.stageFloats;
             const float* vs = xs + A.xFloats;
             for (int t = 0; t < A.count[g]; ++t) {
@@ -1353,7 +1355,9 @@ __global__ void __launch_bounds__(kT) multi_direction32_quad_kernel(long n, floa
                                                                     cudaGraphConditionalHandle cond) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         g->chunkIter += 1;
-        const bool more = *reinterpret_cast<volatile unsigned*>(&g->finished) < 32u;
+        // (after a wait that gave up there are no sums to go on with: the host reports it)
+        const bool more = *reinterpret_cast<volatile unsigned*>(&g->finished) < 32u &&
+                          !*reinterpret_cast<volatile int*>(&g->timeout);
         set_loop<COND>(cond, (more && g->chunkIter < g->chunkLimit) ? 1u : 0u);
     }
     quad_direction_step<float>(n, X, P, R, dinv, S, true,
@@ -1573,6 +1577,8 @@ struct ciecu_multi_s {
     int gridQD3 = 1, gridQ32D3 = 1;
     ciecu::PlaneArgs planes{};  // the staged FP32 triple pass
     size_t planesSmem = 0;      // its shared memory; 0: its stages do not fit
+    unsigned long long waitNs = ciecu::kMbarWaitNs;  // of its waits (ciecu_multi_debug_wait)
+    int withholdRun = 0;
 };
 
 namespace ciecu {
@@ -1895,6 +1901,8 @@ int plan_planes(ciecu_multi_s* M) {
     if (smem + 16 * 1024 > static_cast<size_t>(optin)) return CIECU_OK;  // static: the reductions
     CIECU_TRY(allow_shared(multi_spmv_planes_f32_kernel<true>));
     CIECU_TRY(allow_shared(multi_spmv_planes_f32_kernel<false>));
+    A.waitNs = M->waitNs;
+    A.withholdRun = M->withholdRun;
     M->planes = A;
     M->planesSmem = smem;
     return CIECU_OK;
@@ -2167,6 +2175,26 @@ int ciecu_multi_refinements(ciecu_multi M, int64_t* h_perColumn) {
     CIECU_REQUIRE(M && h_perColumn, "multi_refinements: null argument");
     for (int c = 0; c < M->k; ++c)
         h_perColumn[c] = c < static_cast<int>(M->last.size()) ? M->last[c].refinements : 0;
+    return CIECU_OK;
+}
+
+int ciecu_multi_staged(ciecu_multi M, int* staged) {
+    CIECU_REQUIRE(M && staged, "multi_staged: null argument");
+    *staged = M->refineDelta > 0.0 && M->quad && M->useDia && M->triples && M->planesSmem > 0 ? 1 : 0;
+    return CIECU_OK;
+}
+
+int ciecu_multi_debug_wait(ciecu_multi M, int64_t waitNanoseconds, int withholdRun) {
+    CIECU_REQUIRE(M, "multi_debug_wait: null solver");
+    CIECU_REQUIRE(waitNanoseconds >= 1000 && waitNanoseconds <= 60000000000LL,
+                  "multi_debug_wait: the wait limit must be in [1 us, 60 s]");
+    CIECU_REQUIRE(withholdRun >= 0, "multi_debug_wait: negative run");
+    M->planes.waitNs = M->waitNs = static_cast<unsigned long long>(waitNanoseconds);
+    M->planes.withholdRun = M->withholdRun = withholdRun;
+    if (M->graph32) {  // holds the arguments
+        cudaGraphExecDestroy(M->graph32);
+        M->graph32 = nullptr;
+    }
     return CIECU_OK;
 }
 

@@ -58,11 +58,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
     return ok != 0;
 }
 
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity,
+                                                  unsigned long long limitNs = kMbarWaitNs) {
     const unsigned long long t0 = global_ns();
     for (unsigned spins = 1;; ++spins) {
         if (mbar_try_wait(bar, parity)) return true;
-        if ((spins & 255u) == 0u && global_ns() - t0 > kMbarWaitNs) return false;
+        if ((spins & 255u) == 0u && global_ns() - t0 > limitNs) return false;
     }
 }
 

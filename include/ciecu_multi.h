@@ -39,6 +39,15 @@ int ciecu_multi_format(ciecu_multi solver, int* diagonals);
  * and loads each operand row of a triple once; ciecu_multi_format reports the
  * diagonal count either way. */
 int ciecu_multi_set_format(ciecu_multi solver, int format);
+/* *staged: 1 when the last FP32-refined solve with 32 columns staged its operand rows in
+ * shared memory (Q1 stencils whose planes allow it), 0 otherwise. */
+int ciecu_multi_staged(ciecu_multi solver, int* staged);
+/* Controls the bounded waits of that staged pass, for tests of its timeout path:
+ * waitNanoseconds bounds each wait for a copy (default 2 s; [1 us, 60 s]); withholdRun > 0
+ * makes the first block leave out the copies of its run of that number, so that its wait
+ * runs out and the solve fails with CIECU_ERR_TIMEOUT; 0 (default) copies normally.  The
+ * solver stays usable after a timeout. */
+int ciecu_multi_debug_wait(ciecu_multi solver, int64_t waitNanoseconds, int withholdRun);
 /* delta in (0, 1): FP32-refined form -- every column iterates in FP32 (FP32
  * copies of the matrix in the format of the FP64 solve and of D^-1, FP32 blocks,
  * FP64 dot products) with FP64 reliable updates: every running column's FP32

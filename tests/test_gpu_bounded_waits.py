@@ -1,0 +1,55 @@
+"""The bounded waits of the kernels that read shared memory filled by copies or by other
+blocks: a wait made to run out (a copy or a sum that is left out; limits of a
+millisecond) ends the solve with CIECU_ERR_TIMEOUT, soon, and the same solver then
+solves as before, bit for bit."""
+import ctypes
+import time
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+MS = 1_000_000
+SECOND = 1.0  # far above the waits of one launch, far below those of a loop that ran on
+
+
+def timed_out(solve):
+    from cie_b200._lib import CiecuError
+    torch.cuda.synchronize()
+    begin = time.perf_counter()
+    with pytest.raises(CiecuError) as e:
+        solve()
+    torch.cuda.synchronize()
+    assert e.value.status == 5, e.value
+    assert time.perf_counter() - begin < SECOND
+
+
+@pytest.mark.parametrize("run", [1, 2, 3])
+def test_staged_columns(run):
+    from cie_b200._lib import call
+    from cie_b200.fem import make_poisson
+    from cie_b200.linalg import (CSROperator, CUDASpace, MultiRHSConjugateGradients, Statistics,
+                                 makeDiagonalOperator)
+    space = CUDASpace()
+    problem = make_poisson(space, 3, 1, [24, 24, 4], seed=1)
+    A = CSROperator(problem.matrix, space)
+    solver = MultiRHSConjugateGradients(A, makeDiagonalOperator(problem.matrix, space, csr_handle=A.csr), 32,
+                                        Statistics(500, 0.0, 1e-10))
+    solver.set_refinement(0.1)
+    solver.set_format(1)
+    b = (problem.rhs[:, None] * torch.arange(1, 33, device="cuda", dtype=torch.float64)).contiguous()
+
+    def solve():
+        x = torch.zeros_like(b)
+        solver.product(0.0, b, 1.0, x)
+        return x
+
+    first = solve()
+    staged = ctypes.c_int()
+    call("ciecu_multi_staged", solver._solver, ctypes.byref(staged))
+    assert staged.value == 1
+    call("ciecu_multi_debug_wait", solver._solver, MS, run)
+    timed_out(solve)
+    call("ciecu_multi_debug_wait", solver._solver, 2000 * MS, 0)
+    assert torch.equal(solve(), first)

@@ -22,8 +22,9 @@
 // whole windows).  In FP32 the row pass itself binds, 47 us, and reading the full matrix
 // once (dia_rows4_triples, 41 us) is faster.
 //
-// Every wait is bounded; after one has given up the kernel runs to its end without waiting
-// and op.expired() tells.
+// Every wait is bounded.  After one has given up the warps of rows free no slot any more,
+// the producer brings nothing more, all run to their end without waiting, and op.expired()
+// tells.
 #pragma once
 
 #include "dia.cuh"
@@ -48,7 +49,11 @@ struct DmArgs {
     int T, tiles;     // rows of a tile, tiles of a plane
     int run, planes;  // planes of a block at most, planes of the matrix
     int W;            // rows of a window
+    long long waitClocks;  // bound of a wait
+    int withholdPlane;     // test hook: block 0 leaves out a copy in its plane of this number, from 1 (0: none)
 };
+
+constexpr long long kDmWaitClocks = 1LL << 31;  // about a second
 
 struct DmPlan {
     DmArgs args{};
@@ -60,7 +65,8 @@ __device__ __forceinline__ unsigned dm_shared(const void* p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ bool dm_wait(const unsigned long long* bar, unsigned parity, volatile int* failed) {
+__device__ __forceinline__ bool dm_wait(const unsigned long long* bar, unsigned parity, long long limit,
+                                        volatile int* failed) {
     unsigned ok = 0;
     for (long long begun = clock64();;) {
         asm volatile(
@@ -69,7 +75,7 @@ __device__ __forceinline__ bool dm_wait(const unsigned long long* bar, unsigned 
             : "r"(dm_shared(bar)), "r"(parity)
             : "memory");
         if (ok) return true;
-        if (*failed || clock64() - begun > (1LL << 31)) {  // about a second
+        if (*failed || clock64() - begun > limit) {
             *failed = 1;
             return false;
         }
@@ -84,7 +90,7 @@ __device__ __forceinline__ void dm_arrive(const unsigned long long* bar) {
 // apart, a window beginning at w0 rounded down to kDmAlign bytes; zeros outside [0, n).
 template <int PITCH>
 __device__ __forceinline__ void dm_bring(double* to, int W, const double* from, long stride, int count, int w0, int w1, int n,
-                                         const unsigned long long* bar) {
+                                         const unsigned long long* bar, bool go, bool withhold = false) {
     constexpr int Q = kDmAlign / 8, R = 2;
     const int lane = threadIdx.x & 31;
     const int s0 = w0 & ~(Q - 1);
@@ -103,11 +109,11 @@ __device__ __forceinline__ void dm_bring(double* to, int W, const double* from, 
         __syncwarp();
     }
     const int bytes = (end - lo) * PITCH * 8;
-    if (lane == 0)
+    if (lane == 0 && go)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(dm_shared(bar)), "r"(bytes * count)
                      : "memory");
     __syncwarp();
-    if (lane < count && bytes > 0)
+    if (lane < count && bytes > 0 && go && !withhold)
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                          dm_shared(to + lane * W + (lo - s0) * PITCH)),
                      "l"(from + lane * stride + lo * static_cast<long>(PITCH)), "r"(bytes), "r"(dm_shared(bar))
@@ -145,20 +151,25 @@ __device__ __forceinline__ void dm_rows(const DmArgs& A, const double* __restric
     if (z0 < z1) {
         if (warp == kWarps) {
             int slot = 0, turn = 0, opSlot = 0, opTurn = 0;
-            auto slot_free = [&]() {
-                if (turn) dm_wait(slotFree + slot, (turn - 1) & 1, &s_failed);
+            // After a wait that gave up the lane neither arms a barrier nor copies: the slot may
+            // be in use, and a barrier armed in a phase that has not ended gets an arrival too
+            // many.  (Lanes keep together: the branches around them stay those of the others.)
+            bool stop = false;
+            auto until_free = [&](const unsigned long long* bar, int turns) {
+                if (turns && !dm_wait(bar, (turns - 1) & 1, A.waitClocks, &s_failed)) stop = true;
             };
             auto slot_next = [&]() {
                 if (++slot == kDmSlots) slot = 0, ++turn;
             };
-            auto triple = [&](int k, int w0, int w1) {
-                slot_free();
-                dm_bring<3>(slots + slot * 3 * W, 0, A.triples + k * A.ld * 3, 0, 1, w0, w1, A.n, slotFull + slot);
+            auto triple = [&](int k, int w0, int w1, bool withhold = false) {
+                until_free(slotFree + slot, turn);
+                dm_bring<3>(slots + slot * 3 * W, 0, A.triples + k * A.ld * 3, 0, 1, w0, w1, A.n, slotFull + slot, !stop,
+                            withhold);
                 slot_next();
             };
             auto operand = [&](int w0, int w1) {
-                if (opTurn) dm_wait(opFree + opSlot, (opTurn - 1) & 1, &s_failed);
-                dm_bring<1>(operands + opSlot * W, 0, x, 0, 1, w0, w1, A.n, opFull + opSlot);
+                until_free(opFree + opSlot, opTurn);
+                dm_bring<1>(operands + opSlot * W, 0, x, 0, 1, w0, w1, A.n, opFull + opSlot, !stop);
                 if (++opSlot == kDmOperands) opSlot = 0, ++opTurn;
             };
             for (int z = z0 - 1; z < z1; ++z) {
@@ -166,9 +177,9 @@ __device__ __forceinline__ void dm_rows(const DmArgs& A, const double* __restric
                 if (z < z0) operand(w0, w1);
                 operand(w0 + S, w1 + S);
                 if (z >= z0) {
-                    triple(0, w0, own);
-                    slot_free();
-                    dm_bring<1>(slots + slot * 3 * W, W, A.upper, A.ld, 2, w0, own, A.n, slotFull + slot);
+                    triple(0, w0, own, blockIdx.x == 0 && z - z0 + 1 == A.withholdPlane);
+                    until_free(slotFree + slot, turn);
+                    dm_bring<1>(slots + slot * 3 * W, W, A.upper, A.ld, 2, w0, own, A.n, slotFull + slot, !stop);
                     slot_next();
                 }
                 for (int k = 1; k <= 3; ++k) triple(k, w0, w1);
@@ -176,15 +187,16 @@ __device__ __forceinline__ void dm_rows(const DmArgs& A, const double* __restric
         } else {
             const int j = min(tid, width - 1);  // row of the plane
             int slot = 0, parity = 0, opSlot = 0, opParity = 0;
+            bool dead = false;  // a wait gave up: the slots are freed no more, and the producer stops
             auto next = [&]() {  // the next slot, when it is full
                 double* p = slots + slot * 3 * W;
-                dm_wait(slotFull + slot, parity, &s_failed);
+                if (!dm_wait(slotFull + slot, parity, A.waitClocks, &s_failed)) dead = true;
                 if (++slot == kDmSlots) slot = 0, parity ^= 1;
                 return p;
             };
             auto next_operand = [&]() {
                 double* p = operands + opSlot * W;
-                dm_wait(opFull + opSlot, opParity, &s_failed);
+                if (!dm_wait(opFull + opSlot, opParity, A.waitClocks, &s_failed)) dead = true;
                 if (++opSlot == kDmOperands) opSlot = 0, opParity ^= 1;
                 return p;
             };
@@ -214,7 +226,7 @@ __device__ __forceinline__ void dm_rows(const DmArgs& A, const double* __restric
                         sum = fma(g[k][3 * i + e], xm[i], sum);
                     }
                 __syncwarp();
-                if (lane == 0) {
+                if (lane == 0 && !dead) {
                     for (int k = 0; k < 3; ++k) dm_arrive(slotFree + (gSlot + k) % kDmSlots);
                     dm_arrive(opFree + opFirst);
                 }
@@ -233,7 +245,7 @@ __device__ __forceinline__ void dm_rows(const DmArgs& A, const double* __restric
 #pragma unroll
                 for (int e = 0; e < 3; ++e) sum = fma(line[3 * bc + e], xc[bc + N - 1 + e], sum);
                 __syncwarp();
-                if (lane == 0)
+                if (lane == 0 && !dead)
                     for (int k = 0; k < 2; ++k) dm_arrive(slotFree + (lineSlot + k) % kDmSlots);
                 const double* xp = next_operand();
                 const int bp = at(z + 1);
@@ -254,7 +266,7 @@ __device__ __forceinline__ void dm_rows(const DmArgs& A, const double* __restric
         }
     }
     __syncthreads();
-    if (s_failed) {  // no copy is in flight after some milliseconds
+    if (s_failed) {  // no copy is in flight some milliseconds after the producer's last
         for (const long long begun = clock64(); clock64() - begun < (1LL << 24);) {
         }
         if (tid == 0) op.expired();
@@ -298,7 +310,8 @@ inline DmPlan dm_plan(const DiaArgs<double>& u, int sms, size_t maxSmem) {
         if (2 * N > T / 2 + T / 8 || cost >= best) continue;
         best = cost;
         plan.args =
-            DmArgs{nullptr, u.val, u.ld, u.nrows, S, N, T, used, static_cast<int>(run), static_cast<int>(planes), W};
+            DmArgs{nullptr, u.val, u.ld, u.nrows, S, N, T, used, static_cast<int>(run), static_cast<int>(planes), W,
+                   kDmWaitClocks, 0};
         plan.blocks = used * static_cast<int>((planes + run - 1) / run);
         plan.smem = smem;
     }

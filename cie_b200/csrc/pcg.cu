@@ -149,12 +149,9 @@ __global__ void __launch_bounds__(kT) pcg_spmv_dia_sym_kernel(DiaArgs<double> U,
 // row sums again, each entry of the upper half read from memory once.
 struct MarchPqOp : PqOp {
     PcgScalars* s;
-    __device__ __forceinline__ void expired() const {
-        s->done = 3;
-        s->error = CIECU_ERR_TIMEOUT;
-        s->errorKind = 3;
-        s->errorIter = s->iter;
-    }
+    // `done` is left to the last block: one that starts later must still take its part in
+    // the reduction, or the counter would stay behind for the next solve.
+    __device__ __forceinline__ void expired() const { atomicExch(&s->late, 1); }
 };
 
 template <bool COND>
@@ -170,7 +167,14 @@ __global__ void __launch_bounds__(kDmThreads, 1)
     dm_rows(A, p, op);
     double mine[1] = {op.acc}, tot[1];
     if (grid_reduce_last<1, kDmThreads>(mine, partials, counter, tot) && threadIdx.x == 0) {
-        if (s->done) return;  // a wait gave up
+        if (*reinterpret_cast<volatile int*>(&s->late)) {
+            s->done = 3;
+            s->error = CIECU_ERR_TIMEOUT;
+            s->errorKind = 3;
+            s->errorIter = s->iter;
+            set_loop<COND>(cond, 0);
+            return;
+        }
         s->pq = tot[0];
         if (!(0.0 < tot[0])) {
             s->done = 3;
@@ -800,6 +804,12 @@ int launch_k1(ciecu_pcg_s* S, cudaStream_t st, int schedule, cudaGraphConditiona
 // 52; 81^3 (60 MB): 41 and 34.
 constexpr long kMarchBytes = 112L << 20;
 
+// The settings of ciecu_pcg_debug_exchange in the marching K1's arguments.
+void set_march_wait(ciecu_pcg_s* S) {
+    S->march.args.waitClocks = 2 * S->waitNs;  // SM clocks up to 1.965 GHz
+    S->march.args.withholdPlane = static_cast<int>(std::min<long long>(S->withholdExchange, INT_MAX));
+}
+
 // Plans the marching K1 once per solver; refills its copy of the triples at every solve.
 int refresh_march(ciecu_pcg_s* S, cudaStream_t st) {
     if (!S->marchPlanned) {
@@ -808,6 +818,7 @@ int refresh_march(ciecu_pcg_s* S, cudaStream_t st) {
                                      {reinterpret_cast<const void*>(pcg_spmv_march_kernel<true>),
                                       reinterpret_cast<const void*>(pcg_spmv_march_kernel<false>)},
                                      S->p, st, &S->march, &S->triples));
+        set_march_wait(S);
     }
     return S->march.blocks ? dm_fill(S->diaU, S->triples, st) : CIECU_OK;
 }
@@ -1308,6 +1319,23 @@ int ciecu_pcg_debug_exchange(ciecu_pcg S, int64_t waitNanoseconds, int64_t withh
     CIECU_REQUIRE(withholdExchange >= 0, "pcg_debug_exchange: negative exchange index");
     S->waitNs = waitNanoseconds;
     S->withholdExchange = withholdExchange;
+    if (S->march.blocks) {
+        set_march_wait(S);
+        if (S->graph) {  // holds the arguments
+            cudaGraphExecDestroy(S->graph);
+            S->graph = nullptr;
+        }
+    }
+    return CIECU_OK;
+}
+
+int ciecu_pcg_form(ciecu_pcg S, int* form) {
+    CIECU_REQUIRE(S && form, "pcg_form: null argument");
+    if (S->persistent)
+        *form = S->dp ? CIECU_PCG_SINGLE_DIAGONALS : (S->sliced ? CIECU_PCG_SINGLE_SLICED : CIECU_PCG_SINGLE_CSR);
+    else
+        *form = S->kernel != kDiaSchedule ? CIECU_PCG_GRAPH_CSR
+                : S->diaSym && S->march.blocks ? CIECU_PCG_GRAPH_MARCH : CIECU_PCG_GRAPH_DIAGONALS;
     return CIECU_OK;
 }
 

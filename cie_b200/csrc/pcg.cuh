@@ -21,10 +21,10 @@ struct PcgScalars {
     long long maxIter;
     double absTol, relTol;
     int done;           // 0 running, 1 converged, 2 iteration limit, 3 error
-    int error;          // 0, CIECU_ERR_BREAKDOWN
+    int error;          // 0, CIECU_ERR_BREAKDOWN, CIECU_ERR_TIMEOUT
     long long errorIter;
-    int errorKind;      // 1: r^T z <= 0 at start, 2: p^T A p <= 0
-    int pad;
+    int errorKind;      // 1: r^T z <= 0 at start, 2: p^T A p <= 0, 3: a wait gave up
+    int late;           // set when a bounded wait of K1 gave up
     long long chunkIter;   // iterations run by the current graph launch
     long long chunkLimit;  // iterations one graph launch may run
 };

@@ -247,8 +247,22 @@ int ciecu_pcg_set_loop(ciecu_pcg solver, int mode);
  * withholdExchange > 0 makes the last block skip publishing its partial sums at
  * that exchange of the next launches (counted from 1), so every wait on it runs
  * out, the launch ends and the solve fails with CIECU_ERR_TIMEOUT; 0 (default)
- * publishes normally.  The solver stays usable after a timeout. */
+ * publishes normally.  In the graph loop over a large 3D Q1 stencil, whose row pass
+ * waits for copies, the limit bounds those waits and withholdExchange > 0 leaves out
+ * a copy in the first block's plane of that number.  The solver stays usable after a
+ * timeout. */
 int ciecu_pcg_debug_exchange(ciecu_pcg solver, int64_t waitNanoseconds, int64_t withholdExchange);
+
+/* How the last solve ran its iterations. */
+enum {
+    CIECU_PCG_GRAPH_CSR = 0,        /* graph of three kernels, rows of the CSR matrix */
+    CIECU_PCG_GRAPH_DIAGONALS = 1,  /* ... rows of the diagonal-storage copy */
+    CIECU_PCG_GRAPH_MARCH = 2,      /* ... by tiles marching through the planes of a 3D stencil */
+    CIECU_PCG_SINGLE_DIAGONALS = 3, /* single launch over the diagonal-storage copy */
+    CIECU_PCG_SINGLE_SLICED = 4,    /* single launch over sliced rows */
+    CIECU_PCG_SINGLE_CSR = 5        /* single launch, rows of the CSR matrix in shared memory */
+};
+int ciecu_pcg_form(ciecu_pcg solver, int* form);
 
 #ifdef __cplusplus
 }

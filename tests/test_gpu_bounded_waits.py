@@ -53,3 +53,32 @@ def test_staged_columns(run):
     timed_out(solve)
     call("ciecu_multi_debug_wait", solver._solver, 2000 * MS, 0)
     assert torch.equal(solve(), first)
+
+
+@pytest.mark.parametrize("plane", [1, 2, 9])
+def test_marching_tiles(plane):
+    from cie_b200._lib import call
+    from cie_b200.fem import make_poisson
+    from cie_b200.linalg import ConjugateGradients, CSROperator, CUDASpace, Statistics, makeDiagonalOperator
+    space = CUDASpace()
+    problem = make_poisson(space, 3, 1, [103, 100, 101], seed=1)
+    A = CSROperator(problem.matrix, space)
+    solver = ConjugateGradients(A, space, makeDiagonalOperator(problem.matrix, space, csr_handle=A.csr),
+                                Statistics(12, 0.0, 1e-300))
+    solver.set_loop(1)
+    solver.set_schedule(64)
+
+    def solve():
+        x = torch.zeros_like(problem.rhs)
+        solver.product(0.0, problem.rhs, 1.0, x)
+        return x
+
+    first = solve()
+    form = ctypes.c_int()
+    call("ciecu_pcg_form", solver._solver, ctypes.byref(form))
+    assert form.value == 2
+    solver.debug_exchange(MS, plane)
+    for _ in range(2):
+        timed_out(solve)
+    solver.debug_exchange(2000 * MS, 0)
+    assert torch.equal(solve(), first)

@@ -157,6 +157,7 @@ SIGNATURES = {
     "ciecu_mgcg_coarse_info": (c_int, [P, P, P]),
     "ciecu_mgcg_set_coarse_cluster": (c_int, [P, c_int]),
     "ciecu_mgcg_coarse_apply": (c_int, [P, P, P]),
+    "ciecu_mgcg_debug_wait": (c_int, [P, c_int]),
 }
 
 OPTIONAL = set()

@@ -1,7 +1,7 @@
 """The bounded waits of the kernels that read shared memory filled by copies or by other
-blocks: a wait made to run out (a copy or a sum that is left out; limits of a
-millisecond) ends the solve with CIECU_ERR_TIMEOUT, soon, and the same solver then
-solves as before, bit for bit."""
+blocks: a wait made to run out (a copy that is left out, bytes that nobody sends; limits
+of a millisecond where they can be set) ends the solve with CIECU_ERR_TIMEOUT, soon, and
+the same solver then solves as before, bit for bit."""
 import ctypes
 import time
 
@@ -14,7 +14,7 @@ MS = 1_000_000
 SECOND = 1.0  # far above the waits of one launch, far below those of a loop that ran on
 
 
-def timed_out(solve):
+def timed_out(solve, limit=SECOND):
     from cie_b200._lib import CiecuError
     torch.cuda.synchronize()
     begin = time.perf_counter()
@@ -22,7 +22,7 @@ def timed_out(solve):
         solve()
     torch.cuda.synchronize()
     assert e.value.status == 5, e.value
-    assert time.perf_counter() - begin < SECOND
+    assert time.perf_counter() - begin < limit
 
 
 @pytest.mark.parametrize("run", [1, 2, 3])
@@ -82,3 +82,45 @@ def test_marching_tiles(plane):
         timed_out(solve)
     solver.debug_exchange(2000 * MS, 0)
     assert torch.equal(solve(), first)
+
+
+@pytest.fixture(scope="module")
+def two_level():
+    from cie_b200.fem import make_embedded_poisson
+    from cie_b200.linalg import CUDASpace, Statistics
+    from cie_b200.twolevel import make_two_level_cg
+    space = CUDASpace()
+    problem = make_embedded_poisson(space, 3, 3, [9, 9, 9], radius=0.4, alpha=1e-6, depth=1, seed=0)
+    solver = make_two_level_cg(space, problem, Statistics(30, 0.0, 1e-30), degree=4, coarseIterations=20,
+                               precision="f32")
+    return solver, problem.rhs
+
+
+def solved(solver, b):
+    x = torch.zeros_like(b)
+    solver.product(0.0, b, 1.0, x)
+    return x
+
+
+@pytest.mark.parametrize("what", [1, 2, 3])
+def test_coarse_cluster(two_level, what):
+    """Waits of about a second, up to one after the other in two blocks: a cycle may wait twice as
+    long, and a solve ends after its first cycle or the one after."""
+    from cie_b200._lib import call
+    solver, b = two_level
+    coarse = torch.sin(torch.arange(1000, device="cuda", dtype=torch.float64))
+
+    def apply():
+        out = torch.zeros_like(coarse)
+        solver.coarse_apply(coarse, out)
+        return out
+
+    first, alone = solved(solver, b), apply()
+    info = solver.info()
+    assert info["coarse_cluster_active"] and info["coarse_cluster_ctas"] > 1
+    call("ciecu_mgcg_debug_wait", solver.handle, what)
+    timed_out(lambda: solved(solver, b), 12 * SECOND)
+    timed_out(apply, 6 * SECOND)
+    call("ciecu_mgcg_debug_wait", solver.handle, 0)
+    assert torch.equal(apply(), alone)  # before a full solve: the timeout was that call's
+    assert torch.equal(solved(solver, b), first)

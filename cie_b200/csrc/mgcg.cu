@@ -1677,7 +1677,8 @@ int ciecu_mgcg_coarse_apply(ciecu_mgcg M, const double* d_in, double* d_out) {
 
 int ciecu_mgcg_debug_wait(ciecu_mgcg M, int what) {
     CIECU_REQUIRE(M, "mgcg_debug_wait: null solver");
-    CIECU_REQUIRE(what >= 0 && what <= 3, "mgcg_debug_wait: what must be in [0, 3]");
+    CIECU_REQUIRE(what >= 0 && what <= 4, "mgcg_debug_wait: what must be in [0, 4]");
+    M->slices.args.surplus = what == 4 ? 16 : 0;
     for (int k = 0; k < 3; ++k) M->cluster.surplus[k] = what == k + 1 ? 16 : 0;
     if (M->graph) {  // holds the arguments
         cudaGraphExecDestroy(M->graph);

@@ -50,6 +50,7 @@ struct SlArgs {
     const short* __restrict__ row;     // kSlRows per slice: the row in the block, -1: none
     int n, lo, hi;                     // smallest and largest column offset
     int winLen;                        // window entries of any block
+    int surplus;                       // test hook: bytes that block 0 waits for but nobody copies
 };
 
 struct SlPlan {
@@ -65,6 +66,20 @@ __device__ __forceinline__ void sl_use(float (&acc)[4], const float4& v, const s
     acc[1] = fmaf(v.y, win[o.y], acc[1]);
     acc[2] = fmaf(v.z, win[o.z], acc[2]);
     acc[3] = fmaf(v.w, win[o.w], acc[3]);
+}
+
+// Whether the one phase of `bar` ended within about a second (it never takes that long).
+__device__ __forceinline__ bool sl_arrived(unsigned bar) {
+    unsigned arrived = 0;
+    for (long long begun = clock64(); !arrived;) {
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(arrived)
+            : "r"(bar)
+            : "memory");
+        if (!arrived && clock64() - begun > (1LL << 31)) break;
+    }
+    return arrived != 0;
 }
 
 // Op: Pre pre(row), post(row, pre, sum, operand of the row), expired() when the window's
@@ -90,7 +105,9 @@ __device__ __forceinline__ void sl_rows(const SlArgs& A, const float* __restrict
     const int last = min(rb + nr + A.hi, A.n);                      // one past the window's last entry
     const int bytes = ((last - first) + 3) / 4 * 16;                // the vectors are padded to 16 bytes
     if (tid == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"(bytes + (blockIdx.x == 0 ? A.surplus : 0))
+                     : "memory");
         for (int done = 0; done < bytes; done += 16384)
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                              static_cast<unsigned>(__cvta_generic_to_shared(win)) + done),
@@ -122,16 +139,8 @@ __device__ __forceinline__ void sl_rows(const SlArgs& A, const float* __restrict
         nextStop = A.sliceEnd[ahead];
         nextRow = A.row[ahead * kSlRows + lane / 4];
     }
-    unsigned arrived = 0;
-    for (long long begun = clock64(); !arrived;) {
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(arrived)
-            : "r"(bar)
-            : "memory");
-        if (!arrived && clock64() - begun > (1LL << 31)) break;  // about a second: it never takes that long
-    }
-    if (!__syncthreads_and(arrived)) {
+    if (!__syncthreads_and(sl_arrived(bar))) {
+        sl_arrived(bar);  // the copies may still be under way: the shared memory is kept for them
         if (tid == 0) op.expired();
         return;
     }

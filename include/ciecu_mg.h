@@ -72,8 +72,9 @@ int ciecu_mgcg_set_coarse_cluster(ciecu_mgcg solver, int enable);
 int ciecu_mgcg_coarse_apply(ciecu_mgcg solver, const double* d_in, double* d_out);
 /* Makes a bounded wait (about a second) run out, for tests of the timeout path: the first
  * block waits for bytes that nobody sends, in the one-launch coarse solve beside the first
- * sums (1), the second sums (2) or the first halo (3); 0: none.  The call then fails with
- * CIECU_ERR_TIMEOUT and the solver stays usable. */
+ * sums (1), the second sums (2) or the first halo (3), or in the sliced FP32 smoother
+ * beside its window (4); 0: none.  The call then fails with CIECU_ERR_TIMEOUT and the
+ * solver stays usable. */
 int ciecu_mgcg_debug_wait(ciecu_mgcg solver, int what);
 
 #ifdef __cplusplus

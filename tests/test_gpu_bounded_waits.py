@@ -124,3 +124,22 @@ def test_coarse_cluster(two_level, what):
     call("ciecu_mgcg_debug_wait", solver.handle, 0)
     assert torch.equal(apply(), alone)  # before a full solve: the timeout was that call's
     assert torch.equal(solved(solver, b), first)
+
+
+def test_smoother_window():
+    """Each launch of a cycle waits twice, about a second each: one step of a sweep of two, so
+    that a cycle has three launches, and at most two cycles."""
+    from cie_b200._lib import call
+    from cie_b200.fem import make_embedded_poisson
+    from cie_b200.linalg import CUDASpace, Statistics
+    from cie_b200.twolevel import make_two_level_cg
+    space = CUDASpace()
+    problem = make_embedded_poisson(space, 3, 3, [12, 12, 12], radius=0.4, alpha=1e-6, depth=1, seed=0)
+    solver = make_two_level_cg(space, problem, Statistics(30, 0.0, 1e-30), degree=2, coarseIterations=20,
+                               precision="f32")
+    first = solved(solver, problem.rhs)
+    assert solver.info()["smoother_lanes_per_row"] == 4  # the sliced form
+    call("ciecu_mgcg_debug_wait", solver.handle, 4)
+    timed_out(lambda: solved(solver, problem.rhs), 30 * SECOND)
+    call("ciecu_mgcg_debug_wait", solver.handle, 0)
+    assert torch.equal(solved(solver, problem.rhs), first)

@@ -41,6 +41,7 @@ class MixedStatistics(ctypes.Structure):
 SIGNATURES = {
     "ciecu_last_error": (c_int, [c_char_p, c_int]),
     "ciecu_kernel_launch_count": (c_int64, []),
+    "ciecu_debug_fail_allocation": (c_int, [c_int]),
     "ciecu_device_info": (c_int, [P, P, P]),
     "ciecu_space_create": (c_int, [P, P]),
     "ciecu_space_destroy": (c_int, [P]),

@@ -880,7 +880,13 @@ int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
         cudaError_t e = pool_alloc(&B->p1, sizeof(double) * static_cast<size_t>(std::max<long>(1, B->n)), st);
         if (e == cudaSuccess) e = pool_alloc(&B->abortFlag, sizeof(int), st);
         if (e == cudaSuccess) e = cudaMemsetAsync(B->abortFlag, 0, sizeof(int), st);
-        if (e != cudaSuccess) return cuda_fail(e, "batched pcg: single-launch buffers");
+        if (e != cudaSuccess) {  // no room: the graph loop, and another try at the next solve
+            cudaGetLastError();
+            pool_release({B->p1, B->abortFlag});
+            B->p1 = nullptr;
+            B->abortFlag = nullptr;
+            return CIECU_OK;
+        }
     }
     *used = true;
     CIECU_TRY(sp_fill(B->sp, B->A, st));

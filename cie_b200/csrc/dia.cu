@@ -89,7 +89,10 @@ int dia_offsets(ciecu_csr_s* csr, const std::vector<int>** out) {
     if (csr->rows != csr->cols || csr->rows == 0 || csr->nnz == 0) return CIECU_OK;
     cudaStream_t st = csr->space->stream;
     int* d_table = nullptr;
-    CIECU_CUDA(pool_alloc(&d_table, sizeof(int) * (kHashSlots + 1), st));
+    if (pool_alloc(&d_table, sizeof(int) * (kHashSlots + 1), st) != cudaSuccess) {
+        cudaGetLastError();  // no room for the analysis: no copy either
+        return CIECU_OK;
+    }
     std::vector<int> h(kHashSlots + 1, kEmpty);
     h[kHashSlots] = 0;  // reject flag
     cudaError_t e = cudaMemcpyAsync(d_table, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, st);

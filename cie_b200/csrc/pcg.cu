@@ -892,8 +892,11 @@ int plan_persistent(ciecu_pcg_s* S) {
     CIECU_CUDA(cudaGetDevice(&device));
     CIECU_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     const int sms = sm_count();
-    if (!S->split) CIECU_CUDA(pool_alloc(&S->split, sizeof(int2) * (sms + 1), st));
     S->fits = false;
+    if (!S->split && pool_alloc(&S->split, sizeof(int2) * (sms + 1), st) != cudaSuccess) {
+        cudaGetLastError();  // no room: not this time
+        return CIECU_OK;
+    }
     for (int G : {std::max(1, sms / 4), std::max(1, sms / 2), sms}) {
         persistent_split_kernel<<<(G + 1 + 127) / 128, 128, 0, st>>>(A->rowptr, A->rows, A->nnz, G, S->split);
         count_launch();
@@ -1371,8 +1374,14 @@ int ciecu_pcg_product(ciecu_pcg S, double inScale, const double* d_in, double ou
         else if (automatic) CIECU_TRY(use_persistent(S, &persistent));
     }
     if (persistent) {
-        CIECU_TRY(ensure_persistent_buffers(S));
-    } else {
+        const int status = ensure_persistent_buffers(S);
+        if (status != CIECU_OK && !automatic) return status;
+        if (status != CIECU_OK) {  // no room: the graph loop
+            cudaGetLastError();
+            persistent = S->dp = S->sliced = false;
+        }
+    }
+    if (!persistent) {
         if (!automatic) CIECU_TRY(refresh_dia(S, st));
         CIECU_TRY(tune_solver_spmv(S));
     }

@@ -163,16 +163,20 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (d_scratch) cudaFreeAsync(d_scratch, st);
     if (d_steps) cudaFreeAsync(d_steps, st);
-    if (e != cudaSuccess || status != CIECU_OK) {
-        sp_destroy(p);
-        p.state = 0;
-        return status != CIECU_OK ? status : cuda_fail(e, "sliced copy: shape");
-    }
     auto unsuitable = [&]() {
         sp_destroy(p);
         p.state = 2;
         return CIECU_OK;
     };
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();  // no room: the caller keeps its other loop
+        return unsuitable();
+    }
+    if (e != cudaSuccess || status != CIECU_OK) {
+        sp_destroy(p);
+        p.state = 0;
+        return status != CIECU_OK ? status : cuda_fail(e, "sliced copy: shape");
+    }
     if (64.0 * steps > 1.6 * static_cast<double>(csr->nnz) + 65536.0) return unsuitable();
     int span = 0;
     for (int s = 0; s < systems; ++s) {
@@ -295,6 +299,10 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the host lists are in use until here
     if (d_origin) cudaFreeAsync(d_origin, st);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return unsuitable();
+    }
     if (e != cudaSuccess) {
         sp_destroy(p);
         p.state = 0;

@@ -75,8 +75,11 @@ cudaError_t device_pool(cudaMemPool_t* pool) {
 }
 }  // namespace
 
+thread_local int t_failAllocation = 0;  // ciecu_debug_fail_allocation
+
 cudaError_t pool_alloc(void** ptr, size_t bytes, cudaStream_t stream) {
     *ptr = nullptr;
+    if (t_failAllocation > 0 && --t_failAllocation == 0) return cudaErrorMemoryAllocation;
     cudaMemPool_t pool = nullptr;
     const cudaError_t e = device_pool(&pool);
     if (e != cudaSuccess) return e;
@@ -226,6 +229,12 @@ int ciecu_last_error(char* h_buffer, int size) {
         h_buffer[size - 1] = '\0';
     }
     return static_cast<int>(message.size());
+}
+
+int ciecu_debug_fail_allocation(int which) {
+    CIECU_REQUIRE(which >= 0, "debug_fail_allocation: negative number");
+    t_failAllocation = which;
+    return CIECU_OK;
 }
 
 int64_t ciecu_kernel_launch_count(void) { return g_launches.load(); }

@@ -57,6 +57,9 @@ typedef struct ciecu_statistics {
 int ciecu_last_error(char* h_buffer, int size);
 /* Number of kernels this library launched since load (instrumentation). */
 int64_t ciecu_kernel_launch_count(void);
+/* For tests of what happens without room on the device: the calling thread's allocation of
+ * that number from the library's pool, counted from 1, fails (once); 0: none does. */
+int ciecu_debug_fail_allocation(int which);
 int ciecu_device_info(int* smCount, int* ccMajor, int* ccMinor);
 
 /* ---- space: SYCLSpace / DefaultSpace counterpart ------------------------------

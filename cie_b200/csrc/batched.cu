@@ -724,6 +724,7 @@ struct ciecu_batch_s {
     // Single launch over sliced rows (FP64).
     std::vector<long long> rowOffsets;
     ciecu::SpPlan sp{};
+    bool sliced = false;  // the last FP64 solve ran that way
     double* p1 = nullptr;
     int* abortFlag = nullptr;
     unsigned long long epoch = 1;
@@ -864,17 +865,37 @@ int run_level(ciecu_batch_s* B, Level<T>& L, const BatchGlobal& g0, unsigned pre
     return CIECU_OK;
 }
 
+// Where the batch takes the single launch.  A block works on one part at a time, the tile
+// kernels on all systems at once: 25 us an iteration for few of them, then with every 740
+// tiles more (five to an SM).  Up to four parts for each block the single launch is faster
+// whatever their size, up to seven with 5,000 stored entries in a part, beyond that with
+// 8,192.  Microseconds an iteration, single launch / tiles: systems of 81 rows (625 entries)
+// 592 of them 30 / 29, 740 34 / 32, 4,096 165 / 116; of 289 rows (2,401) 23 / 25, 29 / 27,
+// 153 / 114; of 625 rows (5,329) 740 32 / 31, 1,024 44 / 47, 2,048 87 / 74; of 1,089 rows
+// (9,409) 1,024 59 / 69, 4,096 230 / 262.  Long rows only add to it: 592 systems of 3D order
+// 4 (rows of 729) 354 / 477.
+bool batch_rounds(double rounds, double entries) {
+    return rounds <= 4.0 || entries >= 8192.0 || (rounds <= 7.0 && entries >= 5000.0);
+}
+
+SpLimits batch_limits() {
+    SpLimits limits;
+    limits.rows = kSpRows;
+    limits.rounds = batch_rounds;
+    return limits;
+}
+
 constexpr long long kBatchLaunchIterations = 4096;
 constexpr long long kBatchWaitNs = 20000000000LL;
 
 // The FP64 solve as single launches; *used = false when the matrix does not suit
-// (sp_build).  The right-hand side is in L.r on entry.  64 uneven Q2 systems of 16 to
+// (batch_limits, sp_build).  The right-hand side is in L.r on entry.  64 uneven Q2 systems of 16 to
 // 128 cells a side: 68 ms, by the graph of three kernels 137 ms.
 int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
     *used = false;
     cudaStream_t st = B->A->space->stream;
     Level<double>& L = B->f64;
-    CIECU_TRY(sp_build(B->sp, B->A, B->rowOffsets, kSpRows, st));
+    CIECU_TRY(sp_build(B->sp, B->A, B->rowOffsets, batch_limits(), st));
     if (B->sp.state != 1) return CIECU_OK;
     if (!B->p1) {
         cudaError_t e = pool_alloc(&B->p1, sizeof(double) * static_cast<size_t>(std::max<long>(1, B->n)), st);
@@ -1202,6 +1223,13 @@ int ciecu_batch_info(ciecu_batch B, int* lanesPerRow, int* deviceLoop, int64_t* 
     return CIECU_OK;
 }
 
+int ciecu_batch_form(ciecu_batch B, int* form) {
+    CIECU_REQUIRE(B && form, "batch_form: null argument");
+    const bool f64 = B->reliableDelta == 0.0 && B->innerTolerance == 0.0;
+    *form = f64 && B->sliced ? CIECU_BATCH_SINGLE_SLICED : CIECU_BATCH_GRAPH_TILES;
+    return CIECU_OK;
+}
+
 int ciecu_batch_set_refinement(ciecu_batch B, double innerTolerance) {
     CIECU_REQUIRE(B, "batch_set_refinement: null solver");
     CIECU_REQUIRE(innerTolerance >= 0.0 && innerTolerance < 1.0, "batch_set_refinement: tolerance must be in [0, 1)");
@@ -1263,9 +1291,8 @@ int ciecu_batch_product(ciecu_batch B, double inScale, const double* d_in, doubl
         } else if (B->innerTolerance == 0.0) {
             // FP64: every system runs ConjugateGradients_impl.hpp:49-201 as it is
             CIECU_CUDA(cudaMemsetAsync(B->d_s, 0, sizeof(BatchScalars) * B->systems, st));
-            bool sliced = false;
-            CIECU_TRY(run_sliced(B, g, &sliced));
-            if (!sliced) CIECU_TRY(run_level(B, L, g, 0u));
+            CIECU_TRY(run_sliced(B, g, &B->sliced));
+            if (!B->sliced) CIECU_TRY(run_level(B, L, g, 0u));
             CIECU_CUDA(cudaMemcpyAsync(s.data(), B->d_s, sizeof(BatchScalars) * B->systems, cudaMemcpyDeviceToHost,
                                        st));
             CIECU_CUDA(cudaStreamSynchronize(st));

@@ -1058,10 +1058,50 @@ int launch_sliced_persistent(ciecu_pcg_s* S, cudaStream_t st) {
 
 // Lanes per row: as many as leave one lane group per row of the largest block,
 // and no more than the average row needs.
-template <bool PRE>
-int launch_persistent_rows(ciecu_pcg_s* S, cudaStream_t st) {
+int persistent_lanes(const ciecu_pcg_s* S) {
     int vs = 32;
     while (vs > 1 && (kPT / vs < S->maxRows || vs / 2 >= S->A->avgRow)) vs >>= 1;
+    return vs;
+}
+
+// Where a matrix without a DIA copy takes the single launch over sliced rows, a thread a
+// row; the others are the single launch over CSR rows in shared memory, where they fit, and
+// the graph loop.
+//   Long rows.  A row's chain takes 20.5 ns an entry here, 160 ns over the lanes of a row
+// there, whose iterations begin 3.9, 4.5 and 7 us later (37, 74 and 148 blocks).  Measured
+// us an iteration, sliced against CSR rows: Q3 3D 2^3 cells (rows of 343) 13.9 / 12.0, 4^3
+// 14.0 / 14.5, 8^3 17.1 / 22.2; Q4 3D 2^3 (729) 20.4 / 13.3; one row of 600 among 20,000 of
+// 20 19.4 / 67.2.  Against the graph, where the rows do not fit, rows above 640 count where
+// there are many of them and they show in the padding.  Q10 2D 16^2 (441, 17 % padding)
+// 19.5 / 26.6, 40,000 rows of 801 (none) 66 / 83, Q4 3D 8^3 (24 %) 48 / 33, Q5 3D 4^3
+// (1,331, 35 %) 37.6 / 26.1.
+//   Wide windows.  Each block forms its window, 0.5 us for 1,000 entries: up to 12,288, or
+// with 16 stored entries for each.  Random columns, 6 / 60 entries a row, against CSR rows:
+// 5,000 rows 10.5 / 12.4 against 11.4 / 17.6, 14,000 rows 19.6 / 21.1 against 12.5 / 24.3.
+constexpr int kShortRow = 250;  // faster than CSR rows whatever their lanes
+
+int sliced_limits(ciecu_pcg_s* S, SpLimits* out, bool* tried) {
+    *out = SpLimits{};
+    *tried = true;
+    out->window = 12288;
+    out->entriesPerColumn = 16;
+    const int longest = S->A->maxRow;
+    if (longest <= kShortRow) return CIECU_OK;
+    CIECU_TRY(plan_persistent(S));
+    if (!S->fits) {
+        out->longRows = 8;
+        out->padding = 1.2;
+        return CIECU_OK;
+    }
+    const int lanes = persistent_lanes(S), sms = sm_count();
+    const double later = S->grid <= sms / 4 ? 3900.0 : (S->grid <= sms / 2 ? 4500.0 : 7000.0);
+    *tried = longest <= (lanes <= 2 ? 2 : 1) * kLongRow && (20.5 - 160.0 / lanes) * longest <= later;
+    return CIECU_OK;
+}
+
+template <bool PRE>
+int launch_persistent_rows(ciecu_pcg_s* S, cudaStream_t st) {
+    const int vs = persistent_lanes(S);
     switch (vs) {
         case 32: return launch_persistent<32, PRE>(S, st);
         case 16: return launch_persistent<16, PRE>(S, st);
@@ -1366,7 +1406,13 @@ int ciecu_pcg_product(ciecu_pcg S, double inScale, const double* d_in, double ou
             S->dp = S->dpState == 1;
         }
         if (!S->dp) {
-            CIECU_TRY(sp_build(S->sp, A, {0, n}, LONG_MAX, st));
+            if (S->sp.state == 0) {
+                SpLimits limits;
+                bool tried = false;
+                CIECU_TRY(sliced_limits(S, &limits, &tried));
+                if (tried) CIECU_TRY(sp_build(S->sp, A, {0, n}, limits, st));
+                else S->sp.state = 2;
+            }
             S->sliced = S->sp.state == 1;
             if (S->sliced) CIECU_TRY(sp_fill(S->sp, A, st));
         }

@@ -6,6 +6,9 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <iterator>
+#include <set>
+#include <utility>
 
 namespace ciecu {
 namespace {
@@ -99,7 +102,7 @@ int sp_fill(const SpPlan& p, const ciecu_csr_s* csr, cudaStream_t st) {
     return CIECU_OK;
 }
 
-int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& rowOffsets, long mostRows,
+int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& rowOffsets, const SpLimits& limits,
              cudaStream_t st) {
     if (p.state != 0) return CIECU_OK;
     p.state = 2;
@@ -110,6 +113,10 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     CIECU_CUDA(cudaGetDevice(&device));
     CIECU_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
     const int sms = std::min(sm_count(), kDpMaxBlocks);
+    auto tooMany = [&](long parts) {
+        return limits.rounds && !limits.rounds(static_cast<double>(parts) / sms, static_cast<double>(csr->nnz) / parts);
+    };
+    if (tooMany(systems)) return CIECU_OK;  // each has a part at least
     const long budget = (optin > 4096 ? optin - 4096 : 0) / static_cast<long>(sizeof(double));
     // runs of kSpSort rows, none across two systems
     std::vector<int> runRow, runEnd, runSystem, sliceBase(static_cast<size_t>(systems));
@@ -178,6 +185,8 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
         return status != CIECU_OK ? status : cuda_fail(e, "sliced copy: shape");
     }
     if (64.0 * steps > 1.6 * static_cast<double>(csr->nnz) + 65536.0) return unsuitable();
+    if (csr->longRows > limits.longRows && 64.0 * steps > limits.padding * static_cast<double>(csr->nnz))
+        return unsuitable();
     int span = 0;
     for (int s = 0; s < systems; ++s) {
         lo[s] = std::min(lo[s], 0);
@@ -188,7 +197,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     }
     // Rows of a block: all blocks busy with one part each where that is possible,
     // and at most mostRows or what shared memory holds beside the widest window.
-    const long most = std::min<long>(mostRows, (budget - span - 8) * 2 / 7) / kSpSort * kSpSort;
+    const long most = std::min<long>(limits.rows, (budget - span - 8) * 2 / 7) / kSpSort * kSpSort;
     if (most < kSpSort) return unsuitable();
     long R = std::min(most, ((n + sms - 1) / sms + kSpSort - 1) / kSpSort * kSpSort);
     auto parts = [&](long rowsEach) {
@@ -196,10 +205,13 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
         for (int s = 0; s < systems; ++s) c += (rowOffsets[s + 1] - rowOffsets[s] + rowsEach - 1) / rowsEach;
         return c;
     };
-    while (R + kSpSort <= most && parts(R) > sms) R += kSpSort;
+    while (R + kSpSort <= most && (systems > sms || parts(R) > sms)) R += kSpSort;
     long largest = 0;
     for (int s = 0; s < systems; ++s) largest = std::max<long>(largest, rowOffsets[s + 1] - rowOffsets[s]);
     if ((largest + R - 1) / R > sms) return unsuitable();  // a system needs more blocks than are resident
+    const long allParts = parts(R);
+    if (tooMany(allParts)) return unsuitable();
+    if (R + span > limits.window && csr->nnz < limits.entriesPerColumn * (R + span)) return unsuitable();
     // Systems in descending size to the blocks that are free first; a block's time is
     // measured in iterations, which grow with the square root of a 2D system's rows.
     std::vector<int> order(static_cast<size_t>(systems));
@@ -207,22 +219,24 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return rowOffsets[a + 1] - rowOffsets[a] > rowOffsets[b + 1] - rowOffsets[b];
     });
-    const int G = static_cast<int>(std::min<long>(sms, std::max<long>(1, parts(R))));
-    std::vector<double> freeAt(static_cast<size_t>(G), 0.0);
+    const int G = static_cast<int>(std::min<long>(sms, std::max<long>(1, allParts)));
     std::vector<std::vector<SpItem>> lists(static_cast<size_t>(G));
-    std::vector<int> blocks(static_cast<size_t>(G));
+    // the blocks by the time they are free, equal ones in order
+    std::set<std::pair<double, int>> blocks;
+    for (int b = 0; b < G; ++b) blocks.emplace(0.0, b);
+    std::vector<std::pair<double, int>> taken;
     int slots = 0, rowsMost = kSpSort;
     for (int s : order) {
         const long ns = rowOffsets[s + 1] - rowOffsets[s];
         if (ns == 0) continue;
         const int c = static_cast<int>((ns + R - 1) / R);
         const int each = static_cast<int>(((ns + c - 1) / c + kSpSort - 1) / kSpSort * kSpSort);
-        for (int b = 0; b < G; ++b) blocks[b] = b;
-        std::stable_sort(blocks.begin(), blocks.end(), [&](int a, int b) { return freeAt[a] < freeAt[b]; });
         const int used = static_cast<int>((ns + each - 1) / each);
-        const double start = freeAt[blocks[used - 1]];
+        taken.assign(blocks.begin(), std::next(blocks.begin(), used));
+        blocks.erase(blocks.begin(), std::next(blocks.begin(), used));
+        const double start = taken.back().first;
         for (int k = 0; k < used; ++k) {
-            const int b = blocks[k];
+            const int b = taken[k].second;
             const long begin = rowOffsets[s] + static_cast<long>(k) * each;
             SpItem I{};
             I.system = s;
@@ -238,7 +252,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
             I.slotBase = slots;
             lists[b].push_back(I);
             rowsMost = std::max(rowsMost, each);
-            freeAt[b] = start + std::sqrt(static_cast<double>(ns)) * (1000.0 + each);
+            blocks.emplace(start + std::sqrt(static_cast<double>(ns)) * (1000.0 + each), b);
         }
         slots += used;
     }

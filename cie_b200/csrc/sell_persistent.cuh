@@ -43,6 +43,7 @@
 
 #include "dia_persistent.cuh"
 
+#include <climits>
 #include <vector>
 
 namespace ciecu {
@@ -274,11 +275,22 @@ struct SpPlan {
     DpSlot* slots = nullptr;
 };
 
+// Where this form is taken; the caller has another one outside.
+struct SpLimits {
+    long rows = LONG_MAX;      // rows of a block at most
+    // Rows of more than kLongRow entries (one thread sums each), or ...
+    int longRows = INT_MAX;
+    double padding = 0.0;      // ... this share of the copy's entries to the matrix's, with more of them
+    long window = LONG_MAX;    // window entries of a block, or ...
+    long entriesPerColumn = 0; // ... this many stored entries for each of them: every block forms its own
+    // parts for each block at most, by the stored entries of a part on average
+    bool (*rounds)(double rounds, double entries) = nullptr;
+};
+
 // Builds the copy's layout and column offsets and the plan for the systems
-// [rowOffsets[s], rowOffsets[s + 1]) of a block-diagonal FP64 CSR matrix; state 2 when
-// the windows do not fit in shared memory or padding takes over 60 %.
-// A block takes at most `mostRows` rows.
-int sp_build(SpPlan& plan, const ciecu_csr_s* csr, const std::vector<long long>& rowOffsets, long mostRows,
+// [rowOffsets[s], rowOffsets[s + 1]) of a block-diagonal FP64 CSR matrix; state 2 outside
+// the limits, and when the windows do not fit in shared memory or padding takes over 60 %.
+int sp_build(SpPlan& plan, const ciecu_csr_s* csr, const std::vector<long long>& rowOffsets, const SpLimits& limits,
              cudaStream_t st);
 // The copy's values from the live CSR values.
 int sp_fill(const SpPlan& plan, const ciecu_csr_s* csr, cudaStream_t st);

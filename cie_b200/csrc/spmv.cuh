@@ -259,6 +259,8 @@ int with_schedule(int kernel, F&& f) {
     }
 }
 
+constexpr int kLongRow = 640;
+
 }  // namespace ciecu
 
 struct ciecu_csr_s {
@@ -274,6 +276,7 @@ struct ciecu_csr_s {
     int* d_blocks = nullptr;
     int nblocks = 0;
     int maxRow = 0;
+    int longRows = 0;  // rows of more than ciecu::kLongRow entries
     double avgRow = 0.0;
     int diaState = 0;             // 0 not analysed, 1 DIA offsets found, 2 not a few-diagonal matrix
     std::vector<int> diaOffsets;  // ascending diagonal offsets (dia.cuh)

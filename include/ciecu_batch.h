@@ -39,6 +39,10 @@ int ciecu_batch_info(ciecu_batch solver, int* lanesPerRow, int* deviceLoop, int6
  * system; the other systems are solved and their statistics filled. */
 int ciecu_batch_product(ciecu_batch solver, double inScale, const double* d_in, double outScale,
                         double* d_out, ciecu_statistics* h_stats);
+/* How the last FP64 solve ran: all systems at once in tiles, three kernels an iteration, or a
+ * few at a time in a single launch over sliced rows. */
+enum { CIECU_BATCH_GRAPH_TILES = 0, CIECU_BATCH_SINGLE_SLICED = 1 };
+int ciecu_batch_form(ciecu_batch solver, int* form);
 /* innerTolerance > 0: later products run FP32 inner solves with FP64 refinement
  * -- each round solves the FP32 copy of the matrix to innerTolerance relative
  * to the current residual for the systems not yet converged, adds the

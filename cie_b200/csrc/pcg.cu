@@ -1071,10 +1071,11 @@ int persistent_lanes(const ciecu_pcg_s* S) {
 // there, whose iterations begin 3.9, 4.5 and 7 us later (37, 74 and 148 blocks).  Measured
 // us an iteration, sliced against CSR rows: Q3 3D 2^3 cells (rows of 343) 13.9 / 12.0, 4^3
 // 14.0 / 14.5, 8^3 17.1 / 22.2; Q4 3D 2^3 (729) 20.4 / 13.3; one row of 600 among 20,000 of
-// 20 19.4 / 67.2.  Against the graph, where the rows do not fit, rows above 640 count where
-// there are many of them and they show in the padding.  Q10 2D 16^2 (441, 17 % padding)
-// 19.5 / 26.6, 40,000 rows of 801 (none) 66 / 83, Q4 3D 8^3 (24 %) 48 / 33, Q5 3D 4^3
-// (1,331, 35 %) 37.6 / 26.1.
+// 20 19.4 / 67.2; one of 4,000 among 4,000, by a warp, 15.2 / 64.7.  Against the graph, where
+// the rows do not fit, more than a few rows above kLongRow count where they show in the
+// padding or have over 1,024 entries: Q10 2D 16^2 (441, 17 % padding) 19.5 / 26.6, 40,000 rows
+// of 801 (none) 66 / 83, Q4 3D 8^3 (24 %) 48 / 33, Q5 3D 4^3 (1,331, 35 %) 37.6 / 26.1, 2,197
+// rows of 1,261 on average 53 / 23.
 //   Wide windows.  Each block forms its window, 0.5 us for 1,000 entries: up to 12,288, or
 // with 16 stored entries for each.  Random columns, 6 / 60 entries a row, against CSR rows:
 // 5,000 rows 10.5 / 12.4 against 11.4 / 17.6, 14,000 rows 19.6 / 21.1 against 12.5 / 24.3.
@@ -1088,14 +1089,16 @@ int sliced_limits(ciecu_pcg_s* S, SpLimits* out, bool* tried) {
     const int longest = S->A->maxRow;
     if (longest <= kShortRow) return CIECU_OK;
     CIECU_TRY(plan_persistent(S));
+    const bool few = S->A->longRows <= kFewLongRows;  // warps sum those
     if (!S->fits) {
-        out->longRows = 8;
+        *tried = few || longest <= 1024;
         out->padding = 1.2;
         return CIECU_OK;
     }
     const int lanes = persistent_lanes(S), sms = sm_count();
     const double later = S->grid <= sms / 4 ? 3900.0 : (S->grid <= sms / 2 ? 4500.0 : 7000.0);
-    *tried = longest <= (lanes <= 2 ? 2 : 1) * kLongRow && (20.5 - 160.0 / lanes) * longest <= later;
+    *tried = (few || longest <= (lanes <= 2 ? 2 : 1) * kLongRow) &&
+             (20.5 - 160.0 / lanes) * (few ? std::min(longest, kLongRow) : longest) <= later;
     return CIECU_OK;
 }
 

@@ -18,12 +18,12 @@ constexpr int kT = 256;
 // Deals the rows of each run of kSpSort rows (one block of kSpSort threads; `runRow`
 // the run's first row, `runEnd` its system's end) to its slices by descending length,
 // equal lengths in row order; the steps of the slices and the smallest and largest
-// column offset of the run's system.
+// column offset of the run's system.  Rows of more than `longest` entries are in no slice.
 __global__ void __launch_bounds__(kSpSort) sp_shape_kernel(const int* __restrict__ runRow,
                                                            const int* __restrict__ runEnd,
                                                            const int* __restrict__ runSystem,
                                                            const int* __restrict__ rowptr, const int* __restrict__ col,
-                                                           int* __restrict__ row, int* __restrict__ steps,
+                                                           int longest, int* __restrict__ row, int* __restrict__ steps,
                                                            int* __restrict__ lo, int* __restrict__ hi) {
     __shared__ int s_len[kSpSort];
     constexpr int kSlices = kSpSort / 32;
@@ -38,12 +38,14 @@ __global__ void __launch_bounds__(kSpSort) sp_shape_kernel(const int* __restrict
             mx = max(mx, col[k] - r);
         }
     }
+    const bool sliced = live && len <= longest;
+    if (!sliced) len = -1;
     s_len[i] = len;
     __syncthreads();
     int place = 0;
     for (int j = 0; j < kSpSort; ++j) place += s_len[j] > len || (s_len[j] == len && j < i) ? 1 : 0;
     const long slice = static_cast<long>(blockIdx.x) * kSlices + place / 32;
-    row[slice * 32 + place % 32] = live ? r : -1;
+    row[slice * 32 + place % 32] = sliced ? r : -1;
     if (place % 32 == 0) steps[slice] = (max(len, 0) + 1) / 2;  // the slice's longest row
     mn = __reduce_min_sync(0xffffffffu, mn);
     mx = __reduce_max_sync(0xffffffffu, mx);
@@ -89,7 +91,7 @@ __global__ void sp_fill_kernel(long slices, const int* __restrict__ row, const i
 }  // namespace
 
 void sp_destroy(SpPlan& p) {
-    pool_release({p.val, p.off, p.sliceStep, p.row, p.items, p.itemBegin, p.slots});
+    pool_release({p.val, p.off, p.sliceStep, p.row, p.longRow, p.items, p.itemBegin, p.slots});
     p = SpPlan{};
 }
 
@@ -130,6 +132,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     }
     const long runs = static_cast<long>(runRow.size()), slices = runs * (kSpSort / 32);
     if (slices == 0) return CIECU_OK;
+    const bool few = csr->longRows <= kFewLongRows;  // those rows are in no slice
     int *d_scratch = nullptr, *d_steps = nullptr;
     auto bytes = [](long k) { return sizeof(int) * static_cast<size_t>(std::max<long>(k, 1)); };
     cudaError_t e = pool_alloc(&p.row, bytes(slices * 32), st);
@@ -154,7 +157,8 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     int status = CIECU_OK, steps = 0;
     if (e == cudaSuccess) {
         sp_shape_kernel<<<static_cast<unsigned>(runs), kSpSort, 0, st>>>(d_row, d_end, d_system, csr->rowptr, csr->col,
-                                                                        p.row, d_steps, d_lo, d_hi);
+                                                                        few ? kLongRow : INT_MAX, p.row, d_steps, d_lo,
+                                                                        d_hi);
         count_launch();
         e = cudaGetLastError();
     }
@@ -185,8 +189,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
         return status != CIECU_OK ? status : cuda_fail(e, "sliced copy: shape");
     }
     if (64.0 * steps > 1.6 * static_cast<double>(csr->nnz) + 65536.0) return unsuitable();
-    if (csr->longRows > limits.longRows && 64.0 * steps > limits.padding * static_cast<double>(csr->nnz))
-        return unsuitable();
+    if (!few && 64.0 * steps > limits.padding * static_cast<double>(csr->nnz)) return unsuitable();
     int span = 0;
     for (int s = 0; s < systems; ++s) {
         lo[s] = std::min(lo[s], 0);
@@ -225,6 +228,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     std::set<std::pair<double, int>> blocks;
     for (int b = 0; b < G; ++b) blocks.emplace(0.0, b);
     std::vector<std::pair<double, int>> taken;
+    const std::vector<int> longRows(csr->longRow, csr->longRow + (few ? csr->longRows : 0));
     int slots = 0, rowsMost = kSpSort;
     for (int s : order) {
         const long ns = rowOffsets[s + 1] - rowOffsets[s];
@@ -250,6 +254,9 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
             I.lo = lo[s];
             I.span = hi[s] - lo[s];
             I.slotBase = slots;
+            const auto first = std::lower_bound(longRows.begin(), longRows.end(), I.rowBegin);
+            I.longBegin = static_cast<int>(first - longRows.begin());
+            I.longRows = static_cast<int>(std::lower_bound(first, longRows.end(), I.rowBegin + I.rows) - first);
             lists[b].push_back(I);
             rowsMost = std::max(rowsMost, each);
             blocks.emplace(start + std::sqrt(static_cast<double>(ns)) * (1000.0 + each), b);
@@ -284,6 +291,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     const size_t slotBytes = sizeof(DpSlot) * kSpWords * static_cast<size_t>(std::max(slots, 1));
     e = pool_alloc(&p.val, sizeof(double2) * std::max<size_t>(pairs, 1), st);
     if (e == cudaSuccess) e = pool_alloc(&p.off, sizeof(short2) * std::max<size_t>(pairs, 1), st);
+    if (e == cudaSuccess) e = pool_alloc(&p.longRow, bytes(static_cast<long>(longRows.size())), st);
     if (e == cudaSuccess) e = pool_alloc(&p.items, sizeof(SpItem) * std::max<size_t>(items.size(), 1), st);
     if (e == cudaSuccess) e = pool_alloc(&p.itemBegin, sizeof(int) * begin.size(), st);
     if (e == cudaSuccess) e = pool_alloc(&p.slots, slotBytes, st);
@@ -292,6 +300,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
         e = cudaMemcpyAsync(p.items, items.data(), sizeof(SpItem) * items.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(p.itemBegin, begin.data(), sizeof(int) * begin.size(), cudaMemcpyHostToDevice, st);
+    up(p.longRow, longRows);
     if (e != cudaSuccess) {
         cudaGetLastError();  // no room for the copy: the caller keeps its other loop
         return unsuitable();
@@ -322,7 +331,8 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
         p.state = 0;
         return cuda_fail(e, "sliced copy: offsets");
     }
-    p.args.A = SpMatrix{p.val, p.off, p.sliceStep, p.row};
+    p.args.A = SpMatrix{p.val, p.off, p.sliceStep, p.row, p.longRow, csr->rowptr, csr->col,
+                        static_cast<const double*>(csr->val)};
     p.args.items = p.items;
     p.args.itemBegin = p.itemBegin;
     p.args.slots = p.slots;

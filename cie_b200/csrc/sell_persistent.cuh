@@ -18,7 +18,11 @@
 // 36 % padding with the rows as they come) (a row of one entry per lane and 12-byte entries is bound by the
 // requests, about one per 6 cycles and SM, before it is by L2).  Padding has value 0
 // and offset 0.  A row is summed by one thread in column order, one FMA per entry:
-// the sequential sum of CSROperator.cpp:49-56.  The operand entries of a block's rows
+// the sequential sum of CSROperator.cpp:49-56.  Up to kFewLongRows rows of more than kLongRow
+// entries are summed by a warp each instead, from the matrix itself: 75,777 rows of 48 and
+// two of 8,300 27 us an iteration, 190 with a thread for each; 300,000 rows and two of 3,650
+// 40 and 219.  (Where all rows are long a thread for each is better: 40,000 rows of 801 66,
+// 115 by warps.)  The operand entries of a block's rows
 // lie in one window of R + span columns, formed in shared memory from the z and
 // p_{k-1} of the owners: even columns in its first half, odd ones in its second
 // (sp_place), as the rows of a slice are mostly every other row or neighbours, and
@@ -52,6 +56,7 @@ constexpr int kSpThreads = 512;      // at most: 16 warps of up to 128 registers
 constexpr int kSpSort = 128;         // rows that share their slices; parts are multiples of it
 constexpr int kSpRows = 2816;        // rows of a block at most: 148 blocks' matrices stay in L2 (Q2: 200 B a row)
 constexpr int kSpUnroll = 12;        // steps of a row in flight
+constexpr int kSpLongUnroll = 8;     // entries of a lane in flight in a long row
 
 struct SpItem {
     int system, part, parts;  // part of the system's `parts` blocks
@@ -60,6 +65,7 @@ struct SpItem {
     int sysBegin, sysEnd;     // rows of the system
     int lo, span;             // window: columns rowBegin + lo .. rowBegin + rows - 1 + lo + span
     int slotBase;             // words of the system start at slotBase * kSpWords
+    int longBegin, longRows;  // the part's rows that are in no slice
 };
 
 constexpr int kSpWords = 2 * 2 * kDpCopies;  // words a block has: sets x values x copies
@@ -69,6 +75,11 @@ struct SpMatrix {
     const short2* __restrict__ off;
     const int* __restrict__ sliceStep;  // first step of each slice; one past the last
     const int* __restrict__ row;        // 32 per slice: the lane's row (-1: none)
+    const int* __restrict__ longRow;    // rows that are in no slice, ascending
+    // the matrix itself, for these
+    const int* __restrict__ rowptr;
+    const int* __restrict__ col;
+    const double* __restrict__ entries;
 };
 
 struct SpArgs {
@@ -209,6 +220,29 @@ __device__ __forceinline__ void sp_solve(const SpArgs& P, typename Ctl::Scalars*
                     pq = fma(operand[0], sum, pq);
                 }
             }
+            // A long row to a warp, from the matrix itself: one thread would take 20 ns an entry.
+            for (int k = warp; k < I.longRows; k += warps) {
+                const int row = P.A.longRow[I.longBegin + k], k1 = P.A.rowptr[row + 1];
+                const int at = -rb - I.lo, half = P.winLen / 2;
+                double sum = 0.0;
+                for (int e = P.A.rowptr[row] + lane; e < k1; e += 32 * kSpLongUnroll) {
+                    double a[kSpLongUnroll];
+                    int c[kSpLongUnroll];
+#pragma unroll
+                    for (int u = 0; u < kSpLongUnroll; ++u) {
+                        const bool in = e + 32 * u < k1;
+                        a[u] = in ? __ldg(P.A.entries + e + 32 * u) : 0.0;
+                        c[u] = in ? __ldg(P.A.col + e + 32 * u) : row;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kSpLongUnroll; ++u) sum = fma(a[u], s_win[sp_place(c[u] + at, half)], sum);
+                }
+                sum = warp_sum(sum);
+                if (lane == 0) {
+                    sq[row - rb] = sum;
+                    pq = fma(s_win[sp_place(row + at, half)], sum, pq);
+                }
+            }
             __syncthreads();
             {
                 const double mine[1] = {pq};
@@ -270,6 +304,7 @@ struct SpPlan {
     short2* off = nullptr;
     int* sliceStep = nullptr;
     int* row = nullptr;  // 32 per slice
+    int* longRow = nullptr;
     SpItem* items = nullptr;
     int* itemBegin = nullptr;
     DpSlot* slots = nullptr;
@@ -278,9 +313,9 @@ struct SpPlan {
 // Where this form is taken; the caller has another one outside.
 struct SpLimits {
     long rows = LONG_MAX;      // rows of a block at most
-    // Rows of more than kLongRow entries (one thread sums each), or ...
-    int longRows = INT_MAX;
-    double padding = 0.0;      // ... this share of the copy's entries to the matrix's, with more of them
+    // This share of the copy's entries to the matrix's, at most, where a thread each sums
+    // more rows of over kLongRow entries than kFewLongRows.
+    double padding = 1e30;
     long window = LONG_MAX;    // window entries of a block, or ...
     long entriesPerColumn = 0; // ... this many stored entries for each of them: every block forms its own
     // parts for each block at most, by the stored entries of a part on average

@@ -232,7 +232,7 @@ int ciecu_csr_create(ciecu_space space, int32_t rowCount, int32_t columnCount, i
         return fail(CIECU_ERR_ARGUMENT, "number of column indices (" + std::to_string(nnz) +
                                             ") is inconsistent with the row extents of the provided CSR matrix");
     }
-    int maxRow = 0, longRows = 0;
+    int maxRow = 0;
     for (int r = 0; r < rowCount; ++r) {
         const int len = rowptr[r + 1] - rowptr[r];
         if (len < 0) {
@@ -241,10 +241,9 @@ int ciecu_csr_create(ciecu_space space, int32_t rowCount, int32_t columnCount, i
                                                 std::to_string(r));
         }
         maxRow = std::max(maxRow, len);
-        longRows += len > kLongRow;
+        if (len > kLongRow && csr->longRows++ < kFewLongRows) csr->longRow[csr->longRows - 1] = r;
     }
     csr->maxRow = maxRow;
-    csr->longRows = longRows;
     csr->avgRow = rowCount ? static_cast<double>(nnz) / rowCount : 0.0;
     const std::vector<int> blocks = make_row_blocks(rowptr, rowCount);
     staging.unlock();

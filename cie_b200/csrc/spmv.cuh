@@ -260,6 +260,7 @@ int with_schedule(int kernel, F&& f) {
 }
 
 constexpr int kLongRow = 640;
+constexpr int kFewLongRows = 8;
 
 }  // namespace ciecu
 
@@ -276,7 +277,9 @@ struct ciecu_csr_s {
     int* d_blocks = nullptr;
     int nblocks = 0;
     int maxRow = 0;
-    int longRows = 0;  // rows of more than ciecu::kLongRow entries
+    // rows of more than ciecu::kLongRow entries, and the first of them, ascending
+    int longRows = 0;
+    int longRow[ciecu::kFewLongRows] = {};
     double avgRow = 0.0;
     int diaState = 0;             // 0 not analysed, 1 DIA offsets found, 2 not a few-diagonal matrix
     std::vector<int> diaOffsets;  // ascending diagonal offsets (dia.cuh)

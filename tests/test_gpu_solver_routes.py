@@ -55,13 +55,19 @@ def tensor(dim, order, cells):
     return out
 
 
-def one_long_row(n, length):
+def long_rows(n, length, count=1):
+    """About 20 entries a row near the diagonal, and `count` rows of about `length` more, the
+    first and the last row among them when there are several."""
     rng = np.random.default_rng(n)
     rows = np.repeat(np.arange(n), 10)
-    near = np.clip(rows + rng.integers(1, 300, len(rows)), 0, n - 1)
-    first = max(0, n // 2 - length // 2)
-    rows = np.concatenate([rows, np.full(length, n // 2)])
-    cols = np.concatenate([near, first + np.arange(length)])
+    cols = np.minimum(rows + rng.integers(1, 300, len(rows)), n - 1)
+    keep = cols > rows
+    rows, cols = [rows[keep]], [cols[keep]]
+    for r in np.linspace(0, n - 1, count).astype(int) if count > 1 else [n // 2]:
+        first = min(max(0, r - length // 2), n - length)
+        rows.append(np.full(length, r))
+        cols.append(first + np.arange(length))
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
     m = sp.coo_matrix((np.ones(len(rows)), (rows, cols)), shape=(n, n)).tocsr()
     return m + m.T
 
@@ -76,10 +82,17 @@ def one_long_row(n, length):
     ("rows of 801, past shared memory", lambda: band(9000, 400), SLICED),
     ("3D order 3, 2 cells", lambda: tensor(3, 3, 2), CSR),
     ("3D order 3, 5 cells", lambda: tensor(3, 3, 5), SLICED),
-    ("3D order 4, 3 cells", lambda: tensor(3, 4, 3), CSR),
+    ("3D order 4, 2 cells", lambda: tensor(3, 4, 2), CSR),
+    ("3D order 4, 3 cells", lambda: tensor(3, 4, 3), SLICED),  # 8 rows of 729, by warps
+    ("rows of 1,201, past shared memory", lambda: band(4000, 600), GRAPH_CSR),
     ("3D order 4, 7 cells", lambda: tensor(3, 4, 7), GRAPH_CSR),
-    ("a row of 500 among 12,000", lambda: one_long_row(12000, 500), SLICED),
-    ("a row of 700 among 900", lambda: one_long_row(900, 700), CSR),
+    ("a row of 500 among 12,000", lambda: long_rows(12000, 500), SLICED),
+    ("a row of 700 among 900", lambda: long_rows(900, 700), CSR),
+    ("a row of 3,000 among 12,000", lambda: long_rows(12000, 3000), SLICED),
+    ("8 rows of 800 among 20,001", lambda: long_rows(20001, 800, 8), SLICED),
+    ("9 rows of 800 among 20,001", lambda: long_rows(20001, 800, 9), SLICED),  # few lanes a row there
+    ("9 rows of 800 among 2,001", lambda: long_rows(2001, 800, 9), CSR),
+    ("8 rows of 2,000, past shared memory", lambda: long_rows(140000, 2000, 8), SLICED),
     ("scattered, 4,000 rows of 6", lambda: scattered(4000, 6), SLICED),
     ("scattered, 9,000 rows of 6", lambda: scattered(9000, 6), CSR),
     ("scattered, 9,000 rows of 60", lambda: scattered(9000, 60), SLICED),

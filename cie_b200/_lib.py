@@ -125,6 +125,7 @@ SIGNATURES = {
     "ciecu_batch_destroy": (c_int, [P]),
     "ciecu_batch_info": (c_int, [P, P, P, P]),
     "ciecu_batch_form": (c_int, [P, P]),
+    "ciecu_batch_debug_exchange": (c_int, [P, c_int64, c_int64]),
     "ciecu_batch_product": (c_int, [P, c_double, P, c_double, P, P]),
     "ciecu_batch_set_refinement": (c_int, [P, c_double]),
     "ciecu_batch_set_reliable_updates": (c_int, [P, c_double]),

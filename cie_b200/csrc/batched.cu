@@ -725,6 +725,7 @@ struct ciecu_batch_s {
     std::vector<long long> rowOffsets;
     ciecu::SpPlan sp{};
     bool sliced = false;  // the last FP64 solve ran that way
+    long long waitNs = 0, withholdExchange = 0;  // ciecu_batch_debug_exchange
     double* p1 = nullptr;
     int* abortFlag = nullptr;
     unsigned long long epoch = 1;
@@ -886,7 +887,10 @@ SpLimits batch_limits() {
 }
 
 constexpr long long kBatchLaunchIterations = 4096;
+// A block waits for peers that may be busy with systems before, one after another, each up to
+// kBatchLaunchIterations of at most some 100 us (10 to 40 measured).
 constexpr long long kBatchWaitNs = 20000000000LL;
+constexpr long long kBatchWaitNsPerItem = kBatchLaunchIterations * 100000LL;
 
 // The FP64 solve as single launches; *used = false when the matrix does not suit
 // (batch_limits, sp_build).  The right-hand side is in L.r on entry.  64 uneven Q2 systems of 16 to
@@ -926,8 +930,7 @@ int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
     a.p0 = L.q;
     a.p1 = B->p1;
     a.abortFlag = B->abortFlag;
-    a.waitNs = kBatchWaitNs;
-    a.withholdEpoch = 0;
+    a.waitNs = B->waitNs > 0 ? B->waitNs : kBatchWaitNs + kBatchWaitNsPerItem * B->sp.longestList;
     BatchCtl::Shared shared{B->d_g, g0.maxIter, kBatchLaunchIterations, g0.absTol, g0.relTol};
     CIECU_TRY(allow_shared(batch_sliced_persistent_kernel));
     for (;;) {
@@ -942,6 +945,7 @@ int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
         }
         if (B->h_g->finished >= static_cast<unsigned>(B->systems)) return CIECU_OK;
         a.epoch0 = B->epoch;
+        a.withholdEpoch = B->withholdExchange > 0 ? B->epoch + static_cast<unsigned long long>(B->withholdExchange) : 0ULL;
         B->epoch += 2 * kBatchLaunchIterations + 2;
         void* params[] = {&a, &B->d_s, &shared};
         CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_sliced_persistent_kernel),
@@ -1227,6 +1231,16 @@ int ciecu_batch_form(ciecu_batch B, int* form) {
     CIECU_REQUIRE(B && form, "batch_form: null argument");
     const bool f64 = B->reliableDelta == 0.0 && B->innerTolerance == 0.0;
     *form = f64 && B->sliced ? CIECU_BATCH_SINGLE_SLICED : CIECU_BATCH_GRAPH_TILES;
+    return CIECU_OK;
+}
+
+int ciecu_batch_debug_exchange(ciecu_batch B, int64_t waitNanoseconds, int64_t withholdExchange) {
+    CIECU_REQUIRE(B, "batch_debug_exchange: null solver");
+    CIECU_REQUIRE(waitNanoseconds == 0 || (waitNanoseconds >= 1000 && waitNanoseconds <= 60000000000LL),
+                  "batch_debug_exchange: the wait limit must be 0 (by the plan) or in [1 us, 60 s]");
+    CIECU_REQUIRE(withholdExchange >= 0, "batch_debug_exchange: negative exchange index");
+    B->waitNs = waitNanoseconds;
+    B->withholdExchange = withholdExchange;
     return CIECU_OK;
 }
 

@@ -266,6 +266,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
     std::vector<SpItem> items;
     std::vector<int> begin(1, 0);
     for (const auto& l : lists) {
+        p.longestList = std::max(p.longestList, static_cast<long>(l.size()));
         items.insert(items.end(), l.begin(), l.end());
         begin.push_back(static_cast<int>(items.size()));
     }

@@ -299,6 +299,7 @@ struct SpPlan {
     size_t smem = 0;
     SpArgs args{};  // A, items, itemBegin, R, winLen, homes
     long slices = 0, steps = 0;
+    long longestList = 0;  // items of a block
     // device memory (library pool)
     double* val = nullptr;
     short2* off = nullptr;

@@ -43,6 +43,12 @@ int ciecu_batch_product(ciecu_batch solver, double inScale, const double* d_in, 
  * few at a time in a single launch over sliced rows. */
 enum { CIECU_BATCH_GRAPH_TILES = 0, CIECU_BATCH_SINGLE_SLICED = 1 };
 int ciecu_batch_form(ciecu_batch solver, int* form);
+/* Controls the bounded waits of that single launch, for tests of its timeout path, as
+ * ciecu_pcg_debug_exchange does: waitNanoseconds 0 (default) is 20 s and 0.4 s for each
+ * system that a block works through in turn; withholdExchange > 0 makes the last block of
+ * every system skip that exchange of the next launches, and the solve fails with
+ * CIECU_ERR_TIMEOUT.  The solver stays usable. */
+int ciecu_batch_debug_exchange(ciecu_batch solver, int64_t waitNanoseconds, int64_t withholdExchange);
 /* innerTolerance > 0: later products run FP32 inner solves with FP64 refinement
  * -- each round solves the FP32 copy of the matrix to innerTolerance relative
  * to the current residual for the systems not yet converged, adds the

@@ -143,3 +143,26 @@ def test_smoother_window():
     timed_out(lambda: solved(solver, problem.rhs), 30 * SECOND)
     call("ciecu_mgcg_debug_wait", solver.handle, 0)
     assert torch.equal(solved(solver, problem.rhs), first)
+
+
+@pytest.mark.parametrize("exchange", [1, 2, 7])
+@pytest.mark.parametrize("cells,systems", [(6, 200), (60, 5)])  # one block a system and more rounds; several blocks
+def test_batch_single_launch(cells, systems, exchange):
+    from cie_b200._lib import call
+    from cie_b200.fem import make_poisson
+    from cie_b200.linalg import (BatchedConjugateGradients, CUDASpace, Statistics, block_diagonal, makeDiagonalOperator)
+    space = CUDASpace()
+    problem = make_poisson(space, 2, 2, [cells, cells], seed=3)
+    matrix, offsets = block_diagonal([problem.matrix] * systems)
+    solver = BatchedConjugateGradients(matrix, offsets, space, makeDiagonalOperator(matrix, space),
+                                       Statistics(300, 0.0, 1e-9))
+    b = problem.rhs.repeat(systems)
+    first = solved(solver, b)
+    form = ctypes.c_int()
+    call("ciecu_batch_form", solver._solver, ctypes.byref(form))
+    assert form.value == 1
+    call("ciecu_batch_debug_exchange", solver._solver, MS, exchange)
+    for _ in range(2):
+        timed_out(lambda: solved(solver, b))
+    call("ciecu_batch_debug_exchange", solver._solver, 0, 0)
+    assert torch.equal(solved(solver, b), first)

@@ -397,8 +397,8 @@ __global__ void convert_kernel(long n, const A* __restrict__ a, B* __restrict__ 
 // n = A m kept by recurrences, the two dot products of an iteration, (r, u) and
 // (w, u), come from the same vectors and are reduced together, so an iteration
 // is ONE kernel: n = A m, then on the own rows
-//   z = n + beta z, q = m + beta q, s = w + beta s, p = u + beta p,
-//   x += alpha p, r -= alpha s, u -= alpha q, w -= alpha z, m' = D^-1 w,
+//   z = n + beta z, s = w + beta s, p = D^-1 r + beta p,
+//   x += alpha p, r -= alpha s, w -= alpha z, m' = D^-1 w,
 // and the partial sums of the next (r, u), (w, u); the last block forms the next
 // beta = gamma' / gamma and alpha = gamma' / (delta' - beta gamma' / alpha).  m
 // is double-buffered (a block overwrites its rows of m' while other blocks still
@@ -457,6 +457,32 @@ __global__ void __launch_bounds__(csr_threads<K>())
     }
 }
 
+// Two operands of one row pass, u and q, side by side in v.q: each sum as it would be alone.
+struct alignas(16) CoarsePair {
+    double u, q;
+    CoarsePair() = default;
+    __device__ explicit CoarsePair(double v) : u(v), q(v) {}
+    __device__ CoarsePair(double a, double b) : u(a), q(b) {}
+    __device__ CoarsePair& operator+=(const CoarsePair& o) {
+        u += o.u;
+        q += o.q;
+        return *this;
+    }
+    // what the row passes call on an operand, found by its type alone
+    friend __device__ __forceinline__ CoarsePair fma(const CoarsePair& a, const CoarsePair& x, const CoarsePair& s) {
+        return CoarsePair(::fma(a.u, x.u, s.u), ::fma(a.q, x.q, s.q));
+    }
+    friend __device__ __forceinline__ CoarsePair __ldg(const CoarsePair* p) {
+        const double2 v = ::__ldg(reinterpret_cast<const double2*>(p));
+        return CoarsePair(v.x, v.y);
+    }
+    friend __device__ __forceinline__ CoarsePair __shfl_xor_sync(unsigned mask, const CoarsePair& v, int lanes,
+                                                                 int width) {
+        return CoarsePair(::__shfl_xor_sync(mask, v.u, lanes, width), ::__shfl_xor_sync(mask, v.q, lanes, width));
+    }
+};
+
+template <bool PAIR>
 struct CoarsePipeOp {
     struct Pre {
         double z, s, p, x, r, w, d;
@@ -465,6 +491,7 @@ struct CoarsePipeOp {
     CoarseVectors v;
     const double* __restrict__ mcur;
     double* __restrict__ mnext;
+    bool keep;  // u and q too: the products are recomputed next
     double alpha, beta;
     double gamma, delta;
     __device__ __forceinline__ Pre pre(int i) const {
@@ -481,6 +508,14 @@ struct CoarsePipeOp {
         v.r[i] = r;
         v.w[i] = w;
         mnext[i] = a.d * w;
+        if (keep) {
+            if (PAIR) {
+                reinterpret_cast<CoarsePair*>(v.q)[i] = CoarsePair(u, a.d * s);
+            } else {
+                v.u[i] = u;
+                v.q[i] = a.d * s;
+            }
+        }
         gamma = fma(r, u, gamma);
         delta = fma(w, u, delta);
     }
@@ -488,12 +523,12 @@ struct CoarsePipeOp {
 
 template <int K>
 __global__ void __launch_bounds__(csr_threads<K>())
-    coarse_pipe_kernel(CsrArgs<double> A, const double* __restrict__ dinv, CoarseVectors v, int cur, MgScalars* s,
-                       double* partials, unsigned* counter) {
+    coarse_pipe_kernel(CsrArgs<double> A, const double* __restrict__ dinv, CoarseVectors v, int cur, bool keep,
+                       MgScalars* s, double* partials, unsigned* counter) {
     const volatile MgScalars* vs = s;
     double* const m0 = v.m[0];
     double* const m1 = v.m[1];
-    CoarsePipeOp op{dinv, v, cur ? m1 : m0, cur ? m0 : m1, vs->calpha, vs->cbeta, 0.0, 0.0};
+    CoarsePipeOp<K != 1> op{dinv, v, cur ? m1 : m0, cur ? m0 : m1, keep, vs->calpha, vs->cbeta, 0.0, 0.0};
     csr_rows<K, double, double, false>(A, op.mcur, op);
     double mine[2] = {op.gamma, op.delta}, tot[2];
     if (grid_reduce_last<2, csr_threads<K>()>(mine, partials, counter, tot) && threadIdx.x == 0) {
@@ -517,40 +552,57 @@ __global__ void __launch_bounds__(csr_threads<K>())
 // The recurrences for w = A u and z = A q (q = D^-1 s) lose what a product would
 // keep: after 80 iterations on a finite-cell matrix (alpha = 1e-6, 41^2 rows) the
 // iterate was up to 5e-6 from the Jacobi-PCG's.  Every kCoarseReplace iterations
-// both are recomputed as products (an elementwise kernel and two row passes)
-// together with the next alpha and beta.
+// both are recomputed as products of the u and q that the iteration left, in one
+// launch and one reading of the matrix, together with the next alpha and beta.
+// What it costs: 80 iterations (four recomputations), 4 lanes a row, 17^3 rows 701 us
+// without, 733 with, 765 by an elementwise kernel and a row pass for each product;
+// 49^3 rows 1,428, 1,448 and 1,506.
 constexpr int kCoarseReplace = 16;
 
-__global__ void __launch_bounds__(kT) coarse_precondition_kernel(long m, const double* __restrict__ dinv,
-                                                                 CoarseVectors v) {
-    for (long i = blockIdx.x * static_cast<long>(kT) + threadIdx.x; i < m; i += static_cast<long>(gridDim.x) * kT) {
-        const double d = dinv[i];
-        v.u[i] = d * v.r[i];
-        v.q[i] = d * v.s[i];
+struct CoarseReplaceOp {
+    struct Pre {
+        double r, u, d;
+    };
+    const double* __restrict__ dinv;
+    CoarseVectors v;
+    double* __restrict__ m;
+    const double* __restrict__ uOf;  // u of row i at [i * stride]
+    int stride;
+    bool first;  // of two passes: z = A q; then w, m, gamma, delta from A u
+    double gamma, delta;
+    __device__ __forceinline__ Pre pre(int i) const {
+        return first ? Pre{} : Pre{v.r[i], uOf[static_cast<long>(i) * stride], dinv[i]};
     }
-}
-
-struct CoarseProductOp {
-    struct Pre {};
-    double* __restrict__ out;
-    __device__ __forceinline__ Pre pre(int) const { return Pre{}; }
-    __device__ __forceinline__ void post(int i, const Pre&, double sum) const { out[i] = sum; }
+    __device__ __forceinline__ void post(int i, const Pre& pr, double sum) {
+        if (first) {
+            v.z[i] = sum;
+            return;
+        }
+        v.w[i] = sum;
+        m[i] = pr.d * sum;
+        gamma = fma(pr.r, pr.u, gamma);
+        delta = fma(sum, pr.u, delta);
+    }
+    __device__ __forceinline__ void post(int i, const Pre& pr, const CoarsePair& sum) {
+        v.z[i] = sum.q;
+        post(i, pr, sum.u);
+    }
 };
-
-template <int K>
-__global__ void __launch_bounds__(csr_threads<K>()) coarse_product_kernel(CsrArgs<double> A, CoarseVectors v) {
-    CoarseProductOp op{v.z};
-    csr_rows<K, double, double, false>(A, v.q, op);
-}
 
 template <int K>
 __global__ void __launch_bounds__(csr_threads<K>())
     coarse_replace_kernel(CsrArgs<double> A, const double* __restrict__ dinv, CoarseVectors v, int cur, MgScalars* s,
                           double* partials, unsigned* counter) {
-    double* const m = cur ? v.m[1] : v.m[0];
-    v.m[0] = m;
-    CoarseFirstOp op{dinv, v, 0.0, 0.0};  // w, m, gamma, delta from u
-    csr_rows<K, double, double, false>(A, v.u, op);
+    CoarseReplaceOp op{dinv, v, cur ? v.m[1] : v.m[0], K == 1 ? v.u : v.q, K == 1 ? 1 : 2, K == 1, 0.0, 0.0};
+    if constexpr (K == 1) {  // the staged schedule has no room for a second operand
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+            op.first = k == 0;
+            csr_rows<K, double, double, false>(A, k == 0 ? v.q : v.u, op);
+        }
+    } else {
+        csr_rows<K, CoarsePair, double, false>(A, reinterpret_cast<const CoarsePair*>(v.q), op);
+    }
     double mine[2] = {op.gamma, op.delta}, tot[2];
     if (grid_reduce_last<2, csr_threads<K>()>(mine, partials, counter, tot) && threadIdx.x == 0) {
         if (s->cfrozen) return;
@@ -1211,18 +1263,16 @@ int coarse_solve(ciecu_mgcg_s* M, cudaStream_t st) {
                                  st>>>(Ac->args<double>(), M->dinvc, v, M->d_s, M->partials, M->counter);
         const int g = fit_grid(coarse_pipe_kernel<K>, csr_threads<K>(), grid);
         const int gr = fit_grid(coarse_replace_kernel<K>, csr_threads<K>(), grid);
-        const int gp = fit_grid(coarse_product_kernel<K>, csr_threads<K>(), grid);
         const int its = M->options.coarseIterations;
         for (int it = 0; it < its; ++it) {
-            coarse_pipe_kernel<K><<<g, csr_threads<K>(), 0, st>>>(Ac->args<double>(), M->dinvc, v, it & 1, M->d_s,
-                                                                 M->partials, M->counter);
-            if ((it + 1) % kCoarseReplace == 0 && it + 1 < its) {
-                coarse_precondition_kernel<<<grid_of(m), kT, 0, st>>>(m, M->dinvc, v);
-                coarse_product_kernel<K><<<gp, csr_threads<K>(), 0, st>>>(Ac->args<double>(), v);
+            const bool replace = (it + 1) % kCoarseReplace == 0 && it + 1 < its;
+            coarse_pipe_kernel<K><<<g, csr_threads<K>(), 0, st>>>(Ac->args<double>(), M->dinvc, v, it & 1, replace,
+                                                                 M->d_s, M->partials, M->counter);
+            if (replace) {
                 coarse_replace_kernel<K><<<gr, csr_threads<K>(), 0, st>>>(Ac->args<double>(), M->dinvc, v,
                                                                          (it + 1) & 1, M->d_s, M->partials,
                                                                          M->counter);
-                count_launch(3);
+                count_launch(1);
             }
         }
         count_launch(1 + its);
@@ -1532,7 +1582,8 @@ int ciecu_mgcg_create(ciecu_csr fine, const double* d_fineInverseDiagonal, ciecu
     cudaError_t e = cudaSuccess;
     for (double** v : {&M->x, &M->r, &M->p, &M->q, &M->z, &M->zold, &M->t})
         if (e == cudaSuccess) e = cudaMalloc(v, sizeof(double) * n);
-    for (double** v : {&M->rc, &M->cx, &M->cr, &M->cz, &M->cp, &M->cq, &M->cu, &M->cw, &M->cs, &M->cm0, &M->cm1})
+    if (e == cudaSuccess) e = cudaMalloc(&M->cq, sizeof(double) * 2 * m);  // pairs (CoarsePair)
+    for (double** v : {&M->rc, &M->cx, &M->cr, &M->cz, &M->cp, &M->cu, &M->cw, &M->cs, &M->cm0, &M->cm1})
         if (e == cudaSuccess) e = cudaMalloc(v, sizeof(double) * m);
     if (e == cudaSuccess && !smoother32) e = cudaMalloc(&M->cheb, sizeof(double) * 4 * padded(n));
     if (e == cudaSuccess && smoother32) {

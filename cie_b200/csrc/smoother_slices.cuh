@@ -231,46 +231,67 @@ inline bool sl_layout(int n, const int* rowptr, int lo, int hi, int sms, size_t 
     row.clear();
     steps = 0;
     long longest = 0, done = 0;
-    std::vector<std::vector<short>> byLength;
+    // a block's rows: their steps, the first place of each number of steps, the rows longest
+    // first; the warp of each slice, the slices by warp
+    std::vector<int> length, lengthBegin;
+    std::vector<short> order, warpOf, mine;
+    row.reserve(static_cast<size_t>(n) + static_cast<size_t>(n) / 8 + 8);
+    sliceEnd.reserve(static_cast<size_t>(n) / kSlRows + static_cast<size_t>(n) / 64 + 8);
     for (int begin = 0, part = 0; begin < n; ++part) {
         const long until = std::max<long>(done + 1, work * (part + 1) / parts);
-        int end = begin;
-        while (end < n && end - begin < kSlBlockRows && (done < until || end - begin < kSlRows))
-            done += sl_steps(rowptr[end + 1] - rowptr[end]), ++end;
-        byLength.clear();
-        for (int i = begin; i < end; ++i) {
-            const size_t k = static_cast<size_t>(sl_steps(rowptr[i + 1] - rowptr[i]));
-            if (byLength.size() <= k) byLength.resize(k + 1);
-            byLength[k].push_back(static_cast<short>(i - begin));
+        int end = begin, most = 0;
+        length.clear();
+        while (end < n && end - begin < kSlBlockRows && (done < until || end - begin < kSlRows)) {
+            const int k = sl_steps(rowptr[end + 1] - rowptr[end]);
+            length.push_back(k);
+            most = std::max(most, k);
+            done += k;
+            ++end;
         }
+        const int rows = end - begin, count = (rows + kSlRows - 1) / kSlRows;
+        lengthBegin.assign(static_cast<size_t>(most) + 2, 0);
+        for (int k : length) ++lengthBegin[static_cast<size_t>(k)];
+        for (int k = most, at = 0; k >= 0; --k) {
+            const int here = lengthBegin[static_cast<size_t>(k)];
+            lengthBegin[static_cast<size_t>(k)] = at;
+            at += here;
+        }
+        order.resize(static_cast<size_t>(rows));
+        for (int i = 0; i < rows; ++i)
+            order[static_cast<size_t>(lengthBegin[static_cast<size_t>(length[static_cast<size_t>(i)])]++)] =
+                static_cast<short>(i);
         // slices of 8 rows, longest first, each to the warp with the least work
-        std::vector<std::pair<int, std::vector<short>>> slices;
-        for (int k = static_cast<int>(byLength.size()) - 1; k > 0; --k)
-            for (short i : byLength[k]) {
-                if (slices.empty() || slices.back().second.size() == kSlRows) slices.emplace_back(k, std::vector<short>());
-                slices.back().second.push_back(i);
-            }
-        std::vector<int> mine[kSlWarps];
+        auto stepsOf = [&](int s) { return length[static_cast<size_t>(order[static_cast<size_t>(s) * kSlRows])]; };
         long load[kSlWarps] = {};
-        for (int s = 0; s < static_cast<int>(slices.size()); ++s) {
-            const int w = static_cast<int>(std::min_element(load, load + kSlWarps) - load);
-            mine[w].push_back(s);
-            load[w] += slices[s].first;
+        int warpBegin[kSlWarps + 1] = {};
+        warpOf.resize(static_cast<size_t>(count));
+        mine.resize(static_cast<size_t>(count));
+        for (int s = 0; s < count; ++s) {
+            int w = 0;
+            for (int k = 1; k < kSlWarps; ++k) w = load[k] < load[w] ? k : w;
+            warpOf[static_cast<size_t>(s)] = static_cast<short>(w);
+            load[w] += stepsOf(s);
+            ++warpBegin[w + 1];
+        }
+        for (int w = 0; w < kSlWarps; ++w) warpBegin[w + 1] += warpBegin[w];
+        for (int s = 0, next[kSlWarps] = {}; s < count; ++s) {
+            const int w = warpOf[static_cast<size_t>(s)];
+            mine[static_cast<size_t>(warpBegin[w] + next[w]++)] = static_cast<short>(s);
         }
         SlBlock B{};
         B.rowBegin = begin;
-        B.rows = end - begin;
+        B.rows = rows;
         B.sliceBegin = static_cast<int>(sliceEnd.size());
-        B.slices = static_cast<int>(slices.size());
+        B.slices = count;
         for (int w = 0; w < kSlWarps; ++w) {
             B.warpSlice[w] = static_cast<int>(sliceEnd.size()) - B.sliceBegin;
             B.warpStep[w] = static_cast<int>(steps);
-            for (int s : mine[w]) {
-                steps += slices[s].first;
+            for (int k = warpBegin[w]; k < warpBegin[w + 1]; ++k) {
+                const int s = mine[static_cast<size_t>(k)];
+                steps += stepsOf(s);
                 sliceEnd.push_back(static_cast<int>(steps));
-                for (int i = 0; i < kSlRows; ++i)
-                    row.push_back(i < static_cast<int>(slices[s].second.size()) ? slices[s].second[i]
-                                                                               : static_cast<short>(-1));
+                for (int i = s * kSlRows; i < (s + 1) * kSlRows; ++i)
+                    row.push_back(i < rows ? order[static_cast<size_t>(i)] : static_cast<short>(-1));
             }
         }
         B.warpSlice[kSlWarps] = B.slices;

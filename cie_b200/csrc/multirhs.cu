@@ -1137,8 +1137,8 @@ struct PqQuad {
 };
 
 // K2 and K3 for k = 32 with four columns per lane.  x is updated in K3, which reads the
-// old direction anyway, instead of in K2: ten instead of nine vector passes shrink to
-// eight (R, Q in, R out; X, P, R in, X, P out), in 16-byte accesses.  FP32, 128^3: the
+// old direction anyway, instead of in K2: nine vector passes (X, P, R, Q in, X, R out; P, R
+// in, P out) become eight (R, Q in, R out; X, P, R in, X, P out), in 16-byte accesses.  FP32, 128^3: the
 // row-per-warp pair took 410 + 156 us.
 constexpr int kVecRows = 2;  // rows a thread has in flight
 
@@ -1455,8 +1455,10 @@ __global__ void __launch_bounds__(kT, 3) multi_spmv_quad3_f32_kernel(DiaArgs<flo
     multi_spmv_quad<DiaArgs<float>, float, COND, true>(A, P, Q, S, g, partials, counter, cond);
 }
 
-// ... and the staged one, one CTA per SM, where two stages fit in shared memory (planes
-// of up to about 190 nodes a line).
+// ... and the staged one, one CTA per SM, where two stages fit in shared memory: lines of up
+// to 175 nodes in planes of more than kPlaneRows and two lines (three runs of diagonals), or
+// all diagonals of very small planes in one run.  Between them, planes of some 8^2 to 20^2
+// nodes, one run of the 27 diagonals does not fit twice.
 template <bool COND>
 __global__ void __launch_bounds__(kPlaneThreads, 1)
     multi_spmv_planes_f32_kernel(DiaArgs<float> A, const __grid_constant__ PlaneArgs planes,

@@ -148,3 +148,33 @@ def test_batches(order, cells, systems, form):
     ref = np.linalg.solve(m.toarray(), b.T).T / scale[:, None]
     err = np.linalg.norm(x.cpu().numpy().reshape(systems, n) - ref, axis=1) / np.linalg.norm(ref, axis=1)
     assert err.max() <= 1e-6
+
+
+@pytest.mark.parametrize("line,plane,n,form", [
+    (102, 10302, 1060001, 2), (9, 2707, 1100000, 2), (61, 12205, 1050011, 2), (129, 16641, 1060000, 2),
+    (300, 90000, 1080000, 1),   # the halo of a tile costs more than it saves
+    (102, 10302, 1040000, 1),   # the upper half fits in L2
+])
+def test_large_stencils(line, plane, n, form):
+    """The graph loop over symmetric 27-diagonal matrices: by marching tiles, or rows of the upper half."""
+    from cie_b200._lib import call
+    from cie_b200.linalg import ConjugateGradients, CSRMatrix, CSROperator, CUDASpace, Statistics, makeDiagonalOperator
+    offsets = torch.tensor(sorted(dz * plane + dy * line + dx for dz in (-1, 0, 1) for dy in (-1, 0, 1)
+                                  for dx in (-1, 0, 1)), device="cuda")
+    columns = torch.arange(n, device="cuda")[:, None] + offsets
+    inside = (columns >= 0) & (columns < n)
+    extents = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+    extents[1:] = inside.sum(1).cumsum(0).to(torch.int32)
+    entries = torch.where(offsets == 0, 28.0, -1.0).to(torch.float64).expand(n, 27)[inside]
+    space = CUDASpace()
+    matrix = CSRMatrix(n, extents, columns[inside].to(torch.int32), entries)
+    A = CSROperator(matrix, space)
+    solver = ConjugateGradients(A, space, makeDiagonalOperator(matrix, space, csr_handle=A.csr), Statistics(2, 0.0, 1e-300))
+    solver.set_loop(1)
+    solver.set_schedule(64)
+    b = torch.ones(n, dtype=torch.float64, device="cuda")
+    x = torch.zeros_like(b)
+    solver.product(0.0, b, 1.0, x)
+    got = ctypes.c_int()
+    call("ciecu_pcg_form", solver._solver, ctypes.byref(got))
+    assert solver.info()["dia_symmetric"] and got.value == form

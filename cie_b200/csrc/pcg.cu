@@ -961,7 +961,7 @@ int ensure_persistent_buffers(ciecu_pcg_s* S) {
 }
 
 // The single launch over the DIA copy, where its windows and the vectors q, r and x
-// of a block fit in shared memory (dp_plan): 3D Q1 up to about 88^3, 2D Q1 to 1,400^2.
+// of a block fit in shared memory (dp_plan): 3D Q1 up to 88^3 rows, 2D Q1 to 990^2.
 // Per iteration on B200 against the graph of three kernels (or, where it fitted, the
 // single launch over CSR rows): 2D Q1 256^2 8.0 against 12.9 us, 3D Q1 64^3 15.2
 // against 33 us.  Larger systems keep the graph: with the vectors in global memory a

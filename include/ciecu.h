@@ -131,12 +131,12 @@ int ciecu_csr_autotune(ciecu_csr csr);
 int ciecu_csr_spmv_f64(ciecu_csr csr, double inScale, const double* d_in, double outScale, double* d_out);
 /* CSROperator<int,float>::product for a CIECU_F32 matrix. */
 int ciecu_csr_spmv_f32(ciecu_csr csr, float inScale, const float* d_in, float outScale, float* d_out);
-/* MaskedCSROperator<int,double,double,uint16_t>::product (MaskedCSROperator.cpp:37-118):
- * rows/columns with mask >= threshold are excluded; masked rows receive
- * combine(inScale, out, outScale, 0) (CPU semantics, :51-66). */
 /* enter, ciecu_csr_spmv_f64 or _f32 by the matrix's value type, and leave. */
 int ciecu_csr_product(ciecu_csr csr, void* callerStream, double inScale, const void* d_in, double outScale,
                       void* d_out);
+/* MaskedCSROperator<int,double,double,uint16_t>::product (MaskedCSROperator.cpp:37-118):
+ * rows/columns with mask >= threshold are excluded; masked rows receive
+ * combine(inScale, out, outScale, 0) (CPU semantics, :51-66). */
 int ciecu_csr_masked_spmv_f64(ciecu_csr csr, const uint16_t* d_mask, uint16_t threshold,
                               double inScale, const double* d_in, double outScale, double* d_out);
 

@@ -403,6 +403,7 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
         e = pool_alloc(&P->d_pos, std::max<size_t>(1, static_cast<size_t>(incidences) * nb * P->posBytes), st);
     if (e == cudaSuccess) e = pool_alloc(&P->d_gtab, sizeof(double) * gtab.size(), st);
     if (e == cudaSuccess) e = pool_alloc(&P->d_wq, sizeof(double) * wq.size(), st);
+    if (e == cudaSuccess) e = pool_alloc(&P->d_unit, sizeof(double) * nb * nb, st);
     if (e == cudaSuccess) e = pool_alloc(&scratch, sizeof(int) * scratchInts, st);
     int* d_order = scratch;
     int* d_count = scratch + ncells;
@@ -474,7 +475,7 @@ int ciecu_assembly_create(ciecu_csr csr, int dim, int order, int quadratureOrder
 int ciecu_assembly_destroy(ciecu_assembly P) {
     if (!P) return CIECU_OK;
     // No access to P->csr (it may already be gone); pool_release synchronises the device.
-    pool_release({P->d_incStart, P->d_inc, P->d_pos, P->d_gtab, P->d_wq});
+    pool_release({P->d_incStart, P->d_inc, P->d_pos, P->d_gtab, P->d_wq, P->d_unit});
     delete P;
     return CIECU_OK;
 }
@@ -494,15 +495,23 @@ int ciecu_assemble_stiffness(ciecu_assembly P, const double* d_kappa, const doub
     convention_factors(P->dim, h_cellSize, convention, scale, f);
     // the reference element's sums, once per call: each contribution to an entry is
     // fma(kappa_e scale, S[a][b], entry), one rounding, so that the host restatement
-    // of this summation order reproduces the matrix bit for bit.  The sums belong to
-    // the call, not to the plan: threads may assemble with one plan and different cell
-    // sizes or conventions, and a captured call may be replayed beside another.
+    // of this summation order reproduces the matrix bit for bit
+    auto submit = [&](double* unit) -> int {
+        CIECU_TRY(unit_element(P, 1.0, f, unit, st));
+        return launch_row_gather<double>(P, UniformSource{d_kappa, scale}, unit, accumulate ? 1 : 0, d_entries, st);
+    };
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CIECU_CUDA(cudaStreamIsCapturing(st, &capture));
+    if (capture == cudaStreamCaptureStatusNone) {
+        // threads may assemble with one plan and different cell sizes or conventions
+        std::lock_guard<std::mutex> lock(P->unitMutex);
+        return submit(P->d_unit);
+    }
+    // A captured call has its own buffer, in the graph: it may be replayed beside another call.
     double* unit = nullptr;
     CIECU_CUDA(pool_alloc(&unit, sizeof(double) * P->nb * P->nb, st));
-    int status = unit_element(P, 1.0, f, unit, st);
-    if (status == CIECU_OK)
-        status = launch_row_gather<double>(P, UniformSource{d_kappa, scale}, unit, accumulate ? 1 : 0, d_entries, st);
-    const cudaError_t e = cudaFreeAsync(unit, st);  // stream-ordered: after the gather
+    const int status = submit(unit);
+    const cudaError_t e = cudaFreeAsync(unit, st);
     if (status == CIECU_OK && e != cudaSuccess) return cuda_fail(e, "assemble_stiffness: free");
     return status;
 }

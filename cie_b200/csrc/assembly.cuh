@@ -8,7 +8,7 @@
 
 #include <algorithm>
 #include <cstdint>
-
+#include <mutex>
 #include <vector>
 
 struct ciecu_assembly_s {
@@ -28,6 +28,10 @@ struct ciecu_assembly_s {
     int colors = 0;
     double* d_gtab = nullptr;         // nq * dim * nb parametric gradients
     double* d_wq = nullptr;           // nq weights
+    // nb * nb: the reference element's sums of the call that holds the lock while it submits
+    // what writes and reads them; the next call's come after them on the stream.
+    double* d_unit = nullptr;
+    std::mutex unitMutex;
     int q1 = 0;                       // 1-D quadrature points (nq = q1^dim)
     std::vector<double> gn, gw;       // 1-D Gauss-Legendre rule on [-1, 1]
 };

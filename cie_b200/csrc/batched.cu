@@ -388,10 +388,11 @@ struct BatchCtl {
     }
 };
 
+template <bool LONG>
 __global__ void __launch_bounds__(kSpThreads, 1) batch_sliced_persistent_kernel(const __grid_constant__ SpArgs P,
                                                                                 BatchScalars* s,
                                                                                 BatchCtl::Shared shared) {
-    sp_solve<true, BatchCtl>(P, s, shared);
+    sp_solve<true, LONG, BatchCtl>(P, s, shared);
 }
 
 // ---- reliable-update form: FP32 iterations, FP64 residual replacements ------
@@ -932,7 +933,8 @@ int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
     a.abortFlag = B->abortFlag;
     a.waitNs = B->waitNs > 0 ? B->waitNs : kBatchWaitNs + kBatchWaitNsPerItem * B->sp.longestList;
     BatchCtl::Shared shared{B->d_g, g0.maxIter, kBatchLaunchIterations, g0.absTol, g0.relTol};
-    CIECU_TRY(allow_shared(batch_sliced_persistent_kernel));
+    auto* kernel = B->sp.longRows ? batch_sliced_persistent_kernel<true> : batch_sliced_persistent_kernel<false>;
+    CIECU_TRY(allow_shared(kernel));
     for (;;) {
         int aborted = 0;
         CIECU_CUDA(cudaMemcpyAsync(B->h_g, B->d_g, sizeof(BatchGlobal), cudaMemcpyDeviceToHost, st));
@@ -948,8 +950,8 @@ int run_sliced(ciecu_batch_s* B, const BatchGlobal& g0, bool* used) {
         a.withholdEpoch = B->withholdExchange > 0 ? B->epoch + static_cast<unsigned long long>(B->withholdExchange) : 0ULL;
         B->epoch += 2 * kBatchLaunchIterations + 2;
         void* params[] = {&a, &B->d_s, &shared};
-        CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(batch_sliced_persistent_kernel),
-                                               dim3(B->sp.grid), dim3(B->sp.threads), params, B->sp.smem, st));
+        CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(B->sp.grid),
+                                               dim3(B->sp.threads), params, B->sp.smem, st));
         count_launch();
     }
 }

@@ -672,10 +672,10 @@ struct SpPcgCtl {
     static __device__ void finish(PcgScalars&, Shared) {}
 };
 
-template <bool PRECOND>
+template <bool PRECOND, bool LONG>
 __global__ void __launch_bounds__(kSpThreads, 1) pcg_sliced_persistent_kernel(const __grid_constant__ SpArgs P,
                                                                               PcgScalars* s) {
-    sp_solve<PRECOND, SpPcgCtl>(P, s, SpPcgCtl::Shared{});
+    sp_solve<PRECOND, LONG, SpPcgCtl>(P, s, SpPcgCtl::Shared{});
 }
 
 __global__ void fill_ones_kernel(long n, double* __restrict__ v) {
@@ -1047,7 +1047,9 @@ int launch_sliced_persistent(ciecu_pcg_s* S, cudaStream_t st) {
     a.epoch0 = S->epoch;
     a.waitNs = S->waitNs;
     a.withholdEpoch = S->withholdExchange > 0 ? S->epoch + static_cast<unsigned long long>(S->withholdExchange) : 0ULL;
-    auto* kernel = S->dinv ? pcg_sliced_persistent_kernel<true> : pcg_sliced_persistent_kernel<false>;
+    auto* kernel = S->sp.longRows
+                       ? (S->dinv ? pcg_sliced_persistent_kernel<true, true> : pcg_sliced_persistent_kernel<false, true>)
+                       : (S->dinv ? pcg_sliced_persistent_kernel<true, false> : pcg_sliced_persistent_kernel<false, false>);
     CIECU_TRY(allow_shared(kernel));
     void* params[] = {&a, &S->d_s};
     CIECU_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(S->sp.grid), dim3(S->sp.threads),

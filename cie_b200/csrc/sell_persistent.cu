@@ -332,6 +332,7 @@ int sp_build(SpPlan& p, const ciecu_csr_s* csr, const std::vector<long long>& ro
         p.state = 0;
         return cuda_fail(e, "sliced copy: offsets");
     }
+    p.longRows = !longRows.empty();
     p.args.A = SpMatrix{p.val, p.off, p.sliceStep, p.row, p.longRow, csr->rowptr, csr->col,
                         static_cast<const double*>(csr->val)};
     p.args.items = p.items;

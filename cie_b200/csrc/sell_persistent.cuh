@@ -107,7 +107,8 @@ __host__ __device__ __forceinline__ int sp_place(int x, int half) { return (x & 
 // Ctl: Scalars, Shared (settings of the launch), and as in dia_persistent.cuh
 // start / afterProduct / afterUpdate with the settings as a further argument, and
 // finish(scalars, settings) run by the system's first block after its last exchange.
-template <bool PRECOND, typename Ctl>
+// LONG: some rows are in no slice (a kernel of its own: the test alone cost 1 % of a batch).
+template <bool PRECOND, bool LONG, typename Ctl>
 __device__ __forceinline__ void sp_solve(const SpArgs& P, typename Ctl::Scalars* scalars, typename Ctl::Shared shared) {
     extern __shared__ __align__(16) unsigned char sp_smem[];
     __shared__ typename Ctl::Scalars s_scalars;
@@ -221,7 +222,7 @@ __device__ __forceinline__ void sp_solve(const SpArgs& P, typename Ctl::Scalars*
                 }
             }
             // A long row to a warp, from the matrix itself: one thread would take 20 ns an entry.
-            for (int k = warp; k < I.longRows; k += warps) {
+            for (int k = warp; LONG && k < I.longRows; k += warps) {
                 const int row = P.A.longRow[I.longBegin + k], k1 = P.A.rowptr[row + 1];
                 const int at = -rb - I.lo, half = P.winLen / 2;
                 double sum = 0.0;
@@ -300,6 +301,7 @@ struct SpPlan {
     SpArgs args{};  // A, items, itemBegin, R, winLen, homes
     long slices = 0, steps = 0;
     long longestList = 0;  // items of a block
+    bool longRows = false;
     // device memory (library pool)
     double* val = nullptr;
     short2* off = nullptr;

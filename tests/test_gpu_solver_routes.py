@@ -150,6 +150,29 @@ def test_batches(order, cells, systems, form):
     assert err.max() <= 1e-6
 
 
+@pytest.mark.parametrize("counts,form", [((1, 0, 2), 1), ((8, 0, 0), 1),
+                                         ((3, 3, 3), 0)])  # too many for warps, and too much padding in slices
+def test_batch_with_long_rows(counts, form):
+    from cie_b200._lib import call
+    from cie_b200.linalg import BatchedConjugateGradients, CUDASpace, Statistics, makeDiagonalOperator
+    parts = [symmetric(long_rows(1500 + 130 * k, 700, c) if c else band(900, 12), 11 + k) for k, c in enumerate(counts)]
+    space = CUDASpace()
+    matrix = device_matrix(sp.block_diag(parts, format="csr"))
+    offsets = np.concatenate([[0], np.cumsum([m.shape[0] for m in parts])]).astype(np.int64)
+    solver = BatchedConjugateGradients(matrix, offsets, space, makeDiagonalOperator(matrix, space),
+                                       Statistics(2000, 0.0, 1e-10))
+    b = np.random.default_rng(8).uniform(-1, 1, offsets[-1])
+    x = torch.zeros(len(b), dtype=torch.float64, device="cuda")
+    solver.product(0.0, torch.as_tensor(b).cuda(), 1.0, x)
+    got = ctypes.c_int()
+    call("ciecu_batch_form", solver._solver, ctypes.byref(got))
+    assert got.value == form
+    for k, m in enumerate(parts):
+        part = slice(offsets[k], offsets[k + 1])
+        ref = np.linalg.solve(m.toarray(), b[part])
+        assert np.linalg.norm(x.cpu().numpy()[part] - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
 @pytest.mark.parametrize("line,plane,n,form", [
     (102, 10302, 1060001, 2), (9, 2707, 1100000, 2), (61, 12205, 1050011, 2), (129, 16641, 1060000, 2),
     (300, 90000, 1080000, 1),   # the halo of a tile costs more than it saves

@@ -462,8 +462,9 @@ class ConjugateGradients(LinearOperator):
 
     def set_loop(self, mode):
         """How the fused solver runs its iterations: 0 auto (a single cooperative
-        launch when every SM's rows of the matrix fit in its shared memory), 1 the
-        graph of three kernels per iteration, 2 the single launch."""
+        launch over the diagonal copy, sliced rows or CSR rows where one fits and is
+        faster; ciecu_pcg_set_loop), 1 the graph of three kernels per iteration, 2 a
+        single launch."""
         if self._solver is not None:
             call("ciecu_pcg_set_loop", self._solver, int(mode))
 

@@ -226,8 +226,8 @@ int ciecu_pcg_set_graph_chunk(ciecu_pcg solver, int iterations);
  * (single launch) the pin has no effect. */
 int ciecu_pcg_set_schedule(ciecu_pcg solver, int schedule);
 /* SpMV schedule the solver's autotuner chose for its fused q = A p kernel (0 before
- * the first solve or when the solve ran as a single launch; 1 = row-block stream
- * kernel, else lanes per row) and how the last solve ran: host-polled graph chunks
+ * the first solve or when the solve ran as a single launch, 64 when that was over the
+ * diagonal-storage copy; 1 = row-block stream kernel, else lanes per row) and how the last solve ran: host-polled graph chunks
  * (0), a device-side graph loop (1) or a single cooperative launch (2). */
 int ciecu_pcg_info(ciecu_pcg solver, int* spmvSchedule, int* deviceLoop);
 /* The diagonal-storage copy at the last solve: the diagonals K1 reads (0: no
@@ -235,12 +235,14 @@ int ciecu_pcg_info(ciecu_pcg solver, int* spmvSchedule, int* deviceLoop);
  * symmetric matrix, checked at every solve, whose lower entries K1 reads back from
  * it (about half the matrix bytes; CIECU_DIA_SYMMETRIC=0 keeps the full copy). */
 int ciecu_pcg_dia_info(ciecu_pcg solver, int* storedDiagonals, int* symmetric);
-/* How the iterations run.  mode 0 (default): a single cooperative launch of at
- * most one block per SM (the fewest of SMs/4, SMs/2, SMs that fit), each block
- * holding its rows of the matrix in shared memory, when the rows fit there at one
- * block per SM, else the graph of three kernels per iteration; 1: always the
- * graph; 2: always the single launch (CIECU_ERR_ARGUMENT at the next solve when
- * the matrix does not fit).  The single launch gives results within rounding of
+/* How the iterations run.  mode 0 (default): a single cooperative launch of at most one
+ * block per SM where one is the faster way (over the diagonal-storage copy when a block's
+ * windows and vectors fit in its shared memory; else over sliced rows within measured
+ * limits; else over CSR rows when every block's rows of the matrix fit), otherwise, and
+ * where there is no room for its copies, the graph of three kernels per iteration; 1:
+ * always the graph; 2: always a single launch (CIECU_ERR_ARGUMENT at the next solve when
+ * the CSR rows do not fit the blocks' shared memory).  ciecu_pcg_form tells which ran.
+ * A single launch gives results within rounding of
  * the graph's (its dot products are summed over another grid); a grid-wide wait
  * that gives up fails with CIECU_ERR_TIMEOUT. */
 int ciecu_pcg_set_loop(ciecu_pcg solver, int mode);
